@@ -239,11 +239,9 @@ KERNEL_WHAT = {0: "pass-1 M q_j with |M q_j|^2",
                3: "pass-2 regeneration (solves longer than the basis store)"}
 
 
-def kernel_name(k, shape=""):
-    """Timer class k (4-7: FP32 vectors); shape: the stencil shape the
-    autotuner chose for pass 1 at this lattice and precision."""
-    name = KERNEL_NAMES[k % 4] + (" fp32" if k >= 4 else " fp64")
-    return name + (f" ({shape})" if shape and k % 4 < 2 else "")
+def kernel_name(k):
+    """Timer class k (4-7: FP32 vectors)."""
+    return KERNEL_NAMES[k % 4] + (" fp32" if k >= 4 else " fp64")
 
 
 def cpu_iteration_cost(L, Ls, threads, iters, npole=20):
@@ -691,23 +689,10 @@ def instrumented_chunks(prog, chi0, state0):
     return out
 
 
-def rows_chosen(L, Ls, k):
-    """The stencil shape the autotuner chose for class k's precision."""
-    import chiralheisenberg_b200 as chb
-    elem = 8 if k >= 4 else 16
-    # FP32 solves with Ls even run the split-layout kernels (their own entry)
-    layout = "split" if (k >= 4 and Ls % 2 == 0) else "plain"
-    for t in chb.autotune_report():
-        if (t["L"], t["Lt"], t["Ls"], t["elem_bytes"], t.get("layout", "plain")) == \
-                (L, L, Ls, elem, layout):
-            return t["choice"]
-    return ""
-
-
 def kernel_table(kt, L, Ls):
     kms, ktimed, klaunched, kbytes = kt
     tot = max(float(np.sum(kms)), 1e-30)
-    return {kernel_name(k, rows_chosen(L, Ls, k)): {"launches": int(klaunched[k]),
+    return {kernel_name(k): {"launches": int(klaunched[k]),
                              "avg_us": kms[k] / max(ktimed[k], 1) * 1e3,
                              "share_of_solver_time": kms[k] / tot,
                              "GBps": (kbytes[k] / (kms[k] * 1e-3) / 1e9) if kms[k] > 0 else None}
@@ -824,7 +809,7 @@ def run_b200(args, rank, world, local_rank):
     tp = os.path.join(ROOT, "profiles", "traffic_24x24.json")
     if os.path.exists(tp):
         # ncu figures are per stencil shape; another shape's traffic is unknown
-        traffic = json.load(open(tp)).get(kernel_name(dom, rows_chosen(L, Ls, dom)))
+        traffic = json.load(open(tp)).get(kernel_name(dom))
     prof = profile_of(recs)
     its_value = sum(prof[k] for k in ("it_pf", "it_h0", "it_h1", "it_force"))
     line = {"metric": "s/trajectory", "value": value, "unit": "s", "n_gpus": world,
@@ -837,7 +822,7 @@ def run_b200(args, rank, world, local_rank):
                     "d2h_bytes_per_step": d2h, "same_trajectories_as_value": same,
                     "step_ms": [round(x, 1) for x in step_ms_e2e]},
             "fp64": fp64,
-            "roofline": {"bound": "hbm", "kernel": kernel_name(dom, rows_chosen(L, Ls, dom)),
+            "roofline": {"bound": "hbm", "kernel": kernel_name(dom),
                          "what": KERNEL_WHAT[dom % 4],
                          "achieved": achieved, "peak": peak, "peak_kind": peak_kind,
                          "unit": "GB/s", "frac": achieved / peak, "traffic": traffic,

@@ -10,9 +10,8 @@
 // lattice point (s, site) and all eight components, so every plane access of
 // a warp is a contiguous, coalesced run of 16-byte (FP64) elements and the
 // host<->device copies at the drop-in boundary are plain memcpys.  The
-// solver's FP32 Krylov vectors (Ls even, never copied across the boundary)
-// keep the same planes with each pair of adjacent s split by part: see
-// cpair below.
+// solvers' own vectors never cross it and are laid out differently
+// (planes.cuh).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -101,9 +100,7 @@ __device__ __forceinline__ double2 zcomb(double2 x, double2 y, bool use_i, int s
 
 // ---- single-precision complex (mixed-precision path) ----------------------
 // Also without contraction: every kernel that evaluates the same per-element
-// sequence (the pass-1 kernels and the regenerating pass 2, whatever their
-// thread shape) then produces the same bits, so regenerated Lanczos vectors
-// equal the first pass's.
+// sequence then produces the same bits, whatever its thread shape.
 //
 // On sm_100 an addition or subtraction of FP32 complex numbers is one packed
 // FP32x2 instruction (add/sub.rn.f32x2, written as PTX) instead of two scalar
@@ -158,9 +155,10 @@ __device__ __forceinline__ float2 zcomb(float2 x, float2 y, bool use_i, int sgn)
 }
 
 // ---- FP32 complex numbers of two adjacent points, split by part ------------
-// The solver's FP32 Krylov vectors (Ls even) keep every aligned element pair
-// (e, e+1), e even -- two adjacent s of one component -- as the 16 bytes
-// (re_e, re_e+1, im_e, im_e+1): the "split" layout.  One 16-byte load then
+// Two adjacent s of one component as the 16 bytes (re_s, re_s+1, im_s,
+// im_s+1): the unit of the solvers' FP32 vectors (planes.cuh), and, as a
+// vector of element pairs (e, e+1) in the ABI's order, the "split" layout of
+// dwf_apply_flavour_pair_sp.  One 16-byte load then
 // puts both real parts in one register pair and both imaginary parts in the
 // other, so each complex operation on the two points, i*y included, is two
 // packed instructions with no lane exchange; per element the IEEE operations

@@ -20,6 +20,10 @@
 // on x_k on those two slices alone.
 // alpha~_j = q_j^dagger M^dagger M q_j is evaluated as |M q_j|^2, which lets
 // the three-term update be fused into the M^dagger kernel.
+//
+// The Krylov vectors are site-fastest planes (planes.cuh).
+// CHDWF_STENCIL=rows selects the row-staged kernels for pass 1 instead, whose
+// vectors have the ABI's layout (FP64, and FP32 with odd Ls).
 #include <cmath>
 #include <cstddef>
 #include <cstring>
@@ -28,6 +32,7 @@
 
 #include "dwf_stencil.cuh"
 #include "lanczos.h"
+#include "planes.cuh"
 
 namespace chdwf {
 
@@ -41,18 +46,23 @@ __device__ __forceinline__ double2 widen(float2 v) { return make_double2((double
 
 template <class T>
 __device__ __forceinline__ T* ring(const LzArgsT<T>& a, int j) {
-    if (j < a.hcap) return a.basis + (int64_t)j * a.g.kferm;
+    if (j < a.hcap) return a.basis + (int64_t)j * a.vs;
     const int r = j % 3;
     return r == 0 ? a.rb0 : (r == 1 ? a.rb1 : a.rb2);
 }
 
-// Element e of a Krylov vector: FP32 vectors with Ls even are in the split
-// layout (cpair), FP64 vectors and odd-Ls FP32 vectors plain.
-__device__ __forceinline__ double2 vget(const LzArgsT<double2>&, const double2* v, int64_t e) {
-    return __ldg(v + e);
+// Element (c, s, site) of a Krylov vector, in planes or in the ABI's layout.
+__device__ __forceinline__ double2 vget(const LzArgsT<double2>& a, const double2* v, int c, int s,
+                                        int64_t site) {
+    return a.pl ? v[((int64_t)c * a.pp.U + s) * a.g.kvol + site]
+                : v[s + (int64_t)a.g.Ls * site + a.g.cs * c];
 }
-__device__ __forceinline__ float2 vget(const LzArgsT<float2>& a, const float2* v, int64_t e) {
-    return a.pl ? sp_get(v, e) : __ldg(v + e);
+__device__ __forceinline__ float2 vget(const LzArgsT<float2>& a, const float2* v, int c, int s,
+                                       int64_t site) {
+    if (!a.pl) return v[s + (int64_t)a.g.Ls * site + a.g.cs * c];
+    const float* f = reinterpret_cast<const float*>(
+        v + 2 * (((int64_t)c * a.pp.U + (s >> 1)) * a.g.kvol + site));
+    return make_float2(f[s & 1], f[2 + (s & 1)]);
 }
 
 static_assert(kSplitThreads == kThreads, "the reductions assume kThreads-wide blocks");
@@ -61,19 +71,6 @@ static_assert(kSplitThreads == kThreads, "the reductions assume kThreads-wide bl
 template <class T>
 static inline int timer_class(int c) {
     return c + (std::is_same<T, float2>::value ? 4 : 0);
-}
-
-// Sum of the n chunk partials part[0..n) in a fixed order; every block that
-// calls it gets the same value.  Valid in all threads.
-__device__ __forceinline__ double sum_partials(const double* part, int n) {
-    __shared__ double sh[kThreads / 32];
-    __shared__ double total;
-    double s = 0.0;
-    for (int i = threadIdx.x; i < n; i += kThreads) s += __ldcg(part + i);
-    s = block_sum<kThreads>(s, sh);
-    if (threadIdx.x == 0) total = s;
-    __syncthreads();
-    return total;
 }
 
 // The stop flag, read once per block: every thread of a block takes the same
@@ -85,51 +82,24 @@ __device__ __forceinline__ bool block_stopped(const LzCtl* ctl) {
     return s_done != 0;
 }
 
-// ---- thread mapping ----------------------------------------------------------
+// ---- thread mapping of the regenerating pass 2 on the ABI's layout -----------
 // FP64 vectors: two threads per point, one per flavour (split_point /
-// split_flavour), which halves the accumulator registers and doubles the
-// warps in flight.  FP32 vectors with Ls even (PAIR): a thread takes two
-// adjacent points of one flavour, loading both with one 16-byte float4.
-// FP32 otherwise: one thread per point and both flavours.
-template <class T, bool PAIR = false> struct LzShape;
-template <> struct LzShape<double2, false> {
+// split_flavour).  FP32 vectors: one thread per point and both flavours.
+template <class T> struct LzShape;
+template <> struct LzShape<double2> {
     static constexpr bool split = true;
     static constexpr int min_blocks = 3;          // <= 85 registers: no spills
-    static constexpr int unit = kSplitPoints;     // points per block pass
+    static constexpr int unit = kSplitPoints;     // points per block
 };
-template <> struct LzShape<float2, false> {
+template <> struct LzShape<float2> {
     static constexpr bool split = false;
     static constexpr int min_blocks = 3;          // <= 85 registers a thread
     static constexpr int unit = kThreads;
 };
-template <> struct LzShape<float2, true> {
-    static constexpr bool split = true;
-    static constexpr int min_blocks = 3;
-    static constexpr int unit = 2 * kSplitPoints; // 128 point pairs per flavour
-};
 
-// Pass 1 runs on a persistent grid (a whole number of blocks per SM); block b
-// owns the contiguous, warp-aligned point range below, so every SM gets the
-// same amount of work and none idles through a partial last wave.  Each
-// block leaves its |.|^2 partial in part[b]; the kernel that needs the sum
-// adds the partials itself, in block order, so no block waits on another.
-struct PtRange { int64_t begin, end; };
-__device__ __forceinline__ PtRange block_range(int64_t npts) {
-    const int64_t nb = gridDim.x, b = blockIdx.x;
-    PtRange r;
-    r.begin = (b * npts / nb) & ~(int64_t)31;
-    r.end = b + 1 == nb ? npts : (((b + 1) * npts / nb) & ~(int64_t)31);
-    return r;
-}
-
-// One block pass over points [base, base + unit) of flavour(s) f0..f0+NF-1
-// (PAIR: p is the even point of the thread's pair).
-template <class T, bool PAIR = false>
+template <class T>
 __device__ __forceinline__ void lz_lane(int64_t base, int64_t* p, int* f0) {
-    if (PAIR) {
-        *p = base + 2 * (threadIdx.x & (kSplitPoints - 1));
-        *f0 = split_flavour();
-    } else if (LzShape<T>::split) {
+    if (LzShape<T>::split) {
         *p = base + (threadIdx.x & (kSplitPoints - 1));
         *f0 = split_flavour();
     } else {
@@ -139,8 +109,7 @@ __device__ __forceinline__ void lz_lane(int64_t base, int64_t* p, int* f0) {
 }
 
 // vt = M q_j with q_j = r_j / beta_j, formed as (1/beta_j) (M r_j): one
-// scaling per output element instead of one per stencil load.  The pass-1
-// kernel and the regenerating pass 2 use this same sequence.
+// scaling per output element instead of one per stencil load.
 template <bool DAG, int IMASS, class T>
 __device__ __forceinline__ void apply_scaled(T acc[4], const T* r, typename real_of<T>::type ib,
                                              const LzArgsT<T>& a, const PointIdx& q, int f) {
@@ -150,140 +119,43 @@ __device__ __forceinline__ void apply_scaled(T acc[4], const T* r, typename real
     for (int d = 0; d < 4; d++) acc[d] = zscal(ib, acc[d]);
 }
 
-// ---- pass 1, kernel 1: vt = M q_j and the block partials of |vt|^2 ---------
-// beta_j is the sum of the previous M^dagger launch's partials (beta_1 comes
-// from the source), formed by every block.  The partial buffers: part[0..nb)
-// for this kernel, part[nb..2nb) for M^dagger.
-template <class T, int IMASS, bool PAIR, int OCC>
-__global__ void __launch_bounds__(kThreads, OCC) k_lz1_M(LzArgsT<T> a) {
-    typedef typename real_of<T>::type Real;
-    typedef LzShape<T, PAIR> S;
-    constexpr int NF = S::split ? 1 : 2;
-    // One flavour a thread: beta_j is first needed to scale the block's
-    // first outputs, so its sum over the previous launch's partials (an L2
-    // round trip and two block barriers) is formed after the first pass's
-    // stencil loads are issued.  Every thread of the block reaches it (the
-    // loop's trip count is the same for the whole block).
-    constexpr bool LATE = NF == 1;
-    LzCtl* ctl = a.ctl;
-    if (block_stopped(ctl)) return;
-    const int j = ctl->it_m;
-    const int nb = gridDim.x;
-    bool have = j == 1 || !LATE;
-    double bj = j == 1 ? a.h.beta[1] : (LATE ? 0.0 : sqrt(sum_partials(a.part + nb, nb)));
-    double ibj = j == 1 ? a.h.invbeta[1] : (LATE ? 0.0 : 1.0 / bj);
-    const T* rj = ring(a, j);
-    const PtRange R = block_range(a.g.npts);
-    double loc = 0.0;
-#pragma unroll 1
-    for (int64_t base = R.begin; base < R.end; base += S::unit) {
-        int64_t p;
-        int f0;
-        lz_lane<T, PAIR>(base, &p, &f0);
-        const bool act = p < R.end;
-        const PointIdx q = point_of(a.g, act ? p : R.begin);
-        if constexpr (PAIR) {
-            cpair acc[4];
-            if (act)
-                dwf_apply_flavour_pair_sp<false, IMASS>(acc, rj, a.g, q, f0, a.chif, a.diag,
-                                                        a.hpin, a.apbc != 0);
-            if (!have) {
-                bj = sqrt(sum_partials(a.part + nb, nb));
-                ibj = 1.0 / bj;
-                have = true;
-            }
-            if (!act) continue;
-            const Real ib = (Real)ibj;
-            // |vt|^2 is summed in FP64 from the first term: a pair's partial
-            // sum in FP32 made the FP32 force solves 7% longer (alpha~ and
-            // beta steer the recurrences)
-#pragma unroll
-            for (int d = 0; d < 4; d++) {
-                const cpair v = zscal(ib, acc[d]);
-                st_cpair(a.vt, (uint32_t)p + (uint32_t)a.g.cs * (uint32_t)(d + 4 * f0), v);
-                const double2 w0 = widen(cpair_pt(v, 0)), w1 = widen(cpair_pt(v, 1));
-                loc += w0.x * w0.x + w0.y * w0.y;
-                loc += w1.x * w1.x + w1.y * w1.y;
-            }
-        } else if constexpr (LATE) {
-            T acc[4];
-            if (act)
-                dwf_apply_flavour<false, IMASS>(acc, LdPlainT<T>{rj}, a.g, q, f0, a.chif, a.diag,
-                                                a.hpin, a.apbc != 0);
-            if (!have) {
-                bj = sqrt(sum_partials(a.part + nb, nb));
-                ibj = 1.0 / bj;
-                have = true;
-            }
-            if (!act) continue;
-            const Real ib = (Real)ibj;
-#pragma unroll
-            for (int d = 0; d < 4; d++) {
-                const T v = zscal(ib, acc[d]);   // apply_scaled's scaling
-                a.vt[p + a.g.cs * (d + 4 * f0)] = v;
-                const double2 w = widen(v);
-                loc += w.x * w.x + w.y * w.y;
-            }
-        } else {
-            if (!act) continue;
-            const Real ib = (Real)ibj;
-#pragma unroll
-            for (int f = f0; f < f0 + NF; f++) {
-                T acc[4];
-                apply_scaled<false, IMASS>(acc, rj, ib, a, q, f);
-#pragma unroll
-                for (int d = 0; d < 4; d++) {
-                    a.vt[p + a.g.cs * (d + 4 * f)] = acc[d];
-                    const double2 w = widen(acc[d]);
-                    loc += w.x * w.x + w.y * w.y;
-                }
-            }
-        }
-    }
-    if (!have) {   // a block whose range is empty
-        bj = sqrt(sum_partials(a.part + nb, nb));
-        ibj = 1.0 / bj;
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        ctl->it_md = j;
-        if (j > 1) {
-            a.h.beta[j] = bj;
-            a.h.invbeta[j] = ibj;
-        }
-    }
-    __shared__ double sh[kThreads / 32];
-    loc = block_sum<kThreads>(loc, sh);
-    if (threadIdx.x == 0) a.part[blockIdx.x] = loc;
-}
-
 // Scalar recurrences of qmrherm for iteration j (cheisdwf.f:666-715), one
-// lane per pole (the poles are independent), and the stopping test.
+// lane per pole (the poles are independent), and the stopping test.  d and
+// rho are the lane's pole state; returns the stop code (0: go on).
+struct PoleConst {       // what the scalar step reads of the control block
+    int npole, niter_cap;
+    double phimod, thresh, sigma;
+};
+__device__ __forceinline__ PoleConst pole_const(const LzCtl* ctl) {
+    const int k = threadIdx.x;
+    return PoleConst{ctl->npole, ctl->niter_cap, ctl->phimod, ctl->thresh,
+                     k < kMaxPoles ? ctl->sigma[k] : 0.0};
+}
 template <class T>
-__device__ __forceinline__ void pole_step(const LzArgsT<T>& a, int j, double at) {
+__device__ __forceinline__ int pole_step(const LzArgsT<T>& a, const PoleConst& pc, int j, double at,
+                                         double beta0, double& d, double& rho) {
     LzCtl* ctl = a.ctl;
     const int k = threadIdx.x;
-    const double beta0 = a.h.beta[j];
     if (k == 0) a.h.alphat[j] = at;
-    const int n = ctl->npole;
+    const int n = pc.npole;
     const int64_t H = kMaxIter + 2;
     double v = -1.0;
     if (k < n) {
-        const double alpha = __dadd_rn(at, ctl->sigma[k]);
-        double rho, mu = 0.0;
+        const double alpha = __dadd_rn(at, pc.sigma);
+        double mu = 0.0;
         if (j == 1) {
-            ctl->d[k] = alpha;
+            d = alpha;
             rho = __ddiv_rn(beta0, alpha);
         } else {
-            const double dm1 = ctl->d[k];
+            const double dm1 = d;
             mu = __ddiv_rn(beta0, dm1);
             const double dn = __dsub_rn(alpha, __dmul_rn(beta0, mu));
-            ctl->d[k] = dn;
-            rho = -__ddiv_rn(__dmul_rn(__dmul_rn(mu, dm1), ctl->rho[k]), dn);
+            d = dn;
+            rho = -__ddiv_rn(__dmul_rn(__dmul_rn(mu, dm1), rho), dn);
         }
-        ctl->rho[k] = rho;
         a.h.rho[k * H + j] = rho;
         a.h.mu[k * H + j] = mu;
-        v = fabs(__dmul_rn(ctl->phimod, rho));
+        v = fabs(__dmul_rn(pc.phimod, rho));
     }
     // rhomax as the sequential scan over the poles forms it: start from pole
     // 0 and take any larger value (a NaN in pole 0 stays, NaNs of the other
@@ -292,35 +164,42 @@ __device__ __forceinline__ void pole_step(const LzArgsT<T>& a, int j, double at)
     double m1 = k >= 1 ? v : -1.0;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m1 = fmax(m1, __shfl_xor_sync(0xffffffffu, m1, o));
-    if (k != 0) return;
     const double rhomax = (v0 != v0) ? v0 : fmax(v0, m1);
     int done = 0;
-    if (j >= 2 && rhomax < ctl->thresh) done = 1;
-    else if (j >= ctl->niter_cap) done = 2;
+    if (j >= 2 && rhomax < pc.thresh) done = 1;
+    else if (j >= pc.niter_cap) done = 2;
     if (!(rhomax == rhomax)) done = 3;   // NaN: stop, reported as non-finite
-    if (done) {
-        ctl->done = done;
+    if (done && k == 0) {
         ctl->m = j;
+        ctl->done = done;
         if (a.hflag) {
             *(volatile int*)a.hflag = done;
             __threadfence_system();
         }
     }
+    return done;
 }
 
 // alpha~_j from M(j)'s partials (the same sum, in the same order, as the
-// M^dagger blocks form), the pole recurrences and the stopping test.  One
-// block, launched on a side stream next to M^dagger(j): it overlaps that
-// kernel instead of lengthening either pass-1 kernel.  A converged solve
-// stops before M(j+1).
+// M^dagger blocks form), the pole recurrences and the stopping test, as a
+// one-block kernel beside M^dagger(j) on a side stream (row-staged pass 1).
+// A converged solve stops before M(j+1).
 template <class T>
 __global__ void __launch_bounds__(kThreads) k_lz_pole(LzArgsT<T> a, int nb) {
     LzCtl* ctl = a.ctl;
     if (block_stopped(ctl)) return;
     const int j = ctl->it_md;
-    const double at = sum_partials(a.part, nb);
+    const double at = sum_partials_any(a.part, nb);
     if (threadIdx.x == 0) ctl->it_m = j + 1;
-    if (threadIdx.x < 32) pole_step(a, j, at);
+    if (threadIdx.x < 32) {
+        const int k = threadIdx.x;
+        double d = k < kMaxPoles ? ctl->d[k] : 0.0, rho = k < kMaxPoles ? ctl->rho[k] : 0.0;
+        pole_step(a, pole_const(ctl), j, at, a.h.beta[j], d, rho);
+        if (k < ctl->npole) {
+            ctl->d[k] = d;
+            ctl->rho[k] = rho;
+        }
+    }
 }
 
 // r_{j+1} = x3 - alpha~ q_j - beta_j q_{j-1} at one point (cheisdwf.f:655)
@@ -337,21 +216,6 @@ __device__ __forceinline__ T three_term(const LzArgsT<T>& a, T x3, int64_t e, in
     return v;
 }
 
-// The same update for the two points of an FP32 pair (elements e, e+1) of
-// split-layout vectors, both points at once.
-__device__ __forceinline__ cpair three_term_sp(const LzArgsT<float2>& a, cpair x, uint32_t e,
-                                               int j, double alphat) {
-    const float2* rj = ring(a, j);
-    const float2* rjm = ring(a, j - 1);
-    const float ib = (float)a.h.invbeta[j], at = (float)alphat, bj = (float)a.h.beta[j];
-    cpair v = zsub(x, zscal(at, zscal(ib, ld_cpair(rj, e))));
-    if (j > 1) {
-        const float ibm = (float)a.h.invbeta[j - 1];
-        v = zsub(v, zscal(bj, zscal(ibm, ld_cpair(rjm, e))));
-    }
-    return v;
-}
-
 // Force solves with a wall store: element e of r_{j+1} at point (s, site),
 // component c, also goes to the wall store when s is a wall.
 template <class T>
@@ -364,85 +228,303 @@ __device__ __forceinline__ void wall_put(const LzArgsT<T>& a, int j1, int s, int
     a.wbasis[(int64_t)j1 * 8 * cs2 + (s == 0 ? 0 : 1) + 2 * (int64_t)site + cs2 * c] = v;
 }
 
-// ---- pass 1, kernel 2: r_{j+1} = M^dagger vt - alpha~ q_j - beta_j q_{j-1} ---
-// alpha~_j is the sum of M(j)'s partials, formed by every block.
-template <class T, int IMASS, bool PAIR, bool WALLS, int OCC>
-__global__ void __launch_bounds__(kThreads, OCC) k_lz1_Md(LzArgsT<T> a) {
-    typedef LzShape<T, PAIR> S;
-    constexpr int NF = S::split ? 1 : 2;
-    // alpha~_j, as beta_j in k_lz1_M, is summed after the first pass's
-    // stencil (one flavour a thread)
-    constexpr bool LATE = NF == 1;
-    LzCtl* ctl = a.ctl;
-    if (block_stopped(ctl)) return;
-    const int j = ctl->it_md;
-    const int nb = gridDim.x;
-    bool have = !LATE;
-    double at = LATE ? 0.0 : sum_partials(a.part, nb);
-    T* rn = ring(a, j + 1);
-    const PtRange R = block_range(a.g.npts);
-    double loc = 0.0;
-#pragma unroll 1
-    for (int64_t base = R.begin; base < R.end; base += S::unit) {
-        int64_t p;
-        int f0;
-        lz_lane<T, PAIR>(base, &p, &f0);
-        const bool act = p < R.end;
-        const PointIdx q = point_of(a.g, act ? p : R.begin);
-        if constexpr (PAIR) {
-            cpair acc[4];
-            if (act)
-                dwf_apply_flavour_pair_sp<true, IMASS>(acc, a.vt, a.g, q, f0, a.chif, a.diag,
-                                                       a.hpin, a.apbc != 0);
-            if (!have) {
-                at = sum_partials(a.part, nb);
-                have = true;
-            }
-            if (!act) continue;
-#pragma unroll
-            for (int d = 0; d < 4; d++) {
-                const uint32_t e = (uint32_t)p + (uint32_t)a.g.cs * (uint32_t)(d + 4 * f0);
-                const cpair v = three_term_sp(a, acc[d], e, j, at);
-                st_cpair(rn, e, v);
-                const float2 v0 = cpair_pt(v, 0), v1 = cpair_pt(v, 1);
-                if (WALLS) {
-                    wall_put(a, j + 1, q.s, q.site, d + 4 * f0, v0);
-                    wall_put(a, j + 1, q.s + 1, q.site, d + 4 * f0, v1);
-                }
-                const double2 w0 = widen(v0), w1 = widen(v1);
-                loc += w0.x * w0.x + w0.y * w0.y;
-                loc += w1.x * w1.x + w1.y * w1.y;
-            }
-        } else {
-            T acc[NF][4];
-            if (LATE && act)
-                dwf_apply_flavour<true, IMASS>(acc[0], LdPlainT<T>{a.vt}, a.g, q, f0, a.chif,
-                                               a.diag, a.hpin, a.apbc != 0);
-            if (!have) {
-                at = sum_partials(a.part, nb);
-                have = true;
-            }
-            if (!act) continue;
-#pragma unroll
-            for (int f = f0; f < f0 + NF; f++) {
-                if (!LATE)
-                    dwf_apply_flavour<true, IMASS>(acc[f - f0], LdPlainT<T>{a.vt}, a.g, q, f,
-                                                   a.chif, a.diag, a.hpin, a.apbc != 0);
-#pragma unroll
-                for (int d = 0; d < 4; d++) {
-                    const int64_t e = p + a.g.cs * (d + 4 * f);
-                    const T v = three_term(a, acc[f - f0][d], e, j, at);
-                    rn[e] = v;
-                    if (WALLS) wall_put(a, j + 1, q.s, q.site, d + 4 * f, v);
-                    const double2 w = widen(v);
-                    loc += w.x * w.x + w.y * w.y;
-                }
-            }
+// ---- pass 1 on planes ----------------------------------------------------------
+// Two kernels an iteration: vt = M r_j with |vt|^2, and r_{j+1} =
+// (1/beta_j) M^dagger vt - alpha~_j q_j - beta_j q_{j-1} with |r_{j+1}|^2, where
+// q_j = r_j/beta_j and alpha~_j = |vt|^2/beta_j^2.  Leaving vt unscaled keeps
+// beta_j, a sum over the previous kernel's blocks, out of M.  Block b (of nb
+// workers) takes the items b, b + nb, ... and leaves its |.|^2 partial in
+// part[b] (M) or part[nb + b] (M^dagger); one more block a kernel does the
+// part[b] (M) or part[nb + b] (M^dagger); one more block a kernel does the
+// scalar work.
+//
+// Kernels k = 0..15 of M and M^dagger, after k_lz_tick, are captured as a
+// graph: iteration j = ctl->base + k + 1.  Programmatic dependent launch lets
+// a kernel's blocks start while the previous kernel drains: they work out
+// their item and read base (constant during a replay), then wait for the
+// previous kernel's end.  A kernel lets its dependents start only after its
+// own wait, so base has been set before any other kernel of the replay reads
+// it.
+__device__ __forceinline__ int pass1_begin(const LzCtl* ctl, int k, bool after_tick) {
+    int base = 0;
+    if (!after_tick) base = *(volatile const int*)&ctl->base;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (after_tick) base = *(volatile const int*)&ctl->base;
+    return base + k + 1;
+}
+__global__ void k_lz_tick(LzCtl* ctl, int chunk) {
+    ctl->base = ctl->next;
+    ctl->next += chunk;
+}
+
+// The sum of a kernel's nb partials and the recurrence's scalars, in two
+// steps: asynchronous copies into shared memory when the kernel starts, in
+// front of its stencil loads and holding no registers, and the sum, in one
+// order for all blocks, where it is first needed, after the first unit.
+// Loaded and summed in one step there, the L2 round trip made the kernel
+// about 2 us longer (24^3x24): all blocks run one wave and wait together.
+// Dynamic shared memory: nb + 3 doubles.
+extern __shared__ double lz_smem[];
+__device__ __forceinline__ void cp_async8(double* dst, const double* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                     static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+                 "l"(src)
+                 : "memory");
+}
+struct PartSum {
+    __device__ __forceinline__ static void start(const double* part, int n, const double* x0,
+                                                 const double* x1, const double* x2) {
+        for (int i = (int)threadIdx.x; i < n; i += (int)blockDim.x) cp_async8(lz_smem + i, part + i);
+        if (threadIdx.x == 0 && x0) {
+            cp_async8(lz_smem + n, x0);
+            cp_async8(lz_smem + n + 1, x1);
+            cp_async8(lz_smem + n + 2, x2);
         }
     }
-    __shared__ double sh[kThreads / 32];
-    loc = block_sum<kThreads>(loc, sh);
-    if (threadIdx.x == 0) a.part[nb + blockIdx.x] = loc;
+    __device__ __forceinline__ static double total(int n) {
+        __shared__ double sh[32];
+        __shared__ double res;
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+        double s = 0.0;
+        for (int i = (int)threadIdx.x; i < n; i += (int)blockDim.x) s += lz_smem[i];
+        s = block_sum_any(s, sh);
+        if (threadIdx.x == 0) res = s;
+        __syncthreads();
+        return res;
+    }
+};
+// alpha~_j from |vt|^2 = |M r_j|^2
+__device__ __forceinline__ double alpha_of(double s, double ibj) { return s * ibj * ibj; }
+
+template <class T>
+struct PlaneM {
+    typedef typename unit_of<T>::type V;
+    V* vt;
+    int done;              // the solve has stopped: looked at after the first unit
+    double loc;
+    __device__ __forceinline__ bool operator()(V acc[4], int64_t e, int64_t cst, uint32_t o,
+                                               bool act, int, uint32_t) {
+        if (done) return false;
+        if (!act) return true;
+        // |vt|^2 is summed in FP64 from the first term: a pair's partial sum
+        // in FP32 made the FP32 force solves 7% longer (alpha~ and beta steer
+        // the recurrences)
+#pragma unroll
+        for (int d = 0; d < 4; d++) {
+            st_unit(unit_at(vt + e + d * cst, o), acc[d]);
+            loc += unit_norm2(acc[d]);
+        }
+        return true;
+    }
+};
+
+// Element of a unit that lies on wall sw (0: s = 1, 1: s = Ls).
+__device__ __forceinline__ double2 unit_wall(double2 v, int, int) { return v; }
+__device__ __forceinline__ float2 unit_wall(const cpair& v, int sw, int Ls) {
+    return cpair_pt(v, sw == 0 ? 0 : (Ls & 1 ? 0 : 1));
+}
+
+template <class T, bool WALLS>
+struct PlaneMd {
+    typedef typename unit_of<T>::type V;
+    typedef typename real_of<T>::type Real;
+    const LzArgsT<T>& a;
+    const V *rj, *rjm;
+    V* rn;
+    int nb, j, done;
+    bool have;
+    double loc;
+    Real c0, c1, c2;                  // 1/beta_j, -alpha~/beta_j, -beta_j/beta_{j-1}
+    __device__ __forceinline__ void scalars(double at, double bj, double ibj, double ibm) {
+        c0 = (Real)ibj;
+        c1 = (Real)(-at * ibj);
+        c2 = (Real)(-bj * ibm);
+        have = true;
+    }
+    __device__ __forceinline__ void ready() {
+        if (have) return;
+        const double s = PartSum::total(nb), ibj = lz_smem[nb + 1];
+        scalars(alpha_of(s, ibj), lz_smem[nb], ibj, lz_smem[nb + 2]);
+    }
+    __device__ __forceinline__ bool operator()(V acc[4], int64_t e, int64_t cst, uint32_t o,
+                                               bool act, int u, uint32_t site) {
+        if (done) return false;
+        // FP64: q_j and q_{j-1} are loaded in front of the sum's block barriers.
+        // FP32: behind them; the stencil of a pair leaves no registers for
+        // them (100 bytes of spills; 24^3x24 M^dagger 2.5 us longer, against
+        // 1.9 us shorter for FP64 20^3x20)
+        constexpr bool EARLY = std::is_same<T, double2>::value;
+        V q[4], qm[4];
+        if (EARLY) {
+#pragma unroll
+            for (int d = 0; d < 4; d++) {
+                q[d] = ld_unit(unit_at(rj + e + d * cst, o));
+                qm[d] = j > 1 ? ld_unit(unit_at(rjm + e + d * cst, o)) : V{};
+            }
+        }
+        ready();
+        if (!act) return true;
+#pragma unroll
+        for (int d = 0; d < 4; d++) {
+            // r_{j+1} = x3 - alpha~ q_j - beta_j q_{j-1} (cheisdwf.f:655)
+            if (!EARLY) {
+                q[d] = ld_unit(unit_at(rj + e + d * cst, o));
+                qm[d] = j > 1 ? ld_unit(unit_at(rjm + e + d * cst, o)) : V{};
+            }
+            V v = zaxpy(c1, q[d], zscal2(c0, acc[d]));
+            if (j > 1) v = zaxpy(c2, qm[d], v);
+            st_unit(unit_at(rn + e + d * cst, o), v);
+            loc += unit_norm2(v);
+            if (WALLS && j + 1 < a.wcap && (u == 0 || u == a.pp.U - 1)) {
+                // the two wall slices of r_{j+1}, element (wall, site, c)
+                const int64_t cs2 = 2 * (int64_t)a.g.kvol;
+                const int c = (int)(e >= 4 * cst ? 4 : 0) + d;
+                T* w = a.wbasis + (int64_t)(j + 1) * 8 * cs2 + 2 * (int64_t)site + cs2 * c;
+                if (u == 0) w[0] = unit_wall(v, 0, a.g.Ls);
+                if (u == a.pp.U - 1) w[1] = unit_wall(v, 1, a.g.Ls);
+            }
+        }
+        return true;
+    }
+};
+
+template <class T, int IMASS>
+__device__ __forceinline__ void plane_phase_M(const LzArgsT<T>& a, const PlaneThread& th,
+                                              int b, int nb, PlaneM<T>& epi, const T* rj) {
+    typedef typename unit_of<T>::type V;
+    typedef typename real_of<T>::type Real;
+    for (uint32_t it = (uint32_t)b; it < a.pp.nitem && !epi.done; it += (uint32_t)nb)
+        plane_item<false, IMASS>(reinterpret_cast<const V*>(rj), a.pp, th, it, a.chif, (Real)a.diag,
+                                 (Real)a.hpin, a.apbc != 0, epi);
+}
+template <class T, int IMASS, bool WALLS>
+__device__ __forceinline__ void plane_phase_Md(const LzArgsT<T>& a, const PlaneThread& th,
+                                               int b, int nb, PlaneMd<T, WALLS>& epi) {
+    typedef typename unit_of<T>::type V;
+    typedef typename real_of<T>::type Real;
+    for (uint32_t it = (uint32_t)b; it < a.pp.nitem && !epi.done; it += (uint32_t)nb)
+        plane_item<true, IMASS>(reinterpret_cast<const V*>(a.vt), a.pp, th, it, a.chif,
+                                (Real)a.diag, (Real)a.hpin, a.apbc != 0, epi);
+}
+
+// Pass 1 (REGEN false, k0 the place in the replay): iteration j unless the
+// solve has stopped.  Block 0 is
+// the scalar block: it forms beta_j from M^dagger(j-1)'s partials (beta_1
+// comes from the source).  The regenerating pass 2 (REGEN true, k0 = j) takes
+// every scalar from the history and has no scalar block.
+template <class T, int IMASS, bool REGEN>
+__global__ void __maxnreg__(kPlaneRegs) k_lz1_M(LzArgsT<T> a, int k0) {
+    typedef typename unit_of<T>::type V;
+    LzCtl* ctl = a.ctl;
+    constexpr int X = REGEN ? 0 : 1;
+    const int nb = (int)gridDim.x - X, b = (int)blockIdx.x - X;
+    const PlaneThread th = plane_thread(a.pp);
+    const int j = REGEN ? k0 : pass1_begin(ctl, k0, k0 == 0);
+    PlaneM<T> em{reinterpret_cast<V*>(a.vt), REGEN ? 0 : *(volatile int*)&ctl->done, 0.0};
+    if (!REGEN && b < 0) {
+        if (em.done || j == 1) return;
+        PartSum::start(a.part + nb, nb, nullptr, nullptr, nullptr);
+        const double s = PartSum::total(nb);
+        if (threadIdx.x == 0) {
+            const double beta = sqrt(s);
+            a.h.beta[j] = beta;
+            a.h.invbeta[j] = 1.0 / beta;
+        }
+        return;
+    }
+    plane_phase_M<T, IMASS>(a, th, b, nb, em, ring(a, j));
+    if (REGEN || em.done) return;
+    __shared__ double sh[32];
+    const double loc = block_sum_any(em.loc, sh);
+    if (threadIdx.x == 0) a.part[b] = loc;
+}
+
+// Block 0 is the scalar step of iteration j (alpha~_j, the pole recurrences,
+// the stopping test).  The step, two L2 round trips and two dependent
+// divisions, ends long before the workers do, and the next M sees its stop
+// flag.  (As phases of one cooperative kernel with grid barriers the two
+// kernels were slower: a barrier and the sum after it take 1.9 us at 144
+// blocks and 3.8 us at 577, a kernel boundary about 1 us.)
+template <class T, int IMASS, bool WALLS, bool REGEN>
+__global__ void __maxnreg__(kPlaneRegs) k_lz1_Md(LzArgsT<T> a, int k0) {
+    typedef typename unit_of<T>::type V;
+    LzCtl* ctl = a.ctl;
+    constexpr int X = REGEN ? 0 : 1;
+    const int nb = (int)gridDim.x - X, b = (int)blockIdx.x - X;
+    const PlaneThread th = plane_thread(a.pp);
+    const int j = REGEN ? k0 : pass1_begin(ctl, k0, false);
+    // M(j) ran if the solve had not stopped before iteration j: m is set with
+    // done, by the scalar block of M^dagger(m)
+    const int m = REGEN ? j : *(volatile int*)&ctl->m;
+    // invbeta[0] is 0, so c2 is 0 for j = 1
+    if (!REGEN)
+        PartSum::start(a.part, nb, a.h.beta + j, a.h.invbeta + j, a.h.invbeta + j - 1);
+    PlaneMd<T, WALLS> ed{a, reinterpret_cast<const V*>(ring(a, j)),
+                         reinterpret_cast<const V*>(ring(a, j - 1)),
+                         reinterpret_cast<V*>(ring(a, j + 1)), nb, j, m != 0 && m < j, false, 0.0};
+    if (!REGEN && b < 0) {
+        if (ed.done) return;
+        const int k = threadIdx.x;
+        double d = 0.0, rho = 0.0;
+        if (k < kMaxPoles) {
+            d = ctl->d[k];
+            rho = ctl->rho[k];
+        }
+        const PoleConst pc = pole_const(ctl);
+        const double s = PartSum::total(nb);
+        if (k < 32) {
+            pole_step(a, pc, j, alpha_of(s, lz_smem[nb + 1]), lz_smem[nb], d, rho);
+            if (k < pc.npole) {
+                ctl->d[k] = d;
+                ctl->rho[k] = rho;
+            }
+        }
+        return;
+    }
+    if (REGEN)
+        ed.scalars(a.h.alphat[j], a.h.beta[j], a.h.invbeta[j], j > 1 ? a.h.invbeta[j - 1] : 0.0);
+    plane_phase_Md<T, IMASS, WALLS>(a, th, b, nb, ed);
+    if (REGEN || ed.done) return;
+    __shared__ double sh[32];
+    const double loc = block_sum_any(ed.loc, sh);
+    if (threadIdx.x == 0) a.part[nb + b] = loc;
+}
+
+// Regenerating pass 2: x += c_j q_j (iflag 0), or y_kj q_j on the two wall
+// slices of every pole's x_k (iflag 1), from r_j in planes.
+template <class T, int IFLAG>
+__global__ void __launch_bounds__(kThreads) k_lzp_acc(LzArgsT<T> a, int j) {
+    typedef typename real_of<T>::type Real;
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const T* rj = ring(a, j);
+    const Real ib = (Real)a.h.invbeta[j];
+    if (IFLAG == 0) {
+        if (t >= a.g.kferm) return;
+        const int64_t cs = t / a.g.kvol, site = t - cs * a.g.kvol;
+        const int c = (int)(cs / a.g.Ls), s = (int)(cs - (int64_t)c * a.g.Ls);
+        const double2 q = widen(zscal(ib, vget(a, rj, c, s, site)));
+        const double cj = a.h.c[j];
+        double2* x = a.x + s + (int64_t)a.g.Ls * site + a.g.cs * c;
+        x->x += cj * q.x;
+        x->y += cj * q.y;
+    } else {
+        const int64_t cs2 = 2 * (int64_t)a.g.kvol, kf2 = 8 * cs2;
+        if (t >= kf2) return;
+        const int c = (int)(t / cs2);
+        const int64_t r = t - c * cs2;
+        const double2 q =
+            widen(zscal(ib, vget(a, rj, c, (r & 1) ? a.g.Ls - 1 : 0, r >> 1)));
+        const int64_t H = kMaxIter + 2;
+        for (int k = 0; k < a.npole; k++) {
+            const double y = a.h.y[k * H + j];
+            double2 xv = a.xw[k * kf2 + t];
+            xv.x += y * q.x;
+            xv.y += y * q.y;
+            a.xw[k * kf2 + t] = xv;
+        }
+    }
 }
 
 // ---- pass 1 on staged rows ---------------------------------------------------
@@ -602,9 +684,9 @@ __global__ void __maxnreg__(kRowRegs) k_lz1_Md_rows(LzArgsT<T> a) {
     }
 }
 
-// ---- pass 2: regenerate q_j and accumulate --------------------------------
-// One block pass per block (grid lz_direct_blocks).  The solution update of
-// one element of x (iflag 0) or of the wall fields (iflag 1).
+// ---- pass 2 on the ABI's layout: regenerate q_j and accumulate ---------------
+// (row-staged solves).  One pass per block; the solution update of one
+// element of x (iflag 0) or of the wall fields (iflag 1).
 template <class T, int IFLAG>
 __device__ __forceinline__ void lz2_accumulate(const LzArgsT<T>& a, int j, const T* rj,
                                                typename real_of<T>::type ib, int64_t p,
@@ -613,7 +695,7 @@ __device__ __forceinline__ void lz2_accumulate(const LzArgsT<T>& a, int j, const
         const double cj = a.h.c[j];
         for (int c = c0; c < c0 + nc; c++) {
             const int64_t e = p + a.g.cs * c;
-            const double2 qj = widen(zscal(ib, vget(a, rj, e)));
+            const double2 qj = widen(zscal(ib, rj[e]));
             double2 xv = a.x[e];
             xv.x += cj * qj.x;
             xv.y += cj * qj.y;
@@ -629,7 +711,7 @@ __device__ __forceinline__ void lz2_accumulate(const LzArgsT<T>& a, int j, const
         double2 qv[8];
 #pragma unroll
         for (int c = 0; c < 8; c++)
-            if (c < nc) qv[c] = widen(zscal(ib, vget(a, rj, p + a.g.cs * (c + c0))));
+            if (c < nc) qv[c] = widen(zscal(ib, rj[p + a.g.cs * (c + c0)]));
         const int64_t base = sw + 2 * (int64_t)q.site + cs2 * c0;
         for (int k = 0; k < n; k++) {
             const double y = a.h.y[k * H + j];
@@ -646,103 +728,58 @@ __device__ __forceinline__ void lz2_accumulate(const LzArgsT<T>& a, int j, const
     }
 }
 
-template <class T, int IMASS, int IFLAG, bool PAIR>
-__global__ void __launch_bounds__(kThreads, (LzShape<T, PAIR>::min_blocks))
+template <class T, int IMASS, int IFLAG>
+__global__ void __launch_bounds__(kThreads, LzShape<T>::min_blocks)
     k_lz2_M(LzArgsT<T> a, int j, int apply) {
     typedef typename real_of<T>::type Real;
-    typedef LzShape<T, PAIR> S;
+    typedef LzShape<T> S;
     constexpr int NF = S::split ? 1 : 2;
     int64_t p;
     int f0;
-    lz_lane<T, PAIR>((int64_t)blockIdx.x * S::unit, &p, &f0);
+    lz_lane<T>((int64_t)blockIdx.x * S::unit, &p, &f0);
     if (p >= a.g.npts) return;
     const PointIdx q = point_of(a.g, p);
     const Real ib = (Real)a.h.invbeta[j];
     const T* rj = ring(a, j);
-    if constexpr (PAIR) {
-        if (apply) {
-            cpair acc[4];
-            dwf_apply_flavour_pair_sp<false, IMASS>(acc, rj, a.g, q, f0, a.chif, a.diag, a.hpin,
-                                                    a.apbc != 0);
-#pragma unroll
-            for (int d = 0; d < 4; d++)
-                st_cpair(a.vt, (uint32_t)(p + a.g.cs * (d + 4 * f0)), zscal(ib, acc[d]));
-        }
-        lz2_accumulate<T, IFLAG>(a, j, rj, ib, p, q, 4 * f0, 4);
-        const PointIdx q1 = point_of(a.g, p + 1);
-        lz2_accumulate<T, IFLAG>(a, j, rj, ib, p + 1, q1, 4 * f0, 4);
-    } else {
-        if (apply) {
-#pragma unroll
-            for (int f = f0; f < f0 + NF; f++) {
-                T acc[4];
-                apply_scaled<false, IMASS>(acc, rj, ib, a, q, f);
-#pragma unroll
-                for (int d = 0; d < 4; d++) a.vt[p + a.g.cs * (d + 4 * f)] = acc[d];
-            }
-        }
-        lz2_accumulate<T, IFLAG>(a, j, rj, ib, p, q, 4 * f0, 4 * NF);
-    }
-}
-
-template <class T, int IMASS, bool PAIR>
-__global__ void __launch_bounds__(kThreads, (LzShape<T, PAIR>::min_blocks))
-    k_lz2_Md(LzArgsT<T> a, int j) {
-    typedef LzShape<T, PAIR> S;
-    constexpr int NF = S::split ? 1 : 2;
-    int64_t p;
-    int f0;
-    lz_lane<T, PAIR>((int64_t)blockIdx.x * S::unit, &p, &f0);
-    if (p >= a.g.npts) return;
-    const PointIdx q = point_of(a.g, p);
-    T* rn = ring(a, j + 1);
-    if constexpr (PAIR) {
-        cpair acc[4];
-        dwf_apply_flavour_pair_sp<true, IMASS>(acc, a.vt, a.g, q, f0, a.chif, a.diag, a.hpin,
-                                               a.apbc != 0);
-#pragma unroll
-        for (int d = 0; d < 4; d++) {
-            const uint32_t e = (uint32_t)(p + a.g.cs * (d + 4 * f0));
-            st_cpair(rn, e, three_term_sp(a, acc[d], e, j, a.h.alphat[j]));
-        }
-    } else {
+    if (apply) {
 #pragma unroll
         for (int f = f0; f < f0 + NF; f++) {
             T acc[4];
-            dwf_apply_flavour<true, IMASS>(acc, LdPlainT<T>{a.vt}, a.g, q, f, a.chif, a.diag,
-                                           a.hpin, a.apbc != 0);
+            apply_scaled<false, IMASS>(acc, rj, ib, a, q, f);
 #pragma unroll
-            for (int d = 0; d < 4; d++) {
-                const int64_t e = p + a.g.cs * (d + 4 * f);
-                rn[e] = three_term(a, acc[d], e, j, a.h.alphat[j]);
-            }
+            for (int d = 0; d < 4; d++) a.vt[p + a.g.cs * (d + 4 * f)] = acc[d];
+        }
+    }
+    lz2_accumulate<T, IFLAG>(a, j, rj, ib, p, q, 4 * f0, 4 * NF);
+}
+
+template <class T, int IMASS>
+__global__ void __launch_bounds__(kThreads, LzShape<T>::min_blocks)
+    k_lz2_Md(LzArgsT<T> a, int j) {
+    typedef LzShape<T> S;
+    constexpr int NF = S::split ? 1 : 2;
+    int64_t p;
+    int f0;
+    lz_lane<T>((int64_t)blockIdx.x * S::unit, &p, &f0);
+    if (p >= a.g.npts) return;
+    const PointIdx q = point_of(a.g, p);
+    T* rn = ring(a, j + 1);
+#pragma unroll
+    for (int f = f0; f < f0 + NF; f++) {
+        T acc[4];
+        dwf_apply_flavour<true, IMASS>(acc, LdPlainT<T>{a.vt}, a.g, q, f, a.chif, a.diag, a.hpin,
+                                       a.apbc != 0);
+#pragma unroll
+        for (int d = 0; d < 4; d++) {
+            const int64_t e = p + a.g.cs * (d + 4 * f);
+            rn[e] = three_term(a, acc[d], e, j, a.h.alphat[j]);
         }
     }
 }
 
-template <class T, bool PAIR = false>
+template <class T>
 static unsigned lz_direct_blocks(int64_t npts) {
-    return (unsigned)((npts + LzShape<T, PAIR>::unit - 1) / LzShape<T, PAIR>::unit);
-}
-
-// Persistent pass-1 grid: the resident blocks of both pass-1 kernels on all
-// SMs, at most one block pass per block.
-template <class T, int IMASS, bool PAIR, int OCC>
-static unsigned lz_pass1_blocks(int64_t npts) {
-    int dev = 0, nsm = 0, b1 = 0, b2 = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, k_lz1_M<T, IMASS, PAIR, OCC>, kThreads, 0);
-    int b3 = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b2, k_lz1_Md<T, IMASS, PAIR, false, OCC>,
-                                                  kThreads, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b3, k_lz1_Md<T, IMASS, PAIR, true, OCC>,
-                                                  kThreads, 0);
-    if (b3 < b2) b2 = b3;
-    int64_t nb = (int64_t)nsm * (b1 < b2 ? b1 : b2);
-    const int64_t direct = lz_direct_blocks<T, PAIR>(npts);
-    if (nb < 1 || nb > direct) nb = direct;
-    return (unsigned)nb;
+    return (unsigned)((npts + LzShape<T>::unit - 1) / LzShape<T>::unit);
 }
 
 // ---- between the passes: y_kj and c_j -------------------------------------
@@ -788,26 +825,44 @@ __global__ void __launch_bounds__(kThreads) k_lz_coeffs(LzCtl* ctl, LzHist h, in
     }
 }
 
-// r_1 = Phi in the vector precision; partial sums of |r_1|^2
+// r_1 = Phi in the vector precision and layout; partial sums of |r_1|^2.  In
+// planes a thread takes one unit: its reads of Phi are Ls elements apart from
+// its neighbours', once per solve.
 template <class T>
-__global__ void k_lz_source(T* __restrict__ r1, const double2* __restrict__ phi, int64_t n,
-                            double* __restrict__ part, int pl) {
+__device__ __forceinline__ T narrow(double2 v) {
+    return zmake<T>((typename real_of<T>::type)v.x, (typename real_of<T>::type)v.y);
+}
+template <class T>
+__global__ void k_lz_source(LzArgsT<T> a, T* __restrict__ r1, const double2* __restrict__ phi,
+                            double* __restrict__ part) {
     __shared__ double sh[kThreads / 32];
+    constexpr bool F32 = std::is_same<T, float2>::value;
     double s = 0.0;
+    const int64_t n = a.pl ? 8 * (int64_t)a.pp.U * a.g.kvol : a.g.kferm;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
-        const double2 v = phi[i];
-        T t;
-        t.x = (typename real_of<T>::type)v.x;
-        t.y = (typename real_of<T>::type)v.y;
-        if constexpr (std::is_same<T, float2>::value) {
-            if (pl) sp_put(r1, i, t);
-            else r1[i] = t;
-        } else {
+        if (!a.pl) {
+            const T t = narrow<T>(phi[i]);
             r1[i] = t;
+            const double2 w = widen(t);
+            s += w.x * w.x + w.y * w.y;
+            continue;
         }
-        const double2 w = widen(t);
-        s += w.x * w.x + w.y * w.y;
+        const int64_t cu = i / a.g.kvol, site = i - cu * a.g.kvol;
+        const int c = (int)(cu / a.pp.U), u = (int)(cu - (int64_t)c * a.pp.U);
+        const double2* src = phi + (int64_t)a.g.Ls * site + a.g.cs * c;
+        if constexpr (F32) {
+            const float2 z = make_float2(0.0f, 0.0f);
+            const float2 p0 = narrow<T>(src[2 * u]);
+            const float2 p1 = 2 * u + 1 < a.g.Ls ? narrow<T>(src[2 * u + 1]) : z;
+            const cpair v{make_float2(p0.x, p1.x), make_float2(p0.y, p1.y)};
+            st_unit(reinterpret_cast<cpair*>(r1) + i, v);
+            s += unit_norm2(v);
+        } else {
+            const double2 v = src[u];
+            r1[i] = v;
+            s += v.x * v.x + v.y * v.y;
+        }
     }
     s = block_sum<kThreads>(s, sh);
     if (threadIdx.x == 0) part[blockIdx.x] = s;
@@ -822,38 +877,66 @@ __global__ void k_lz_init(LzCtl* ctl, LzHist h, const double* part, int nb) {
         const double b = sqrt(s);
         h.beta[1] = b;
         h.invbeta[1] = 1.0 / b;
+        h.invbeta[0] = 0.0;
         ctl->phimod = b;
     }
 }
 
-template <class T, int IMASS, bool PAIR, int OCC>
-static void launch_pass1_occ(const LzArgsT<T>& a, unsigned nb, cudaStream_t st,
-                             const LzSide& side, KernelTimer* tm) {
-    // algorithmic bytes: M reads q, writes vt; M^dagger reads vt, r_j, r_{j-1}
-    // and writes r_{j+1}; both read chi as REAL*4
+// Pass 1 on planes.  Algorithmic bytes: M reads q, writes vt; M^dagger reads
+// vt, r_j, r_{j-1} and writes r_{j+1}; both read chi as REAL*4.
+// dep: programmatic dependent launch (see pass1_begin).
+template <class... P, class... A>
+static void launch_dep(bool dep, void (*k)(P...), unsigned nb, unsigned nt, cudaStream_t st,
+                       A... args) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(nb + 1);                        // nb workers and the scalar block
+    c.blockDim = dim3(nt);
+    c.dynamicSmemBytes = sizeof(double) * (nb + 3);
+    c.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = dep ? 1 : 0;
+    cudaLaunchKernelEx(&c, k, P(args)...);
+}
+template <class T, int IMASS>
+static void launch_pass1_planes(const LzArgsT<T>& a, unsigned nb, int k0, int chunk, cudaStream_t st,
+                                KernelTimer* tm) {
     const double V = (double)a.g.kferm * sizeof(T), chi = 12.0 * a.g.kvol;
+    const unsigned nt = (unsigned)a.pp.threads;
+    const bool dep = !tm || !tm->enabled;   // events need the kernel's own start
+    if (k0 == 0) k_lz_tick<<<1, 1, 0, st>>>(a.ctl, chunk);
     if (tm) tm->begin(timer_class<T>(0), st, 2 * V + chi);
-    k_lz1_M<T, IMASS, PAIR, OCC><<<nb, kThreads, 0, st>>>(a);
+    launch_dep(dep, k_lz1_M<T, IMASS, false>, nb, nt, st, a, k0);
     if (tm) tm->end(st);
-    // the scalar step of iteration j on the side stream, beside M^dagger(j)
-    cudaEventRecord(side.fork, st);
-    cudaStreamWaitEvent(side.stream, side.fork, 0);
-    k_lz_pole<T><<<1, kThreads, 0, side.stream>>>(a, (int)nb);
-    cudaEventRecord(side.join, side.stream);
     if (tm) tm->begin(timer_class<T>(1), st, 4 * V + chi);
-    if (a.wcap > 0) k_lz1_Md<T, IMASS, PAIR, true, OCC><<<nb, kThreads, 0, st>>>(a);
-    else k_lz1_Md<T, IMASS, PAIR, false, OCC><<<nb, kThreads, 0, st>>>(a);
+    if (a.wcap > 0) launch_dep(dep, k_lz1_Md<T, IMASS, true, false>, nb, nt, st, a, k0);
+    else launch_dep(dep, k_lz1_Md<T, IMASS, false, false>, nb, nt, st, a, k0);
     if (tm) tm->end(st);
-    cudaStreamWaitEvent(st, side.join, 0);
 }
 
-// The point-gather pass 1 at the register budget the autotuner chose: 3
-// blocks of 256 a SM (80 registers a thread) or 4 (64 registers).
-template <class T, int IMASS, bool PAIR>
-static void launch_pass1(const LzArgsT<T>& a, unsigned nb, cudaStream_t st, const LzSide& side,
-                         KernelTimer* tm) {
-    if (a.occ == 4) launch_pass1_occ<T, IMASS, PAIR, 4>(a, nb, st, side, tm);
-    else launch_pass1_occ<T, IMASS, PAIR, 3>(a, nb, st, side, tm);
+// Worker blocks of pass 1: the blocks of both kernels that are resident at
+// once (one fewer: the scalar block), at most one per work item.
+template <class T, int IMASS>
+static unsigned pass1_workers(const PlanePlan& pp, int nsm) {
+    const void* k[3] = {(const void*)k_lz1_M<T, IMASS, false>,
+                        (const void*)k_lz1_Md<T, IMASS, false, false>,
+                        (const void*)k_lz1_Md<T, IMASS, true, false>};
+    int64_t res = kMaxPartBlocks;
+    for (const void* f : k) {
+        int per_sm = 0;
+        const int64_t most = (int64_t)(24 / (pp.threads / 32)) * nsm;   // by registers
+        const size_t smem = sizeof(double) * (size_t)((most < res ? most : res) + 3);
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, pp.threads, smem) !=
+            cudaSuccess) {
+            cudaGetLastError();
+            return 0;
+        }
+        const int64_t r = (int64_t)per_sm * nsm - 1;
+        if (r < res) res = r;
+    }
+    return res < 1 ? 0 : (unsigned)(res < (int64_t)pp.nitem ? res : (int64_t)pp.nitem);
 }
 
 // Row-staged pass 1 (same protocol: M, the scalar step on the side stream,
@@ -877,8 +960,7 @@ static void launch_pass1_rows_ppt(const LzArgsT<T>& a, unsigned nb, cudaStream_t
     cudaStreamWaitEvent(st, side.join, 0);
 }
 
-// One point a thread: the FP64 solves and odd-Ls FP32 solves (even-Ls FP32
-// vectors are in the split layout, which only the point-gather kernels read).
+// One point a thread: the FP64 solves and odd-Ls FP32 solves.
 template <class T, int IMASS>
 static void launch_pass1_rows(const LzArgsT<T>& a, unsigned nb, cudaStream_t st,
                               const LzSide& side, KernelTimer* tm) {
@@ -896,11 +978,11 @@ static void lz_rows_kernels(const void* kern[6]) {
     kern[5] = (const void*)k_lz1_Md_rows<T, 3, true, PPT>;
 }
 
-// Whether pass 1 runs on the row-staged kernels (the autotuner's choice),
-// and their plan and grid.
+// Whether pass 1 runs on the row-staged kernels (CHDWF_STENCIL=rows, where
+// they fit), and their plan and grid.
 template <class T>
-static bool lz_rows_setup(const Geom& g, RowPlan* rp, unsigned* nb, cudaStream_t st) {
-    if (stencil_choice(g, (int)sizeof(T), st) != kStencilRows) return false;
+static bool lz_rows_setup(const Geom& g, RowPlan* rp, unsigned* nb) {
+    if (stencil_mode() != 2) return false;
     if (!row_plan(g, sizeof(T), rp) || rp->ppt != 1) return false;
     const void* kern[6];
     lz_rows_kernels<T, 1>(kern);
@@ -971,8 +1053,8 @@ static void set_stream_window(cudaStream_t st, const cudaAccessPolicyWindow& w) 
 // as a CUDA graph and replayed; the graph is rebuilt when any argument
 // changes.
 template <class T>
-static void launch_pass1_any(const LzArgsT<T>& a, unsigned nb, cudaStream_t st, const LzSide& side,
-                             KernelTimer* tm, int imass);
+static void launch_pass1_any(const LzArgsT<T>& a, unsigned nb, int k0, int chunk, cudaStream_t st,
+                             const LzSide& side, KernelTimer* tm, int imass);
 
 template <class T>
 static cudaGraphExec_t pass1_graph(LzWork& w, const LzArgsT<T>& a_in, unsigned nb, int imass,
@@ -996,7 +1078,7 @@ static cudaGraphExec_t pass1_graph(LzWork& w, const LzArgsT<T>& a_in, unsigned n
         return nullptr;
     }
     for (int c = 0; c < chunk; c++) {
-        launch_pass1_any<T>(a, nb, st, w.side, nullptr, imass);
+        launch_pass1_any<T>(a, nb, c, chunk, st, w.side, nullptr, imass);
     }
     if (cudaStreamEndCapture(st, &graph) != cudaSuccess || !graph) {
         cudaGetLastError();
@@ -1032,21 +1114,31 @@ static cudaGraphExec_t pass1_graph(LzWork& w, const LzArgsT<T>& a_in, unsigned n
     return exec;
 }
 
-template <class T, int IMASS, bool PAIR>
+template <class T, int IMASS>
 static void launch_pass2(const LzArgsT<T>& a, int j, int m, int iflag, cudaStream_t st,
                          KernelTimer& tm) {
-    const unsigned nb = lz_direct_blocks<T, PAIR>(a.g.npts);
     const int apply = j < m;
     const double V = (double)a.g.kferm * sizeof(T), chi = 12.0 * a.g.kvol;
     const double acc = iflag == 0 ? 2.0 * a.g.kferm * sizeof(double2) + V : 0.0;
     if (apply) tm.begin(timer_class<T>(3), st, 2 * V + chi + acc);
-    if (iflag == 0) k_lz2_M<T, IMASS, 0, PAIR><<<nb, kThreads, 0, st>>>(a, j, apply);
-    else k_lz2_M<T, IMASS, 1, PAIR><<<nb, kThreads, 0, st>>>(a, j, apply);
-    count_launches(1);
+    if (a.pl) {
+        const int64_t n = iflag == 0 ? a.g.kferm : 16 * (int64_t)a.g.kvol;
+        const unsigned nbe = (unsigned)((n + kThreads - 1) / kThreads);
+        if (iflag == 0) k_lzp_acc<T, 0><<<nbe, kThreads, 0, st>>>(a, j);
+        else k_lzp_acc<T, 1><<<nbe, kThreads, 0, st>>>(a, j);
+        if (apply) k_lz1_M<T, IMASS, true><<<a.pp.nitem, a.pp.threads, 0, st>>>(a, j);
+        count_launches(1 + apply);
+    } else {
+        const unsigned nb = lz_direct_blocks<T>(a.g.npts);
+        if (iflag == 0) k_lz2_M<T, IMASS, 0><<<nb, kThreads, 0, st>>>(a, j, apply);
+        else k_lz2_M<T, IMASS, 1><<<nb, kThreads, 0, st>>>(a, j, apply);
+        count_launches(1);
+    }
     if (apply) {
         tm.end(st);
         tm.begin(timer_class<T>(3), st, 4 * V + chi);
-        k_lz2_Md<T, IMASS, PAIR><<<nb, kThreads, 0, st>>>(a, j);
+        if (a.pl) k_lz1_Md<T, IMASS, false, true><<<a.pp.nitem, a.pp.threads, 0, st>>>(a, j);
+        else k_lz2_Md<T, IMASS><<<lz_direct_blocks<T>(a.g.npts), kThreads, 0, st>>>(a, j);
         tm.end(st);
         count_launches(1);
     }
@@ -1054,63 +1146,26 @@ static void launch_pass2(const LzArgsT<T>& a, int j, int m, int iflag, cudaStrea
 
 template <class T>
 static int pass1_shape(const LzArgsT<T>& a) {
-    return a.rows ? kStencilRows : (a.occ == 4 ? kStencilGather4 : kStencilGather3);
-}
-
-// Shape dispatch: FP32 vectors with Ls even take the two-point kernels.
-template <class T>
-static bool lz_pair(const Geom& g) {
-    return std::is_same<T, float2>::value && pair_ok(g);
+    return a.rows ? kStencilRows : kStencilGather3;
 }
 
 template <class T>
-static void launch_pass1_any(const LzArgsT<T>& a, unsigned nb, cudaStream_t st, const LzSide& side,
-                             KernelTimer* tm, int imass) {
-    if (a.rows) {
-        if (imass == 3) launch_pass1_rows<T, 3>(a, nb, st, side, tm);
-        else launch_pass1_rows<T, 1>(a, nb, st, side, tm);
+static void launch_pass1_any(const LzArgsT<T>& a, unsigned nb, int k0, int chunk, cudaStream_t st,
+                             const LzSide& side, KernelTimer* tm, int imass) {
+    if (a.pl) {
+        if (imass == 3) launch_pass1_planes<T, 3>(a, nb, k0, chunk, st, tm);
+        else launch_pass1_planes<T, 1>(a, nb, k0, chunk, st, tm);
         return;
     }
-    if constexpr (std::is_same<T, float2>::value) {
-        if (lz_pair<T>(a.g)) {
-            if (imass == 3) launch_pass1<T, 3, true>(a, nb, st, side, tm);
-            else launch_pass1<T, 1, true>(a, nb, st, side, tm);
-            return;
-        }
-    }
-    if (imass == 3) launch_pass1<T, 3, false>(a, nb, st, side, tm);
-    else launch_pass1<T, 1, false>(a, nb, st, side, tm);
+    if (imass == 3) launch_pass1_rows<T, 3>(a, nb, st, side, tm);
+    else launch_pass1_rows<T, 1>(a, nb, st, side, tm);
 }
 
 template <class T>
 static void launch_pass2_any(const LzArgsT<T>& a, int j, int m, int iflag, cudaStream_t st,
                              KernelTimer& tm, int imass) {
-    if constexpr (std::is_same<T, float2>::value) {
-        if (lz_pair<T>(a.g)) {
-            if (imass == 3) launch_pass2<T, 3, true>(a, j, m, iflag, st, tm);
-            else launch_pass2<T, 1, true>(a, j, m, iflag, st, tm);
-            return;
-        }
-    }
-    if (imass == 3) launch_pass2<T, 3, false>(a, j, m, iflag, st, tm);
-    else launch_pass2<T, 1, false>(a, j, m, iflag, st, tm);
-}
-
-template <class T, bool PAIR>
-static unsigned lz_pass1_blocks_occ(const Geom& g, int imass, int occ) {
-    if (occ == 4)
-        return imass == 3 ? lz_pass1_blocks<T, 3, PAIR, 4>(g.npts)
-                          : lz_pass1_blocks<T, 1, PAIR, 4>(g.npts);
-    return imass == 3 ? lz_pass1_blocks<T, 3, PAIR, 3>(g.npts)
-                      : lz_pass1_blocks<T, 1, PAIR, 3>(g.npts);
-}
-
-template <class T>
-static unsigned lz_pass1_blocks_any(const Geom& g, int imass, int occ) {
-    if constexpr (std::is_same<T, float2>::value) {
-        if (lz_pair<T>(g)) return lz_pass1_blocks_occ<T, true>(g, imass, occ);
-    }
-    return lz_pass1_blocks_occ<T, false>(g, imass, occ);
+    if (imass == 3) launch_pass2<T, 3>(a, j, m, iflag, st, tm);
+    else launch_pass2<T, 1>(a, j, m, iflag, st, tm);
 }
 
 // ---- kernel timer ----------------------------------------------------------
@@ -1256,10 +1311,9 @@ cudaError_t LzWork::ensure(const Geom& g, int npole_max, int prec, bool walls) {
         hist.rho = hist_mem + 4 * H;
         hist.mu = hist.rho + kMaxPoles * H;
         hist.y = hist.mu + kMaxPoles * H;
-        // block partials of the two pass-1 kernels (at most split_blocks
-        // blocks each), and the source norm's block partials
-        const int64_t nb = 2 * (int64_t)split_blocks(g.npts);
-        if ((e = cudaMalloc(&part, sizeof(double) * (nb + 2048)))) return e;
+        // block partials of the two pass-1 phases (at most kMaxPartBlocks
+        // resident blocks), or the source norm's block partials
+        if ((e = cudaMalloc(&part, sizeof(double) * 2 * kMaxPartBlocks))) return e;
         if ((e = cudaHostAlloc(&hflag_host, sizeof(int), cudaHostAllocMapped))) return e;
         if ((e = cudaStreamCreateWithFlags(&side.stream, cudaStreamNonBlocking))) return e;
         if ((e = cudaEventCreateWithFlags(&side.fork, cudaEventDisableTiming))) return e;
@@ -1273,15 +1327,16 @@ cudaError_t LzWork::ensure(const Geom& g, int npole_max, int prec, bool walls) {
     }
     if (prec == kPrecF32 && !rb32[0]) {
         for (int i = 0; i < 3; i++)
-            if ((e = cudaMalloc(&rb32[i], sizeof(float2) * g.kferm))) return e;
-        if ((e = cudaMalloc(&vt32, sizeof(float2) * g.kferm))) return e;
+            if ((e = cudaMalloc(&rb32[i], sizeof(float2) * plane_elems<float2>(g)))) return e;
+        if ((e = cudaMalloc(&vt32, sizeof(float2) * plane_elems<float2>(g)))) return e;
     }
     // Basis store: up to kMaxIter+2 vectors, at most 40% of the free HBM per
     // precision.  Solves longer than the store regenerate their vectors.
     if (basis_enabled && ((prec == kPrecF64 && !basis) || (prec == kPrecF32 && !basis32))) {
         size_t fr = 0, tot = 0;
         cudaMemGetInfo(&fr, &tot);
-        const size_t vb = (prec == kPrecF64 ? sizeof(double2) : sizeof(float2)) * (size_t)g.kferm;
+        const size_t vb = prec == kPrecF64 ? sizeof(double2) * (size_t)g.kferm
+                                           : sizeof(float2) * (size_t)plane_elems<float2>(g);
         // an explicit budget names the FP64 store; the FP32 store keeps the
         // same number of vectors in half the bytes
         const double budget = basis_max_bytes >= 0.0
@@ -1371,7 +1426,7 @@ __global__ void __launch_bounds__(kThreads) k_lz_walls_of(LzArgsT<T> a, const T*
     const int sw = (int)(rr & 1);
     const int64_t site = rr >> 1;
     a.wbasis[(int64_t)j * 8 * cs2 + t] =
-        vget(a, r, (sw ? a.g.Ls - 1 : 0) + (int64_t)a.g.Ls * site + a.g.cs * c);
+        vget(a, r, c, sw ? a.g.Ls - 1 : 0, site);
 }
 
 // q_j's wall slices (j = 1..m) into every pole's two-slice x_k: the same
@@ -1389,15 +1444,13 @@ __global__ void __launch_bounds__(kThreads, 2) k_lz_accum_walls(LzArgsT<T> a, in
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const int64_t cs2 = 2 * (int64_t)a.g.kvol, kf2 = 8 * cs2;
     const bool act = t < kf2;
-    int64_t e = t, stride = kf2;
-    const T* src = a.wbasis;
-    if (!STORE) {
-        const int c = act ? (int)(t / cs2) : 0;             // component
-        const int64_t r = act ? t - c * cs2 : 0;           // s' + 2 site
-        e = ((r & 1) ? a.g.Ls - 1 : 0) + (int64_t)a.g.Ls * (r >> 1) + a.g.cs * c;
-        stride = a.g.kferm;
-        src = a.basis;
-    }
+    // from the basis: component, wall and site of the element
+    const int c = act ? (int)(t / cs2) : 0;
+    const int64_t r = act ? t - c * cs2 : 0;
+    const int s = (r & 1) ? a.g.Ls - 1 : 0;
+    auto load = [&](int j) {
+        return STORE ? __ldg(a.wbasis + j * kf2 + t) : vget(a, a.basis + j * a.vs, c, s, r >> 1);
+    };
     const int64_t H = kMaxIter + 2;
     const int n = a.npole;
     double2 acc[NC];
@@ -1415,15 +1468,11 @@ __global__ void __launch_bounds__(kThreads, 2) k_lz_accum_walls(LzArgsT<T> a, in
         __syncthreads();
         if (act) {
             // q_{j+1} is loaded while q_j is accumulated
-            const int64_t b = e + j0 * stride;
-            T qn = STORE ? __ldg(src + b) : vget(a, src, b);
+            T qn = load(j0);
 #pragma unroll 1
             for (int jj = 0; jj < jn; jj++) {
                 const T q = qn;
-                if (jj + 1 < jn) {
-                    const int64_t bn = b + (jj + 1) * stride;
-                    qn = STORE ? __ldg(src + bn) : vget(a, src, bn);
-                }
+                if (jj + 1 < jn) qn = load(j0 + jj + 1);
                 const double2 qj = widen(zscal(ibs[jj], q));
 #pragma unroll
                 for (int k = 0; k < NC; k++) {
@@ -1454,22 +1503,77 @@ static void launch_accum_walls(const LzArgsT<T>& a, int m, int n, int64_t kvol, 
 
 // ---- pass 2 from the stored basis ---------------------------------------
 // x += sum_j c_j q_j, q_j = r_j / beta_j, j = 1..m, in j order per element
-// (the same sequence of operations as the regenerating pass 2).
+// (the same sequence of operations as the regenerating pass 2).  A thread
+// takes one 16-byte unit of the vectors (planes: one FP64 or two FP32
+// elements; the ABI's layout: one element), so the stored vectors, m of them
+// against one read and write of x, stream coalesced.
+template <class T> struct AccUnit;
+template <> struct AccUnit<double2> {
+    static constexpr int N = 1;
+    __device__ __forceinline__ static void get(const LzArgsT<double2>&, const double2* v,
+                                               int64_t i, double2* q) {
+        q[0] = __ldg(v + i);
+    }
+};
+template <> struct AccUnit<float2> {
+    static constexpr int N = 2;
+    __device__ __forceinline__ static void get(const LzArgsT<float2>& a, const float2* v,
+                                               int64_t i, float2* q) {
+        if (a.pl) {
+            const float4 f = __ldg(reinterpret_cast<const float4*>(v) + i);
+            const cpair p{make_float2(f.x, f.y), make_float2(f.z, f.w)};
+            q[0] = cpair_pt(p, 0);
+            q[1] = cpair_pt(p, 1);
+        } else {
+            q[0] = __ldg(v + i);
+            q[1] = make_float2(0.0f, 0.0f);
+        }
+    }
+};
+// Units of a stored vector, and the x elements of unit i: the first one's
+// index and the number of elements (x is in the ABI's layout, the elements
+// of a unit adjacent).
+template <class T>
+__host__ __device__ __forceinline__ int64_t acc_units(const LzArgsT<T>& a) {
+    return a.pl ? 8 * (int64_t)a.pp.U * a.g.kvol : a.g.kferm;
+}
+template <class T>
+__device__ __forceinline__ int64_t acc_elem(const LzArgsT<T>& a, int64_t i, int* n) {
+    constexpr int N = AccUnit<T>::N;
+    *n = 1;
+    if (!a.pl) return i;
+    const int64_t cu = i / a.g.kvol, site = i - cu * a.g.kvol;
+    const int c = (int)(cu / a.pp.U), u = (int)(cu - (int64_t)c * a.pp.U);
+    if (N == 2 && 2 * u + 1 < a.g.Ls) *n = 2;
+    return (int64_t)N * u + (int64_t)a.g.Ls * site + a.g.cs * c;
+}
+
 template <class T>
 __global__ void __launch_bounds__(kThreads) k_lz_accum_x(LzArgsT<T> a, int j0, int j1) {
     typedef typename real_of<T>::type Real;
-    const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (e >= a.g.kferm) return;
-    double2 xv = a.x[e];
-    const int64_t stride = a.g.kferm;
+    constexpr int N = AccUnit<T>::N;
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= acc_units(a)) return;
+    int n;
+    const int64_t e = acc_elem(a, i, &n);
+    double2 xv[N];
+    xv[0] = a.x[e];
+    if (N == 2) xv[N - 1] = n == 2 ? a.x[e + 1] : make_double2(0.0, 0.0);
 #pragma unroll 4
     for (int j = j0; j <= j1; j++) {
-        const double2 qj = widen(zscal((Real)a.h.invbeta[j], vget(a, a.basis, e + j * stride)));
+        T q[N];
+        AccUnit<T>::get(a, a.basis + j * a.vs, i, q);
+        const Real ib = (Real)a.h.invbeta[j];
         const double cj = a.h.c[j];
-        xv.x += cj * qj.x;
-        xv.y += cj * qj.y;
+#pragma unroll
+        for (int k = 0; k < N; k++) {
+            const double2 qj = widen(zscal(ib, q[k]));
+            xv[k].x += cj * qj.x;
+            xv[k].y += cj * qj.y;
+        }
     }
-    a.x[e] = xv;
+    a.x[e] = xv[0];
+    if (N == 2 && n == 2) a.x[e + 1] = xv[N - 1];
 }
 
 static constexpr int kAccumChunk = 64;
@@ -1480,29 +1584,44 @@ template <class T>
 __global__ void __launch_bounds__(kThreads) k_lz_accum_poles(LzArgsT<T> a, int m, int k0,
                                                              double2* const* xk) {
     typedef typename real_of<T>::type Real;
-    const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (e >= a.g.kferm) return;
-    const int64_t H = kMaxIter + 2, stride = a.g.kferm;
+    constexpr int N = AccUnit<T>::N;
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= acc_units(a)) return;
+    int ne;
+    const int64_t e = acc_elem(a, i, &ne);
+    const int64_t H = kMaxIter + 2;
     const int n = a.npole;
-    double2 acc[8];
+    double2 acc[8][N];
 #pragma unroll
-    for (int k = 0; k < 8; k++) acc[k] = make_double2(0.0, 0.0);
+    for (int k = 0; k < 8; k++)
+#pragma unroll
+        for (int p = 0; p < N; p++) acc[k][p] = make_double2(0.0, 0.0);
     for (int j = 1; j <= m; j++) {
-        const double2 qj = widen(zscal((Real)a.h.invbeta[j], vget(a, a.basis, j * stride + e)));
+        T q[N];
+        AccUnit<T>::get(a, a.basis + j * a.vs, i, q);
+        const Real ib = (Real)a.h.invbeta[j];
+        double2 qj[N];
+#pragma unroll
+        for (int p = 0; p < N; p++) qj[p] = widen(zscal(ib, q[p]));
 #pragma unroll
         for (int k = 0; k < 8; k++) {
             if (k0 + k < n) {
                 const double y = a.h.y[(k0 + k) * H + j];
-                acc[k].x += y * qj.x;
-                acc[k].y += y * qj.y;
+#pragma unroll
+                for (int p = 0; p < N; p++) {
+                    acc[k][p].x += y * qj[p].x;
+                    acc[k][p].y += y * qj[p].y;
+                }
             }
         }
     }
 #pragma unroll
     for (int k = 0; k < 8; k++)
-        if (k0 + k < n) xk[k0 + k][e] = acc[k];
+        if (k0 + k < n) {
+            xk[k0 + k][e] = acc[k][0];
+            if (N == 2 && ne == 2) xk[k0 + k][e + 1] = acc[k][N - 1];
+        }
 }
-
 
 template <class T>
 static cudaError_t lz_solve_t(LzWork& w, const Geom& g, const double2* phi, float res, int ndiag,
@@ -1544,22 +1663,24 @@ static cudaError_t lz_solve_t(LzWork& w, const Geom& g, const double2* phi, floa
     a.xw = w.xw;
     a.npole = ndiag;
     unsigned nb = 0;
-    // FP32 vectors with Ls even live in the split layout, which only the
-    // point-gather kernels read (the row-staged shape serves the FP64 solves
-    // and odd Ls)
-    a.pl = lz_pair<T>(g) ? 1 : 0;
-    a.rows = !a.pl && lz_rows_setup<T>(g, &a.rp, &nb, st) ? 1 : 0;
-    a.occ = (a.pl ? stencil_choice_split(g, st) : stencil_choice(g, (int)sizeof(T), st)) ==
-                    kStencilGather4
-                ? 4
-                : 3;
-    if (!a.rows) nb = lz_pass1_blocks_any<T>(g, imass, a.occ);
+    a.rows = lz_rows_setup<T>(g, &a.rp, &nb) ? 1 : 0;
+    a.pl = !a.rows;
+    a.vs = a.pl ? plane_elems<T>(g) : g.kferm;
+    if (a.pl) {
+        if (!plane_ok(g)) return cudaErrorInvalidValue;
+        int dev = 0, nsm = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+        a.pp = plane_plan(g, std::is_same<T, float2>::value, nsm);
+        nb = imass == 3 ? pass1_workers<T, 3>(a.pp, nsm) : pass1_workers<T, 1>(a.pp, nsm);
+        if (nb < 1) return cudaErrorLaunchOutOfResources;
+    }
     const int nbr = reduce_blocks(g.kferm);
     // r_1 lives where ring(a, 1) looks for it: the basis store when present
-    T* r1 = a.hcap > 1 ? a.basis + g.kferm : a.rb1;
+    T* r1 = a.hcap > 1 ? a.basis + a.vs : a.rb1;
 
     // r_1 = Phi, beta_1 = |r_1|
-    k_lz_source<T><<<nbr, kThreads, 0, st>>>(r1, phi, g.kferm, w.part, a.pl);
+    k_lz_source<T><<<nbr, kThreads, 0, st>>>(a, r1, phi, w.part);
     k_lz_init<<<1, kThreads, 0, st>>>(w.ctl, w.hist, w.part, nbr);
     count_launches(2);
     if (a.wcap > 1) {                    // r_1's wall slices (pass 1 adds r_2, r_3, ...)
@@ -1576,12 +1697,12 @@ static cudaError_t lz_solve_t(LzWork& w, const Geom& g, const double2* phi, floa
     cudaEvent_t ev[kAhead + 1];
     for (cudaEvent_t& e : ev) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
     int launched = 0, nchunk = 0;
-    // the per-launch path when kernels are being timed, else graph replays
-    const cudaAccessPolicyWindow win = vt_window(a.vt, sizeof(T) * (size_t)g.kferm);
+    const cudaAccessPolicyWindow win = vt_window(a.vt, sizeof(T) * (size_t)a.vs);
     if (win.num_bytes) set_stream_window(st, win);
     // per-launch timing issues pass 1 launch by launch; chunk timing keeps
     // the graph replays and brackets each one
     const bool chunked = w.timer.enabled && w.timer.chunks;
+    const int per_it = a.pl ? 2 : 3;      // kernels an iteration
     cudaGraphExec_t gexec = w.timer.enabled && !chunked
                                 ? nullptr
                                 : pass1_graph<T>(w, a, nb, imass, chunk, st, win);
@@ -1590,16 +1711,13 @@ static cudaError_t lz_solve_t(LzWork& w, const Geom& g, const double2* phi, floa
             if (chunked) w.timer.chunk_begin(st, launched + 1);
             cudaGraphLaunch(gexec, st);
             if (chunked) w.timer.chunk_end(st);
-            launched += chunk;
-            count_launches(3 * chunk);
-            note_stencil(pass1_shape(a), 2 * chunk);
         } else {
-            for (int c = 0; c < chunk && launched < kMaxIter; c++, launched++) {
-                launch_pass1_any<T>(a, nb, st, w.side, &w.timer, imass);
-                count_launches(3);
-                note_stencil(pass1_shape(a), 2);
-            }
+            for (int c = 0; c < chunk; c++)
+                launch_pass1_any<T>(a, nb, c, chunk, st, w.side, &w.timer, imass);
         }
+        launched += chunk;
+        count_launches(per_it * chunk + a.pl);
+        note_stencil(pass1_shape(a), 2 * chunk);
         cudaEventRecord(ev[nchunk % (kAhead + 1)], st);
         if (nchunk >= kAhead) {
             cudaEventSynchronize(ev[(nchunk - kAhead) % (kAhead + 1)]);
@@ -1642,20 +1760,20 @@ static cudaError_t lz_solve_t(LzWork& w, const Geom& g, const double2* phi, floa
     if ((e = cudaStreamSynchronize(st))) return e;
     const int m = hr.m;
     *itercg = m;
-    if (hr.done == 4) return cudaErrorLaunchTimeout;   // a staged copy never arrived
+    if (hr.done == 4) return cudaErrorLaunchTimeout;   // a bounded wait ran out
     *status = hr.done == 1 ? 0 : (hr.done == 2 ? 1 : 2);
     if (stats) { stats->iters = m; stats->pass1_launches = 2 * launched; }
     if (m < 1) return cudaErrorUnknown;
 
     // coefficients, then pass 2 over the regenerated vectors
     k_lz_coeffs<<<1, kThreads, 0, st>>>(w.ctl, w.hist, iflag);
-    k_lz_source<T><<<nbr, kThreads, 0, st>>>(r1, phi, g.kferm, w.part, a.pl);
+    k_lz_source<T><<<nbr, kThreads, 0, st>>>(a, r1, phi, w.part);
     count_launches(2);
     if (iflag == 2) {
         // every x_k from the stored basis, poles in chunks of 8 (one pass over
         // the basis per chunk); needs the whole basis in HBM
         if (!(m < a.hcap) || !w.pole_out) return cudaErrorInvalidValue;
-        const unsigned nbx = (unsigned)((g.kferm + kThreads - 1) / kThreads);
+        const unsigned nbx = (unsigned)((acc_units(a) + kThreads - 1) / kThreads);
         for (int k0 = 0; k0 < ndiag; k0 += 8) {
             k_lz_accum_poles<T><<<nbx, kThreads, 0, st>>>(a, m, k0, w.pole_out);
             count_launches(1);
@@ -1677,7 +1795,7 @@ static cudaError_t lz_solve_t(LzWork& w, const Geom& g, const double2* phi, floa
             // a chunk of stored vectors per launch: x (FP64) is carried in
             // memory between chunks, so each element still sums j = 1..m in
             // order, and the pages a launch touches stay few
-            const unsigned nbx = (unsigned)((g.kferm + kThreads - 1) / kThreads);
+            const unsigned nbx = (unsigned)((acc_units(a) + kThreads - 1) / kThreads);
             for (int j0 = 1; j0 <= m; j0 += kAccumChunk) {
                 const int j1 = j0 + kAccumChunk - 1 < m ? j0 + kAccumChunk - 1 : m;
                 k_lz_accum_x<T><<<nbx, kThreads, 0, st>>>(a, j0, j1);

@@ -3,6 +3,7 @@
 #include <vector>
 
 #include "internal.h"
+#include "planes.cuh"
 #include "row_stage.cuh"
 
 namespace chdwf {
@@ -15,8 +16,9 @@ struct LzArgsT {
     typedef typename real_of<T>::type Real;
     Geom g;
     T *rb0, *rb1, *rb2;         // Lanczos residual ring: r_j lives in rb[j % 3] ...
-    T* basis;                   // ... unless j < hcap: then in basis + j*kferm
+    T* basis;                   // ... unless j < hcap: then in basis + j*vs
     int hcap;
+    int64_t vs;                 // elements of one stored vector
     T* vt;                      // M q_j
     const float* chif;          // chi rounded to REAL*4 (wall coupling)
     Real diag, hpin;
@@ -30,11 +32,14 @@ struct LzArgsT {
     int npole;
     T* wbasis;                  // force solves: the two wall slices of each r_j,
     int wcap;                   // j < wcap, at wbasis + j*16*kvol (0: no wall store)
-    int pl;                     // FP32 vectors in the split layout (cpair; Ls even)
-    int rows;                   // pass 1 on the row-staged kernels (plan rp)
-    int occ;                    // else the point-gather kernels at 3 or 4 blocks a SM
+    int pl;                     // vectors in planes, pass 1 on the plane kernels (plan pp)
+    int rows;                   // else: ABI layout, row-staged kernels (plan rp)
+    PlanePlan pp;
     RowPlan rp;
 };
+
+// Block partials a pass-1 phase may leave (resident blocks).
+constexpr int kMaxPartBlocks = 4096;
 
 struct LzStats {
     int iters;
@@ -88,8 +93,8 @@ struct LzGraph {
     int imass = 0, chunk = 0;
 };
 
-// Side stream of the pass-1 loop: the scalar step of each iteration runs
-// there, beside the M^dagger kernel, forked and joined with events.
+// Side stream of the row-staged pass 1: the scalar step of each iteration
+// runs there, beside the M^dagger kernel, forked and joined with events.
 struct LzSide {
     cudaStream_t stream = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
