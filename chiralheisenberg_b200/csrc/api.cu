@@ -42,6 +42,7 @@ Ctx::~Ctx() {
     lz.release();
     cg.release();
     free_batch(batch);
+    free_multishift(ms);
     for (int i = 0; i < kSpin; i++)
         if (spin[i]) cudaFree(spin[i]);
     if (chid) cudaFree(chid);

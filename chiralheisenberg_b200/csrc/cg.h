@@ -4,33 +4,19 @@
 
 namespace chdwf {
 
+template <class T> struct PcgWork;      // plane_cg.cuh
+
+// Control block of the single-precision CGNE of hmc.cu.
 struct CgCtl {
     int nx, done, iters, niterc;
     float alpha, beta, alphan, betad, resid, pad2_;
     unsigned count1, count2;
 };
 
-struct CgArgs {
-    Geom g;
-    double2 *x, *p, *r, *x1;
-    const float* chif;
-    double diag, hpin;
-    int apbc;
-    CgCtl* ctl;
-    double* part;
-    int* hflag;
-};
-
 struct CgWork {
-    Geom geom{};
-    CgCtl* ctl = nullptr;
-    double* part = nullptr;
-    double2 *x1 = nullptr, *p = nullptr, *r = nullptr;
-    int* hflag_host = nullptr;
-    int* hflag_dev = nullptr;
+    PcgWork<double2>* w = nullptr;
     ~CgWork();
     void release();
-    cudaError_t ensure(const Geom& g);
 };
 
 // Solves M^dagger M x = Phi starting from x (in/out).  status 0 converged,

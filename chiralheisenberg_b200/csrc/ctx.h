@@ -10,6 +10,7 @@ namespace chdwf {
 
 struct BatchWork;                       // batch.cu
 void free_batch(BatchWork* w);
+void free_multishift(PcgWork<float2>* w);   // multishift.cu
 
 // One rational approximation as the reference reads it (rhmc/cheisdwf.f:
 // 140-159): anum[0] = a0, anum[1..n], aden = sigma_1..n; same for b.
@@ -50,6 +51,7 @@ struct Ctx {
     RemezSet rz_hb, rz_act;
     int prec_md = 0, prec_accept = 0;   // vector precision of the resident solves
     BatchWork* batch = nullptr;         // workspace of chdwf_congrad_batch
+    PcgWork<float2>* ms = nullptr;      // inner solves of chdwf_multishift_dev
     double2* prop_x = nullptr;          // chdwf_traj_propagators: solutions and
     double2* prop_phi = nullptr;        // right-hand sides of nsrc sources
     int prop_cap = 0;

@@ -9,10 +9,14 @@
 // FP32: the same solve with FP32 vectors stopped at max(res, 1e-6), x_k
 // accumulated in FP64; then, per shift, while the FP64 true residual
 // |Phi - (M^dag M + sigma_k) x_k| / |Phi| exceeds res: an FP32 CG on the
-// shifted system with the FP64 residual as right-hand side, run until its
-// own residual falls by 1e-4 (or stagnates), and its solution added to x_k
-// in FP64 -- defect correction, each outer step recomputing the true
+// shifted system with the FP64 residual as right-hand side, and its solution
+// added to x_k in FP64 -- defect correction, each round recomputing the true
 // residual in FP64.  The result meets the same true-residual target as FP64.
+//
+// The corrections of several shifts run as one batch (plane_cg.cuh): their
+// scalars stay on the device and each iteration is three launches for all of
+// them: 20 shifts at 16^3x16 to 1e-10 take 98 ms.  One shift at a time, with
+// the scalars on the host (two round trips an iteration), they took 615 ms.
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -20,6 +24,7 @@
 #include "../../include/chdwf.h"
 #include "ctx.h"
 #include "lanczos.h"
+#include "plane_cg.cuh"
 
 using namespace chdwf;
 
@@ -45,118 +50,168 @@ __global__ void k_ms_resid(double2* __restrict__ r, const double2* __restrict__ 
     if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
 
-// FP32 vector kernels of the inner CG; reductions in FP64
-__global__ void k_ms_to32(float2* __restrict__ o, const double2* __restrict__ i, double scale,
-                          int64_t n) {
-    const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (k < n) o[k] = make_float2((float)(i[k].x * scale), (float)(i[k].y * scale));
-}
-__global__ void k_ms_dot32(const float2* __restrict__ a, const float2* __restrict__ b, int64_t n,
-                           double* __restrict__ part) {
-    __shared__ double sh[kThreads / 32];
-    double s = 0.0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x)
-        s += (double)a[i].x * b[i].x + (double)a[i].y * b[i].y;
-    s = block_sum<kThreads>(s, sh);
-    if (threadIdx.x == 0) part[blockIdx.x] = s;
-}
-// ap = t + sigma p
-__global__ void k_ms_shift32(float2* __restrict__ ap, const float2* __restrict__ t,
-                             const float2* __restrict__ p, float sigma, int64_t n) {
-    const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (k < n) ap[k] = make_float2(t[k].x + sigma * p[k].x, t[k].y + sigma * p[k].y);
-}
-// e += alpha p ; r -= alpha ap
-__global__ void k_ms_update32(float2* __restrict__ e, float2* __restrict__ r,
-                              const float2* __restrict__ p, const float2* __restrict__ ap,
-                              float alpha, int64_t n) {
-    const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (k < n) {
-        e[k] = make_float2(e[k].x + alpha * p[k].x, e[k].y + alpha * p[k].y);
-        r[k] = make_float2(r[k].x - alpha * ap[k].x, r[k].y - alpha * ap[k].y);
+// r (FP64, ABI layout) times scale into planes: the inner solve's r and p, e
+// = 0, and the blocks' partials of |p|^2 (k_pcg3's blocks)
+__global__ void __launch_bounds__(kPcgThreads) k_ms_planes(cpair* p, cpair* rp, cpair* x,
+                                                           double* part, Geom g, int U,
+                                                           const double2* __restrict__ r,
+                                                           double scale) {
+    const int64_t nu = 8 * (int64_t)U * g.kvol;
+    const int64_t i0 = (int64_t)blockIdx.x * (kPcgThreads * kPcgUnits) + threadIdx.x;
+    double loc = 0.0;
+    for (int q = 0; q < kPcgUnits; q++) {
+        const int64_t i = i0 + q * kPcgThreads;
+        if (i >= nu) break;
+        const PlaneUnit pu = plane_unit_of<float2>(g, U, i);
+        const double2 a = r[pu.e], b = pu.n == 2 ? r[pu.e + 1] : make_double2(0.0, 0.0);
+        const cpair v{make_float2((float)(a.x * scale), (float)(b.x * scale)),
+                      make_float2((float)(a.y * scale), (float)(b.y * scale))};
+        const cpair z{make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
+        st_unit(p + i, v);
+        st_unit(rp + i, v);
+        st_unit(x + i, z);
+        loc += unit_norm2(v);
     }
+    __shared__ double sh[32];
+    loc = block_sum_any(loc, sh);
+    if (threadIdx.x == 0) part[blockIdx.x] = loc;
 }
-// p = r + beta p
-__global__ void k_ms_dir32(float2* __restrict__ p, const float2* __restrict__ r, float beta,
-                           int64_t n) {
-    const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (k < n) p[k] = make_float2(r[k].x + beta * p[k].x, r[k].y + beta * p[k].y);
-}
-// x += scale * e (FP64)
-__global__ void k_ms_add(double2* __restrict__ x, const float2* __restrict__ e, double scale,
-                         int64_t n) {
-    const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (k < n) x[k] = make_double2(x[k].x + scale * e[k].x, x[k].y + scale * e[k].y);
-}
-
-double host_sum(const double* part_dev, int nb, cudaStream_t st) {
-    std::vector<double> h(nb);
-    cudaMemcpyAsync(h.data(), part_dev, sizeof(double) * nb, cudaMemcpyDeviceToHost, st);
-    cudaStreamSynchronize(st);
-    double s = 0.0;
-    for (double v : h) s += v;
-    return s;
+// x += scale * e (FP64, ABI layout; e in planes)
+__global__ void k_ms_add(double2* __restrict__ x, const cpair* __restrict__ ev, Geom g, int U,
+                         double scale) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= 8 * (int64_t)U * g.kvol) return;
+    const PlaneUnit pu = plane_unit_of<float2>(g, U, i);
+    const cpair e = ld_unit(ev + i);
+    for (int k = 0; k < pu.n; k++) {
+        const float2 v = cpair_pt(e, k);
+        x[pu.e + k] = make_double2(x[pu.e + k].x + scale * v.x, x[pu.e + k].y + scale * v.y);
+    }
 }
 
 struct MsWork {
-    double2 *t = nullptr, *r = nullptr;
-    float2 *e = nullptr, *rr = nullptr, *p = nullptr, *ap = nullptr, *t32 = nullptr;
+    double2 *t = nullptr, *r = nullptr;   // r: one residual per system of a part
     double* part = nullptr;
     double2** xk_dev = nullptr;
     ~MsWork() {
-        cudaFree(t); cudaFree(r); cudaFree(e); cudaFree(rr); cudaFree(p); cudaFree(ap);
-        cudaFree(t32); cudaFree(part); cudaFree(xk_dev);
+        cudaFree(t); cudaFree(r); cudaFree(part); cudaFree(xk_dev);
     }
 };
 
-// |Phi - (M^dag M + sigma) x|^2 into *r2 (FP64), residual vector in w.r
-cudaError_t true_residual(Ctx* c, MsWork& w, const double2* phi, const double2* x, double sigma,
-                          float hpin, int imass, double* r2) {
+// Residual vector Phi - (M^dag M + sigma) x into r, block partials of its
+// square into part (FP64)
+void true_residual(Ctx* c, MsWork& w, const double2* phi, const double2* x, double sigma,
+                   float hpin, int imass, double2* r, double* part) {
     const Geom& g = c->g;
     launch_dslash64(false, imass, w.t, x, c->chif, g, c->am3, hpin, c->ibound, c->stream);
     launch_dslash64(true, imass, c->spin[3], w.t, c->chif, g, c->am3, hpin, c->ibound, c->stream);
-    const int nb = reduce_blocks(g.kferm);
-    k_ms_resid<<<nb, kThreads, 0, c->stream>>>(w.r, phi, c->spin[3], x, sigma, g.kferm, w.part);
+    k_ms_resid<<<reduce_blocks(g.kferm), kThreads, 0, c->stream>>>(r, phi, c->spin[3], x, sigma,
+                                                                  g.kferm, part);
     count_launches(1);
-    *r2 = host_sum(w.part, nb, c->stream);
-    return cudaGetLastError();
 }
 
-// FP32 CG on (M^dag M + sigma) e = r/|r|, to a relative residual of tol or
-// maxit iterations; e (FP32) holds the solution of the normalised system.
-cudaError_t inner_cg32(Ctx* c, MsWork& w, float sigma, float hpin, int imass, double tol,
-                       int maxit, int* iters) {
-    const Geom& g = c->g;
-    const int64_t n = g.kferm;
-    const int nb = reduce_blocks(n), nbe = (int)nb_of(n);
-    cudaStream_t st = c->stream;
-    cudaMemsetAsync(w.e, 0, sizeof(float2) * n, st);
-    cudaMemcpyAsync(w.p, w.rr, sizeof(float2) * n, cudaMemcpyDeviceToDevice, st);
-    k_ms_dot32<<<nb, kThreads, 0, st>>>(w.rr, w.rr, n, w.part);
-    double rr = host_sum(w.part, nb, st);
-    const double rr0 = rr;
-    int it = 0;
-    for (; it < maxit && rr > tol * tol * rr0; it++) {
-        launch_dslash_lp(false, imass, 0, w.t32, w.p, c->chif, g, c->am3, hpin, c->ibound, st);
-        launch_dslash_lp(true, imass, 0, w.ap, w.t32, c->chif, g, c->am3, hpin, c->ibound, st);
-        k_ms_shift32<<<nbe, kThreads, 0, st>>>(w.ap, w.ap, w.p, sigma, n);
-        k_ms_dot32<<<nb, kThreads, 0, st>>>(w.p, w.ap, n, w.part);
-        const double pap = host_sum(w.part, nb, st);
-        if (!(pap > 0.0)) break;
-        const double alpha = rr / pap;
-        k_ms_update32<<<nbe, kThreads, 0, st>>>(w.e, w.rr, w.p, w.ap, (float)alpha, n);
-        k_ms_dot32<<<nb, kThreads, 0, st>>>(w.rr, w.rr, n, w.part);
-        const double rn = host_sum(w.part, nb, st);
-        k_ms_dir32<<<nbe, kThreads, 0, st>>>(w.p, w.rr, (float)(rn / rr), n);
-        count_launches(6);
-        rr = rn;
+// Sums of n consecutive runs of len partials.
+cudaError_t run_sums(const double* part_dev, int n, int len, double* out, cudaStream_t st) {
+    std::vector<double> h((size_t)n * len);
+    cudaError_t e = cudaMemcpyAsync(h.data(), part_dev, sizeof(double) * h.size(),
+                                    cudaMemcpyDeviceToHost, st);
+    if (!e) e = cudaStreamSynchronize(st);
+    for (int i = 0; i < n; i++) {
+        out[i] = 0.0;
+        for (int k = 0; k < len; k++) out[i] += h[(size_t)i * len + k];
     }
-    *iters = it;
+    return e;
+}
+
+constexpr int kMsRounds = 20;          // corrections of one shift at most
+constexpr double kMsInner = 1e-5;      // least relative residual of an inner solve
+
+// Defect correction of the shifts k0..k0+n-1 together, until each one's true
+// residual is at most res or stops falling.
+cudaError_t correct_part(Ctx* c, MsWork& w, PcgWork<float2>& P, const double2* phi, double phin,
+                         float res, float hpin, int imass, int k0, int n, const double* sigma,
+                         void* const* x, double* true_res, int* iters) {
+    const Geom& g = c->g;
+    cudaStream_t st = c->stream;
+    const int nb = reduce_blocks(g.kferm);
+    const size_t ve = (size_t)plane_elems<float2>(g) / 2;     // units of a vector
+    std::vector<int> run(n);           // the part's shifts still to be corrected
+    for (int i = 0; i < n; i++) run[i] = i;
+    std::vector<double> rel(n, HUGE_VAL), r2(n), rr(n);
+    cudaError_t e;
+    for (int round = 0; !run.empty(); round++) {
+        for (size_t a = 0; a < run.size(); a++) {
+            const int i = run[a];
+            true_residual(c, w, phi, (const double2*)x[k0 + i], sigma[k0 + i], hpin, imass,
+                          w.r + g.kferm * (int64_t)a, w.part + (size_t)nb * a);
+        }
+        if ((e = run_sums(w.part, (int)run.size(), nb, r2.data(), st))) return e;
+        std::vector<int> next, slot;
+        for (size_t a = 0; a < run.size(); a++) {
+            const int i = run[a];
+            const double now = std::sqrt(r2[a]) / phin;
+            const bool falls = now < rel[i];
+            rel[i] = now;
+            true_res[k0 + i] = now;
+            if (falls && now > (double)res && round < kMsRounds) {
+                next.push_back(i);
+                slot.push_back((int)a);
+            }
+        }
+        run = next;
+        if (run.empty()) break;
+        PcgBatch<float2> B;
+        std::vector<PcgDyn<float2>> dyn;
+        std::vector<PcgSlot> slots(run.size());
+        for (size_t q = 0; q < run.size(); q++)
+            if (!B.add(g, 2.0f * ((3.0f - c->am3) + 1.0f), hpin, c->ibound == -1, imass, 1, pcg_sms()))
+                return cudaErrorInvalidValue;
+        P.bind(B, c->chif);
+        const int U = B.geo(0).pl.U, neblk = B.geo(0).neblk, nblk = B.geo(0).nblk;
+        for (size_t a = 0; a < run.size(); a++) {
+            cpair* p = P.vec + B.a.vec0[a];
+            double* part3 = P.part + B.a.part0[a] + 2 * nblk;
+            k_ms_planes<<<neblk, kPcgThreads, 0, st>>>(p, p + ve, p + 3 * ve, part3, g, U,
+                                                       w.r + g.kferm * (int64_t)slot[a],
+                                                       1.0 / std::sqrt(r2[slot[a]]));
+            count_launches(1);
+        }
+        for (size_t a = 0; a < run.size(); a++) {
+            if ((e = run_sums(P.part + B.a.part0[a] + 2 * nblk, 1, neblk, &rr[a], st))) return e;
+            // one round to a tenth of res where FP32 can reach it: x is then
+            // 1.5e-10 from 64 bits (a quarter of res: 3.8e-10; rounds of a
+            // fixed 1e-4: 2.6e-10)
+            double tol = 0.1 * (double)res / rel[run[a]];
+            tol = tol < kMsInner ? kMsInner : (tol > 0.5 ? 0.5 : tol);
+            memset(&slots[a], 0, sizeof(PcgSlot));
+            slots[a].rr = rr[a];
+            PcgDyn<float2> d;
+            memset(&d, 0, sizeof(d));
+            d.x = P.vec + B.a.vec0[a] + 3 * ve;
+            d.sigma = (float)sigma[k0 + run[a]];
+            d.rstop = tol * tol * rr[a];
+            d.niterc = 4 * kMaxIter;
+            dyn.push_back(d);
+        }
+        if ((e = P.solve(B, dyn, slots, st))) return e;
+        for (size_t a = 0; a < run.size(); a++) {
+            *iters += slots[a].iters;
+            k_ms_add<<<nb_of((int64_t)ve), kThreads, 0, st>>>((double2*)x[k0 + run[a]], dyn[a].x, g, U,
+                                                             std::sqrt(r2[slot[a]]));
+            count_launches(1);
+        }
+    }
     return cudaGetLastError();
 }
 
 }  // namespace
+
+void free_multishift(PcgWork<float2>* w) {
+    if (w) {
+        w->release();
+        delete w;
+    }
+}
 }  // namespace chdwf
 
 extern "C" int chdwf_multishift_dev(chdwf_ctx* ctx, const void* Phi, float res, const void* chi,
@@ -172,17 +227,15 @@ extern "C" int chdwf_multishift_dev(chdwf_ctx* ctx, const void* Phi, float res, 
     launch_round_chi((const double*)chi, c->chif, g.kvol, st);
     MsWork w;
     cudaError_t e;
+    // shifts that are corrected together: as many as keep their four FP32
+    // vectors in L2
+    const size_t ve = (size_t)plane_elems<float2>(g) / 2;
+    int np = prec == CHDWF_PREC_F32 ? (int)(90e6 / (64.0 * (double)ve)) : 1;
+    np = np < 1 ? 1 : (np > n ? n : np);
     if ((e = cudaMalloc(&w.t, sizeof(double2) * g.kferm)) ||
-        (e = cudaMalloc(&w.r, sizeof(double2) * g.kferm)) ||
-        (e = cudaMalloc(&w.part, sizeof(double) * 8192)) ||
+        (e = cudaMalloc(&w.r, sizeof(double2) * g.kferm * np)) ||
+        (e = cudaMalloc(&w.part, sizeof(double) * 2048 * np)) ||
         (e = cudaMalloc(&w.xk_dev, sizeof(double2*) * n)))
-        return c->status_of(e, "multishift");
-    if (prec == CHDWF_PREC_F32 &&
-        ((e = cudaMalloc(&w.e, sizeof(float2) * g.kferm)) ||
-         (e = cudaMalloc(&w.rr, sizeof(float2) * g.kferm)) ||
-         (e = cudaMalloc(&w.p, sizeof(float2) * g.kferm)) ||
-         (e = cudaMalloc(&w.ap, sizeof(float2) * g.kferm)) ||
-         (e = cudaMalloc(&w.t32, sizeof(float2) * g.kferm))))
         return c->status_of(e, "multishift");
     cudaMemcpyAsync(w.xk_dev, x, sizeof(double2*) * n, cudaMemcpyHostToDevice, st);
     std::vector<double> anum(n + 1, 1.0);
@@ -203,32 +256,29 @@ extern "C" int chdwf_multishift_dev(chdwf_ctx* ctx, const void* Phi, float res, 
     cudaStreamSynchronize(st);
     const double phin = std::sqrt(phi2);
     *refine_iters = 0;
-    for (int k = 0; k < n; k++) {
-        double2* xk = (double2*)x[k];
-        double r2 = 0.0;
-        if ((e = true_residual(c, w, (const double2*)Phi, xk, sigma[k], hpin, imass, &r2)))
-            return c->status_of(e, "multishift residual");
-        double rel = std::sqrt(r2) / phin;
-        if (prec == CHDWF_PREC_F32) {
-            // defect correction: FP32 CG on the FP64 residual, added in FP64
-            for (int outer = 0; outer < 20 && rel > (double)res; outer++) {
-                const double rn = std::sqrt(r2);
-                k_ms_to32<<<nb_of(g.kferm), kThreads, 0, st>>>(w.rr, w.r, 1.0 / rn, g.kferm);
-                count_launches(1);
-                int it = 0;
-                if ((e = inner_cg32(c, w, (float)sigma[k], hpin, imass, 1e-4, 4 * kMaxIter, &it)))
-                    return c->status_of(e, "multishift refinement");
-                *refine_iters += it;
-                k_ms_add<<<nb_of(g.kferm), kThreads, 0, st>>>(xk, w.e, rn, g.kferm);
-                count_launches(1);
-                if ((e = true_residual(c, w, (const double2*)Phi, xk, sigma[k], hpin, imass, &r2)))
-                    return c->status_of(e, "multishift residual");
-                const double nrel = std::sqrt(r2) / phin;
-                if (!(nrel < rel)) { rel = nrel; break; }   // stagnation
-                rel = nrel;
-            }
+    if (prec == CHDWF_PREC_F32) {
+        if (!c->ms) c->ms = new PcgWork<float2>();
+        PcgWork<float2>& P = *c->ms;
+        PcgBatch<float2> B;                 // the largest part
+        for (int i = 0; i < np; i++)
+            if (!plane_ok(g) || !B.add(g, 0.0f, 0.0f, 0, imass, 1, pcg_sms()))
+                return c->status_of(cudaErrorInvalidValue, "multishift: lattice");
+        if ((e = P.reserve(B.units, 0, B.parts))) return c->status_of(e, "multishift: workspace");
+        for (int k0 = 0; k0 < n; k0 += np) {
+            const int m = n - k0 < np ? n - k0 : np;
+            if ((e = correct_part(c, w, P, (const double2*)Phi, phin, res, hpin, imass, k0, m, sigma,
+                                  x, true_res, refine_iters)))
+                return c->status_of(e, "multishift refinement");
         }
-        true_res[k] = rel;
+    } else {
+        for (int k = 0; k < n; k++) {
+            double r2 = 0.0;
+            true_residual(c, w, (const double2*)Phi, (const double2*)x[k], sigma[k], hpin, imass, w.r,
+                          w.part);
+            if ((e = run_sums(w.part, 1, reduce_blocks(g.kferm), &r2, st)))
+                return c->status_of(e, "multishift residual");
+            true_res[k] = std::sqrt(r2) / phin;
+        }
     }
     return c->status_of(cudaStreamSynchronize(st), "multishift");
 }

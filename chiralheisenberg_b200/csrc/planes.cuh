@@ -112,19 +112,23 @@ static_assert(kPlaneMaxThreads / 4 * kPlaneRegs <= 16384, "a block exceeds an SM
 // over the tiles of whole x rows that fit a block and the runs.  Halo reads
 // from L2 (2/ny + 2/nt of a site's) and the block barriers of large blocks
 // weigh a few per cent of a step, and a block's partial 3 cycles.
-inline PlanePlan plane_plan(const Geom& g, bool f32, int nsm) {
+//
+// block > 0: the kernel's blocks have that many threads whatever the tile
+// (several lattices in one launch, plane_cg.cuh); tiles then hold at most that.
+inline PlanePlan plane_plan(const Geom& g, bool f32, int nsm, int block = 0) {
+    const int most = block ? block : kPlaneMaxThreads;
     PlanePlan best{};
     double best_cost = 1e300;
     const int U = plane_units(g.Ls, f32);
     const int sx = (g.L + 63) / 64, nx = (g.L + sx - 1) / sx;
-    for (int nt = 1; nt <= g.Lt && nx * nt <= kPlaneMaxThreads; nt++)
-        for (int ny = 1; ny <= g.L && nx * ny * nt <= kPlaneMaxThreads; ny++) {
+    for (int nt = 1; nt <= g.Lt && nx * nt <= most; nt++)
+        for (int ny = 1; ny <= g.L && nx * ny * nt <= most; ny++) {
             const int warps = (nx * ny * nt + 31) / 32;
             const int tx = (g.L + nx - 1) / nx, ty = (g.L + ny - 1) / ny;
             const int tt = (g.Lt + nt - 1) / nt;
             const int64_t ntile = (int64_t)tx * ty * tt;
             const double halo = 1.0 + (ny < g.L ? 2.0 / ny : 0.0) + (nt < g.Lt ? 2.0 / nt : 0.0);
-            const int occ = 4 * (16384 / (32 * kPlaneRegs)) / warps;   // resident blocks an SM
+            const int occ = 4 * (16384 / (32 * kPlaneRegs)) / (block ? block / 32 : warps);
             for (int nrun = 1; nrun <= U; nrun++) {
                 const int64_t nitem = ntile * 2 * nrun;
                 if (nitem > 0x7fffffff) break;
@@ -309,7 +313,12 @@ __device__ __forceinline__ PlaneThread plane_thread(const PlanePlan& pl) {
     const int tid = threadIdx.x, r = tid / pl.nx, t = r / pl.ny;
     return PlaneThread{tid - r * pl.nx, r - t * pl.ny, t};
 }
-template <bool DAG, int IMASS, class V, class Real, class Epi>
+// SKIP: warps without a site return at once (no block barrier in epi).
+// S_LATE: the units above and below are loaded behind the diagonal term, which
+// suits kernels that would spill otherwise (CG in FP64 207 -> 193 ms for 32
+// solves; the multi-shift kernels with imass 1 are 3% faster with it off).
+template <bool DAG, int IMASS, bool SKIP = false, bool S_LATE = IMASS == 3, class V, class Real,
+          class Epi>
 __device__ __forceinline__ void plane_item(const V* in, const PlanePlan& pl, const PlaneThread& th,
                                            uint32_t item, const float* chif, Real diag, Real hpin, bool apbc,
                                            Epi& epi) {
@@ -325,6 +334,9 @@ __device__ __forceinline__ void plane_item(const V* in, const PlanePlan& pl, con
     const int lx = th.x, ly = th.y, lt = th.t;
     int x = (int)tix * pl.nx + lx, y = (int)tiy * pl.ny + ly, t = (int)tit * pl.nt + lt;
     const bool act = lt < pl.nt && x < L && y < L && t < Lt;
+    // whole warps only: behind a branch of single threads nothing is kept in
+    // uniform registers
+    if (SKIP && !__any_sync(0xffffffffu, act)) return;
     if (!act) { x = (int)tix * pl.nx; y = (int)tiy * pl.ny; t = (int)tit * pl.nt; }
     const uint32_t uL = (uint32_t)L, kv = pl.kvol, LL = uL * uL;
     const uint32_t site = (uint32_t)x + uL * ((uint32_t)y + uL * (uint32_t)t);
@@ -380,14 +392,17 @@ __device__ __forceinline__ void plane_item(const V* in, const PlanePlan& pl, con
         cur[0] = ld_unit(unit_at(p0, o_0)); cur[1] = ld_unit(unit_at(p1, o_0));
         cur[2] = ld_unit(unit_at(p2, o_0)); cur[3] = ld_unit(unit_at(p3, o_0));
         nx[0] = nx[1] = pv[0] = pv[1] = V{};
-        if (has_next) {
-            nx[0] = ld_unit(unit_at((DAG ? p0 : p2) + kv, o_0));
-            nx[1] = ld_unit(unit_at((DAG ? p1 : p3) + kv, o_0));
-        }
-        if (u > 0) {
-            pv[0] = ld_unit(unit_at((DAG ? p2 : p0) - kv, o_0));
-            pv[1] = ld_unit(unit_at((DAG ? p3 : p1) - kv, o_0));
-        }
+        auto load_s = [&] {                  // the units above and below
+            if (has_next) {
+                nx[0] = ld_unit(unit_at((DAG ? p0 : p2) + kv, o_0));
+                nx[1] = ld_unit(unit_at((DAG ? p1 : p3) + kv, o_0));
+            }
+            if (u > 0) {
+                pv[0] = ld_unit(unit_at((DAG ? p2 : p0) - kv, o_0));
+                pv[1] = ld_unit(unit_at((DAG ? p3 : p1) - kv, o_0));
+            }
+        };
+        if (!S_LATE) load_s();
         plane_kappa(acc, cur, diag);                                     // :2815-2829
         if (apbc) {                                                      // :2831-2876
             if (t == Lt - 1) { CHDWF_PLANE_LD(o_tp) hop<2, SF, true>(acc, r); }
@@ -395,6 +410,7 @@ __device__ __forceinline__ void plane_item(const V* in, const PlanePlan& pl, con
         }
 #undef CHDWF_PLANE_LD
         // s hops (:2879-2908; M^dagger :3313-3342)
+        if (S_LATE) load_s();
 #pragma unroll
         for (int d = 0; d < 2; d++) plane_shop<true>(acc[UP + d], cur[UP + d], nx[d], has_next);
 #pragma unroll
@@ -416,6 +432,19 @@ __device__ __forceinline__ void plane_item(const V* in, const PlanePlan& pl, con
         p0 += kv; p1 += kv; p2 += kv; p3 += kv;
         e += kv;
     }
+}
+
+// ---- between the ABI's layout and planes ---------------------------------------
+// Units are visited in plane order: coalesced on that side, Ls elements apart
+// on the other.  Once or twice a solve.
+struct PlaneUnit { int64_t e; int n; };   // first element in the ABI's layout, elements
+template <class T>
+__device__ __forceinline__ PlaneUnit plane_unit_of(const Geom& g, int U, int64_t i) {
+    constexpr int N = std::is_same<T, float2>::value ? 2 : 1;
+    const int64_t cu = i / g.kvol, site = i - cu * g.kvol;
+    const int c = (int)(cu / U), u = (int)(cu - (int64_t)c * U);
+    return PlaneUnit{(int64_t)N * u + (int64_t)g.Ls * site + g.cs * c,
+                     N == 2 && N * u + 1 < g.Ls ? 2 : 1};
 }
 
 }  // namespace chdwf

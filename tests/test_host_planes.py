@@ -20,10 +20,13 @@ from test_host_kernels import CSRC, RHMC_PROGRAM, _build
 PLANES_PROGRAM = RHMC_PROGRAM.split('#include "dwf_stencil.cuh"')[0] + r"""
 #include <cmath>
 #include <algorithm>
+static inline int __any_sync(unsigned, int p) { return p; }
 static inline float __fmaf_rn(float a, float b, float c) { return fmaf(a, b, c); }
 static inline double __fma_rn(double a, double b, double c) { return fma(a, b, c); }
 #include "planes.cuh"
 using namespace chdwf;
+static bool skip;
+static int block;
 struct Ld { const double2* p; double2 operator()(int64_t j) const { return p[j]; } };
 template <class V> struct Store {
     V* out; int* hits;
@@ -44,7 +47,8 @@ void sweep(const std::vector<V>& in, std::vector<V>& out, std::vector<int>& hits
     for (uint32_t it = 0; it < pl.nitem; it++)
         for (int t = 0; t < pl.threads; t++) {
             threadIdx.x = t;
-            plane_item<DAG, IMASS>(in.data(), pl, plane_thread(pl), it, chif, diag, hpin, apbc, st);
+            if (skip) plane_item<DAG, IMASS, true, true>(in.data(), pl, plane_thread(pl), it, chif, diag, hpin, apbc, st);
+            else plane_item<DAG, IMASS>(in.data(), pl, plane_thread(pl), it, chif, diag, hpin, apbc, st);
         }
 }
 template <class V, class Real, class F>
@@ -62,6 +66,8 @@ void all(const std::vector<V>& in, const PlanePlan& pl, const float* chif, Real 
 }
 int main(int argc, char** argv) {
     const int L = atoi(argv[1]), Lt = atoi(argv[2]), Ls = atoi(argv[3]), nsm = atoi(argv[4]);
+    block = atoi(argv[5]);
+    skip = block != 256;
     const Geom g = make_geom(L, Lt, Ls);
     std::vector<double2> R(g.kferm), ref(g.kferm);
     std::vector<float> chif(3 * g.kvol);
@@ -85,7 +91,7 @@ int main(int argc, char** argv) {
     long long bad = 0;
     double worst = 0.0;
     {
-        const PlanePlan pl = plane_plan(g, false, nsm);
+        const PlanePlan pl = plane_plan(g, false, nsm, block);
         std::vector<double2> in(plane_elems<double2>(g));
         auto at = [&](int c, int s, int site) { return ((int64_t)c * pl.U + s) * g.kvol + site; };
         for (int c = 0; c < 8; c++) for (int i = 0; i < g.kvol; i++) for (int s = 0; s < Ls; s++)
@@ -99,7 +105,7 @@ int main(int argc, char** argv) {
         });
     }
     {
-        const PlanePlan pl = plane_plan(g, true, nsm);
+        const PlanePlan pl = plane_plan(g, true, nsm, block);
         std::vector<cpair> in(plane_elems<float2>(g) / 2);
         auto half = [&](std::vector<cpair>& v, int c, int s, int site, bool im) -> float& {
             cpair& p = v[((int64_t)c * pl.U + s / 2) * g.kvol + site];
@@ -137,9 +143,12 @@ def planes_exe(tmp_path_factory):
 # nsm steers the plan: many SMs give small tiles and short runs, one SM large ones
 @pytest.mark.parametrize("L,Lt,Ls", [(4, 4, 4), (2, 2, 2), (3, 5, 3), (5, 4, 7), (6, 3, 5),
                                      (67, 2, 2), (9, 7, 2)])
+# block: 256 threads, the multi-shift solver's, and 192, the conjugate gradients',
+# whose warps without a site leave at once
 @pytest.mark.parametrize("nsm", [1, 148])
-def test_plane_stencil_matches_point_operator(planes_exe, L, Lt, Ls, nsm):
-    out = subprocess.run([planes_exe, *map(str, (L, Lt, Ls, nsm))], check=True,
+@pytest.mark.parametrize("block", [256, 192])
+def test_plane_stencil_matches_point_operator(planes_exe, L, Lt, Ls, nsm, block):
+    out = subprocess.run([planes_exe, *map(str, (L, Lt, Ls, nsm, block))], check=True,
                          capture_output=True, text=True).stdout
     bad, worst = out.split()
     assert int(bad) == 0, out
