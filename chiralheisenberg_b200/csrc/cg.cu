@@ -65,9 +65,10 @@ struct StaticCtl {
     PcgRun run;
 };
 constexpr size_t kStaticCtl = 1024;
-// element blocks: kferm units, kPcgThreads*kPcgUnits of them a block
+// stencil blocks twice, element blocks (kferm units, rounded up), alpha
 constexpr size_t kStaticParts =
-    2 * (size_t)kPcgMaxBlocks + kStaticMaxFerm / (kPcgThreads * kPcgUnits) + 1;
+    2 * (size_t)kPcgMaxBlocks +
+    kStaticMaxFerm / (kPcgThreads * pcg_units_thread<double2>()) + 2;
 static_assert(sizeof(StaticCtl) <= kStaticCtl, "the control block outgrew its place");
 static_assert(kStaticParts * sizeof(double) <= 64 * 1024, "the partials outgrew their place");
 constexpr size_t kStaticBytes = kStaticCtl + 64 * 1024 +    // control block, partials

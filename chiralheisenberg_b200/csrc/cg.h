@@ -6,13 +6,6 @@ namespace chdwf {
 
 template <class T> struct PcgWork;      // plane_cg.cuh
 
-// Control block of the single-precision CGNE of hmc.cu.
-struct CgCtl {
-    int nx, done, iters, niterc;
-    float alpha, beta, alphan, betad, resid, pad2_;
-    unsigned count1, count2;
-};
-
 struct CgWork {
     PcgWork<double2>* w = nullptr;
     ~CgWork();

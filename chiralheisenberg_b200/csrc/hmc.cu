@@ -21,7 +21,6 @@
 #include <string>
 #include <vector>
 
-#include "cg.h"
 #include "chdwf_hmc.h"
 #include "common.cuh"
 #include "internal.h"
@@ -91,6 +90,32 @@ __device__ __forceinline__ Elem elem_of(const Geom& g, int64_t j) {
     return e;
 }
 
+// Wall coupling (:1549-1679, :1897-2026) of one element: group A at s=kthird,
+// else group B at s=1; r and ro are the other wall's element of the same and
+// of the other flavour.  Stage 1 couples equal flavours through spm1, stage 2
+// the other flavour through spm2 (flavour 2: conjg(spm2)).
+template <bool DAG, int IMASS>
+__device__ __forceinline__ float2 hmc_wall(float2 phi, bool grpA, int f, float2 r, float2 ro,
+                                           float c1, float c2, float c3) {
+#pragma unroll
+    for (int stage = 0; stage < 2; stage++) {
+        float2 spm;
+        int sg;
+        if (IMASS == 1) {
+            spm = stage == 0 ? make_float2(c3, 0.0f) : make_float2(c1, -c2);
+            sg = (stage == 0 && f == 1) ? -1 : 1;
+        } else {
+            if (stage == 0) spm = make_float2(0.0f, DAG ? -c3 : c3);
+            else spm = DAG ? make_float2(-c2, -c1) : make_float2(c2, c1);
+            const int first = (grpA == !DAG) ? -1 : 1;    // sign for flavour 1
+            sg = f == 0 ? first : -first;
+        }
+        const float2 t = stage == 0 ? fc_mul(spm, r) : fc_mul(f == 0 ? spm : fc_conj(spm), ro);
+        phi = sg > 0 ? fc_add(phi, t) : fc_sub(phi, t);
+    }
+    return phi;
+}
+
 // One element (s, site, d, f) of Phi = M R (DAG false: mh/cheisdwf_hmc.f:1334-1681)
 // or Phi = M^dagger R (DAG true: :1683-2028), updates applied in the order of
 // the reference's sweeps.
@@ -146,35 +171,15 @@ __device__ float2 hmc_element(const float2* __restrict__ R, const Geom& g, int s
     } else if (s > 0) {
         phi = fc_sub(phi, at(s - 1, i0, d, f));
     }
-    // wall coupling (:1549-1679, :1897-2026).  Group A: s=kthird, the pair
-    // that takes s+1 (M: Dirac 3,4), reading s=1; group B: s=1, the other
-    // pair, reading s=kthird.  Stage 1 couples equal flavours through spm1,
-    // stage 2 the other flavour through spm2 (flavour 2: conjg(spm2)).
+    // walls.  Group A: s=kthird, the pair that takes s+1 (M: Dirac 3,4),
+    // reading s=1; group B: s=1, the other pair, reading s=kthird.
     int sr = -1;
     if (s == Ls - 1 && from_up) sr = 0;
     else if (s == 0 && !from_up) sr = Ls - 1;
     if (sr >= 0) {
         const bool grpA = sr == 0;
         const float c1 = chi[i0], c2 = chi[kvol + i0], c3 = chi[2 * kvol + i0];
-#pragma unroll
-        for (int stage = 0; stage < 2; stage++) {
-            float2 spm;
-            int sg;
-            if (IMASS == 1) {
-                spm = stage == 0 ? make_float2(c3, 0.0f) : make_float2(c1, -c2);
-                sg = (stage == 0 && f == 1) ? -1 : 1;
-            } else {
-                if (stage == 0) spm = make_float2(0.0f, DAG ? -c3 : c3);
-                else spm = DAG ? make_float2(-c2, -c1) : make_float2(c2, c1);
-                const int first = (grpA == !DAG) ? -1 : 1;    // sign for flavour 1
-                sg = f == 0 ? first : -first;
-            }
-            float2 t;
-            if (stage == 0) t = fc_mul(spm, at(sr, i0, d, f));
-            else if (f == 0) t = fc_mul(spm, at(sr, i0, d, 1));
-            else t = fc_mul(fc_conj(spm), at(sr, i0, d, 0));
-            phi = sg > 0 ? fc_add(phi, t) : fc_sub(phi, t);
-        }
+        phi = hmc_wall<DAG, IMASS>(phi, grpA, f, at(sr, i0, d, f), at(sr, i0, d, 1 - f), c1, c2, c3);
     }
     return phi;
 }
@@ -191,87 +196,45 @@ __global__ void __launch_bounds__(kThreads) k_hmc_dslash(float2* __restrict__ ou
 }
 
 // ---- congrad (mh/cheisdwf_hmc.f:625-716) ----------------------------------
-struct HcgArgs {
-    Geom g;
-    float2 *x, *p, *r, *x1;
-    const float* chi;
-    float diag;
-    int apbc;
-    CgCtl* ctl;
-    double* part;
-    int* hflag;
+// On planes, three kernels an iteration (plane_cg.cuh): 16^3x16, 436
+// iterations, 10.9 ms against 22.5 with one thread an element in the ABI's
+// layout, three direct launches and two last-block sums an iteration.
+}  // namespace
+}  // namespace chdwf
+#include "hmc_planes.cuh"
+#include "plane_cg.cuh"
+namespace chdwf {
+template <> struct PcgOp<hmc32> {
+    static constexpr bool kShifted = false;
+    static constexpr bool kLateX = true;
+    template <bool DAG, int IMASS, class Epi>
+    static __device__ __forceinline__ void item(const float2* in, const PlanePlan& pl,
+                                                const PlaneThread& th, uint32_t it,
+                                                const float* chif, float diag, float, bool apbc,
+                                                Epi& epi) {
+        hmc_plane_item<DAG, IMASS>(in, pl, th, it, chif, diag, apbc, epi);
+    }
+    static __device__ __forceinline__ float2 axpy(float s, float2 a, float2 b) {
+        return fc_add(b, fc_scal(s, a));
+    }
+    static __device__ __forceinline__ double norm2(float2 v) {
+        return (double)__fmul_rn(v.x, v.x) + (double)__fmul_rn(v.y, v.y);
+    }
 };
+namespace {
 
-// x1 = M p ; alphad = |x1|^2 ; alpha = alphan/alphad  (:657-667)
-template <int IMASS>
-__global__ void __launch_bounds__(kThreads) k_hcg1(HcgArgs a) {
-    CgCtl* c = a.ctl;
-    if (c->done) return;
-    const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    double loc = 0.0;
-    if (j < a.g.kferm) {
-        const Elem e = elem_of(a.g, j);
-        const float2 v = hmc_element<false, IMASS>(a.p, a.g, e.s, e.x, e.y, e.t, e.d, e.f, a.chi,
-                                                   a.diag, a.apbc != 0);
-        a.x1[j] = v;
-        loc = (double)__fmul_rn(v.x, v.x) + (double)__fmul_rn(v.y, v.y);
-    }
-    double tot;
-    if (!last_block_total<kThreads>(loc, a.part, &c->count1, &tot)) return;
-    if (threadIdx.x == 0 && c->nx > 1) c->alpha = c->alphan / (float)tot;
+// ABI layout -> planes (p = x, r = Phi), and back
+__global__ void k_hcg_in(float2* __restrict__ p, float2* __restrict__ r,
+                         const float2* __restrict__ x, const float2* __restrict__ phi, Geom g) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= g.kferm) return;
+    const int64_t e = plane_unit_of<double2>(g, g.Ls, i).e;
+    p[i] = x[e];
+    r[i] = phi[e];
 }
-
-// x2 = M^dagger x1 ; x += alpha p (nx > 1) ; r -= alpha x2 ; betan = |r|^2,
-// beta, stopping test  (:671-704)
-template <int IMASS>
-__global__ void __launch_bounds__(kThreads) k_hcg2(HcgArgs a) {
-    CgCtl* c = a.ctl;
-    if (c->done) return;
-    const int nx = c->nx;
-    const float alpha = c->alpha;
-    const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    double loc = 0.0;
-    if (j < a.g.kferm) {
-        const Elem e = elem_of(a.g, j);
-        const float2 v = hmc_element<true, IMASS>(a.x1, a.g, e.s, e.x, e.y, e.t, e.d, e.f, a.chi,
-                                                  a.diag, a.apbc != 0);
-        if (nx > 1) a.x[j] = fc_add(a.x[j], fc_scal(alpha, a.p[j]));
-        const float2 r = fc_sub(a.r[j], fc_scal(alpha, v));
-        a.r[j] = r;
-        loc = (double)__fmul_rn(r.x, r.x) + (double)__fmul_rn(r.y, r.y);
-    }
-    double tot;
-    if (!last_block_total<kThreads>(loc, a.part, &c->count2, &tot)) return;
-    if (threadIdx.x == 0) {
-        const float betan = (float)tot;
-        float beta = betan / c->betad;
-        c->betad = betan;
-        c->alphan = betan;
-        if (nx == 1) beta = 0.0f;
-        c->beta = beta;
-        if (betan < c->resid) {
-            c->done = 1;
-            c->iters = nx;
-        } else if (nx >= c->niterc) {
-            c->done = 2;
-            c->iters = nx;
-        }
-        if (!(betan == betan)) { c->done = 3; c->iters = nx; }
-        if (c->done && a.hflag) {
-            *(volatile int*)a.hflag = c->done;
-            __threadfence_system();
-        }
-        if (!c->done) c->nx = nx + 1;
-    }
-}
-
-// p = r + beta p  (:700-702)
-__global__ void __launch_bounds__(kThreads) k_hcg3(HcgArgs a) {
-    CgCtl* c = a.ctl;
-    if (c->done) return;
-    const float beta = c->beta;
-    const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (j < a.g.kferm) a.p[j] = fc_add(a.r[j], fc_scal(beta, a.p[j]));
+__global__ void k_hcg_out(float2* __restrict__ x, const float2* __restrict__ xs, Geom g) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i < g.kferm) x[plane_unit_of<double2>(g, g.Ls, i).e] = xs[i];
 }
 
 // ---- force, Hamiltonian and the leapfrog updates ---------------------------
@@ -391,12 +354,10 @@ struct chdwf_hmc {
     cudaStream_t st = nullptr;
     float *chi = nullptr, *chit = nullptr, *pp = nullptr, *dS = nullptr, *chi_io = nullptr;
     float2 *Phi = nullptr, *X0 = nullptr, *X1 = nullptr, *R = nullptr;
-    float2 *cp = nullptr, *cr = nullptr, *cx1 = nullptr;
-    float* gauss = nullptr;
+    chdwf::PcgWork<chdwf::hmc32> cg;
     double* part = nullptr;
-    chdwf::CgCtl* ctl = nullptr;
-    int* hflag_host = nullptr;
-    int* hflag_dev = nullptr;
+    // the Gaussian numbers of the heatbath, in the solver's vectors
+    float* gauss() const { return (float*)cg.vec; }
     chdwf::Rng rng;
     int isweep = 0, itot = 0, naccp = 0;
     float action = 0.0f, gaction = 0.0f, paction = 0.0f;
@@ -435,65 +396,30 @@ void launch_dslash(chdwf_hmc* h, bool dag, int imass, float2* out, const float2*
 // converged, 1 at the cap kthird*kvol, 2 non-finite.
 cudaError_t hcg_solve(chdwf_hmc* h, const float2* phi, float res, int imass, const float* chi,
                       float2* x, int* itercg, int* status) {
+    using namespace chdwf;
     const Geom& g = h->g;
-    chdwf::CgCtl hc;
-    memset(&hc, 0, sizeof(hc));
-    hc.nx = 1;
-    hc.alpha = 1.0f;                                                    // :651-652
-    hc.betad = 1.0f;
-    hc.resid = (float)g.kferm * res * res;                              // :638
-    hc.niterc = (int)(g.Ls * (int64_t)g.kvol);
-    cudaError_t e;
-    if ((e = cudaMemcpyAsync(h->ctl, &hc, sizeof(hc), cudaMemcpyHostToDevice, h->st))) return e;
-    *h->hflag_host = 0;
-    cudaMemcpyAsync(h->cp, x, sizeof(float2) * g.kferm, cudaMemcpyDeviceToDevice, h->st);   // :647-650
-    cudaMemcpyAsync(h->cr, phi, sizeof(float2) * g.kferm, cudaMemcpyDeviceToDevice, h->st);
-    chdwf::HcgArgs a;
-    memset(&a, 0, sizeof(a));
-    a.g = g;
-    a.x = x; a.p = h->cp; a.r = h->cr; a.x1 = h->cx1;
-    a.chi = chi;
-    a.diag = h->diag();
-    a.apbc = 1;
-    a.ctl = h->ctl;
-    a.part = h->part;
-    a.hflag = h->hflag_dev;
-    const unsigned nb = chdwf::nblk(g.kferm);
-    const int chunk = 16;
-    cudaEvent_t ev[2];
-    cudaEventCreateWithFlags(&ev[0], cudaEventDisableTiming);
-    cudaEventCreateWithFlags(&ev[1], cudaEventDisableTiming);
-    int64_t launched = 0;
-    int nchunk = 0;
-    const int64_t cap = hc.niterc;
-    while (launched < cap) {
-        for (int c = 0; c < chunk && launched < cap; c++, launched++) {
-            if (imass == 3) {
-                chdwf::k_hcg1<3><<<nb, chdwf::kThreads, 0, h->st>>>(a);
-                chdwf::k_hcg2<3><<<nb, chdwf::kThreads, 0, h->st>>>(a);
-            } else {
-                chdwf::k_hcg1<1><<<nb, chdwf::kThreads, 0, h->st>>>(a);
-                chdwf::k_hcg2<1><<<nb, chdwf::kThreads, 0, h->st>>>(a);
-            }
-            chdwf::k_hcg3<<<nb, chdwf::kThreads, 0, h->st>>>(a);
-            chdwf::count_launches(3);
-        }
-        cudaEventRecord(ev[nchunk & 1], h->st);
-        if (nchunk >= 1) {
-            cudaEventSynchronize(ev[(nchunk - 1) & 1]);
-            if (*(volatile int*)h->hflag_host) break;
-        }
-        nchunk++;
-    }
-    cudaEventDestroy(ev[0]);
-    cudaEventDestroy(ev[1]);
-    if ((e = cudaGetLastError())) return e;
-    chdwf::CgCtl hr;
-    if ((e = cudaMemcpyAsync(&hr, h->ctl, sizeof(hr), cudaMemcpyDeviceToHost, h->st))) return e;
-    if ((e = cudaStreamSynchronize(h->st))) return e;
-    *itercg = hr.iters;
-    *status = hr.done == 1 ? 0 : (hr.done == 2 ? 1 : 2);
-    return cudaSuccess;
+    PcgBatch<hmc32> B;
+    if (!B.add(g, h->diag(), 0.0f, 1, imass, 0, pcg_sms())) return cudaErrorInvalidValue;
+    h->cg.bind(B, chi);
+    const unsigned nb = nblk(g.kferm);
+    float2* p = h->cg.vec;
+    const size_t bytes = sizeof(float2) * g.kferm;
+    k_hcg_in<<<nb, kThreads, 0, h->st>>>(p, p + g.kferm, x, phi, g);      // :647-650
+    cudaMemcpyAsync(x, p, bytes, cudaMemcpyDeviceToDevice, h->st);        // x in planes too
+    PcgDyn<hmc32> d;
+    memset(&d, 0, sizeof(d));
+    d.x = x;
+    d.resid = (float)g.kferm * res * res;                                // :638
+    d.niterc = (int)(g.Ls * (int64_t)g.kvol);
+    std::vector<PcgSlot> slots(1, pcg_congrad_slot());                   // :651-652
+    cudaError_t e = h->cg.solve(B, {d}, slots, h->st);
+    if (e) return e;
+    k_hcg_out<<<nb, kThreads, 0, h->st>>>(p, x, g);
+    cudaMemcpyAsync(x, p, bytes, cudaMemcpyDeviceToDevice, h->st);
+    count_launches(2);
+    *itercg = slots[0].iters;
+    *status = pcg_status(slots[0]);
+    return cudaGetLastError();
 }
 
 void launch_derivs(chdwf_hmc* h, int imass, const float2* X1, const float* chi, float* dS) {
@@ -596,17 +522,12 @@ int chdwf_hmc_create(chdwf_hmc** out, int ksize, int ksizet, int kthird, float d
     if (!e) e = dalloc(&h->X0, nf);
     if (!e) e = dalloc(&h->X1, nf);
     if (!e) e = dalloc(&h->R, nf);
-    if (!e) e = dalloc(&h->cp, nf);
-    if (!e) e = dalloc(&h->cr, nf);
-    if (!e) e = dalloc(&h->cx1, nf);
-    if (!e) e = dalloc(&h->gauss, 16 * (size_t)h->g.kvol * kthird);
-    const int64_t nbmax = std::max<int64_t>(chdwf::nblk(nf), chdwf::kHfBlocks);
-    if (!e) e = dalloc(&h->part, nbmax + 64);
-    if (!e) e = dalloc(&h->ctl, 1);
-    if (!e) e = cudaHostAlloc((void**)&h->hflag_host, sizeof(int), cudaHostAllocMapped);
-    if (!e) e = cudaHostGetDevicePointer((void**)&h->hflag_dev, h->hflag_host, 0);
+    chdwf::PcgBatch<chdwf::hmc32> B;
+    if (!e && (!chdwf::plane_ok(h->g) || !B.add(h->g, h->diag(), 0.0f, 1, imass, 0, chdwf::pcg_sms())))
+        e = cudaErrorInvalidValue;
+    if (!e) e = h->cg.reserve(B.units, 0, B.parts);
+    if (!e) e = dalloc(&h->part, chdwf::kHfBlocks);
     if (!e) e = cudaMemsetAsync(h->chi, 0, sizeof(float) * n3, h->st);
-    if (!e) e = cudaMemsetAsync(h->ctl, 0, sizeof(chdwf::CgCtl), h->st);
     if (!e) e = cudaStreamSynchronize(h->st);
     if (e) {
         g_hmc_create_err = std::string("chdwf_hmc_create: ") + cudaGetErrorString(e);
@@ -622,11 +543,10 @@ void chdwf_hmc_destroy(chdwf_hmc* h) {
     if (!h) return;
     cudaSetDevice(h->device);
     if (h->st) cudaStreamSynchronize(h->st);
-    for (float* p : {h->chi, h->chit, h->pp, h->dS, h->chi_io, h->gauss}) if (p) cudaFree(p);
-    for (float2* p : {h->Phi, h->X0, h->X1, h->R, h->cp, h->cr, h->cx1}) if (p) cudaFree(p);
+    for (float* p : {h->chi, h->chit, h->pp, h->dS, h->chi_io}) if (p) cudaFree(p);
+    for (float2* p : {h->Phi, h->X0, h->X1, h->R}) if (p) cudaFree(p);
     if (h->part) cudaFree(h->part);
-    if (h->ctl) cudaFree(h->ctl);
-    if (h->hflag_host) cudaFreeHost(h->hflag_host);
+    h->cg.release();
     if (h->st) cudaStreamDestroy(h->st);
     delete h;
 }
@@ -721,9 +641,9 @@ int chdwf_hmc_sweep(chdwf_hmc* h, chdwf_hmc_record* rec) {
     // pseudofermion heatbath: 8*kthird gauss0 calls, Phi = M^dagger R (:154-165)
     std::vector<float> gauss(16 * (size_t)kvol * g.Ls);
     for (int c = 0; c < 8 * g.Ls; c++) h->rng.gauss0(kvol, gauss.data() + (size_t)c * 2 * kvol);
-    CKC(cudaMemcpyAsync(h->gauss, gauss.data(), sizeof(float) * gauss.size(),
+    CKC(cudaMemcpyAsync(h->gauss(), gauss.data(), sizeof(float) * gauss.size(),
                         cudaMemcpyHostToDevice, h->st), "hmc_sweep");
-    chdwf::k_hmc_noise<<<chdwf::nblk(g.kferm), chdwf::kThreads, 0, h->st>>>(h->R, h->gauss, g);
+    chdwf::k_hmc_noise<<<chdwf::nblk(g.kferm), chdwf::kThreads, 0, h->st>>>(h->R, h->gauss(), g);
     chdwf::count_launches(1);
     launch_dslash(h, true, h->imass, h->Phi, h->R, h->chit);
     cudaMemcpyAsync(h->X0, h->Phi, sizeof(float2) * g.kferm, cudaMemcpyDeviceToDevice, h->st);  // :167-175

@@ -56,10 +56,11 @@ __global__ void __launch_bounds__(kPcgThreads) k_ms_planes(cpair* p, cpair* rp, 
                                                            double* part, Geom g, int U,
                                                            const double2* __restrict__ r,
                                                            double scale) {
+    constexpr int kN = pcg_units_thread<float2>();
     const int64_t nu = 8 * (int64_t)U * g.kvol;
-    const int64_t i0 = (int64_t)blockIdx.x * (kPcgThreads * kPcgUnits) + threadIdx.x;
+    const int64_t i0 = (int64_t)blockIdx.x * (kPcgThreads * kN) + threadIdx.x;
     double loc = 0.0;
-    for (int q = 0; q < kPcgUnits; q++) {
+    for (int q = 0; q < kN; q++) {
         const int64_t i = i0 + q * kPcgThreads;
         if (i >= nu) break;
         const PlaneUnit pu = plane_unit_of<float2>(g, U, i);

@@ -1,18 +1,23 @@
 // plane_cg.cuh -- conjugate gradients on M^dagger M (+ sigma) for a batch of
 // independent systems whose vectors are planes (planes.cuh).
 //
-// Two rules share the kernels:
+// Three kinds of system share the kernels:
 //   T = double2  congrad (rhmc/cheisdwf.f:1064-1157): FP64 vectors, REAL*4
 //                scalars, sums formed in FP64 and rounded once (the reference
 //                adds element by element in REAL*4, an order that no parallel
 //                sum can follow), the reference's stopping rule;
+//   T = hmc32    congrad of the HMC predecessor (hmc_planes.cuh): the same
+//                rule on FP32 vectors with every operation rounded;
 //   T = float2   the inner solver of the per-shift defect correction: FP32
 //                vectors, FP64 scalars, (M^dagger M + sigma) e = r to a
 //                relative residual.
 // One iteration is three kernels over the blocks of all systems:
 //   k_pcg1  x1 = M p, |x1|^2
-//   k_pcg2  x += alpha p, r -= alpha (M^dagger x1 + sigma p), |r|^2
+//   k_pcg2  r -= alpha (M^dagger x1 + sigma p), |r|^2, x += alpha p
 //   k_pcg3  p = r + beta p (and |p|^2 where sigma enters), the scalars
+// x is updated beside the stencil, whose latencies hide it (in k_pcg3, which
+// moves bytes only, 32 FP64 solves took 202 ms instead of 193); hmc32 does it
+// in k_pcg3, where it spares registers and a load of p (11.6 -> 10.8 ms).
 // A block leaves its partial; the kernel that needs a sum adds the system's
 // partials itself, in one order.  A system's scalars are kept in two slots by
 // the parity of the iteration: k_pcg3 reads one while its first block of the
@@ -39,7 +44,11 @@ namespace chdwf {
 
 constexpr int kPcgThreads = 192;      // a block; 4 an SM at kPlaneRegs
 constexpr int kPcgMaxBlocks = 2048;   // stencil blocks of one system
-constexpr int kPcgUnits = 4;          // units a thread takes in k_pcg3
+// bytes of a vector a thread takes in k_pcg3
+constexpr int kPcgBytes = 64;
+template <class T> constexpr int pcg_units_thread() {
+    return kPcgBytes / (int)sizeof(typename unit_of<T>::type);
+}
 
 struct PcgSlot {
     float alphan, betad;     // congrad
@@ -79,7 +88,7 @@ struct PcgArgs {
     PcgGeo<T> geo[kPcgGeo];
     int64_t vec0[kPcgSys];            // system's vectors p, r, x1 (units from vec)
     int chi0[kPcgSys];                // its REAL*4 chi (from chif)
-    int part0[kPcgSys];               // its partials of |x1|^2, |r|^2, |p|^2 (from part)
+    int part0[kPcgSys];               // its partials of |x1|^2, |r|^2, |p|^2, and alpha (from part)
     int blk0[kPcgSys + 1], eblk0[kPcgSys + 1];
     unsigned char gid[kPcgSys];
     int nsys, ngeo;
@@ -112,8 +121,34 @@ __device__ __forceinline__ void pcg_wait() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-template <class V>
+// What a kind of system brings: its stencil, and s*a + b of its updates.
+// congrad's without fused multiply-add, as the reference rounds them; the FP32
+// correction's with.
+template <class T> struct PcgOp {
+    typedef typename unit_of<T>::type V;
+    typedef typename real_of<T>::type Real;
+    static constexpr bool kShifted = std::is_same<T, float2>::value;
+    static constexpr bool kLateX = false;              // x in k_pcg3
+    template <bool DAG, int IMASS, class Epi>
+    static __device__ __forceinline__ void item(const V* in, const PlanePlan& pl,
+                                                const PlaneThread& th, uint32_t it,
+                                                const float* chif, Real diag, Real hpin,
+                                                bool apbc, Epi& epi) {
+        plane_item<DAG, IMASS, true, std::is_same<T, double2>::value || IMASS == 3>(
+            in, pl, th, it, chif, diag, hpin, apbc, epi);
+    }
+    static __device__ __forceinline__ double2 axpy(double s, double2 a, double2 b) {
+        return zadd(b, zscal(s, a));
+    }
+    static __device__ __forceinline__ cpair axpy(float s, const cpair& a, const cpair& b) {
+        return zaxpy(s, a, b);
+    }
+    static __device__ __forceinline__ double norm2(const V& v) { return unit_norm2(v); }
+};
+
+template <class T>
 struct PcgEpi1 {
+    typedef typename unit_of<T>::type V;
     V* x1;
     double loc;
     __device__ __forceinline__ bool operator()(V acc[4], int64_t e, int64_t cst, uint32_t o,
@@ -122,21 +157,15 @@ struct PcgEpi1 {
 #pragma unroll
         for (int d = 0; d < 4; d++) {
             st_unit(unit_at(x1 + e + d * cst, o), acc[d]);
-            loc += unit_norm2(acc[d]);
+            loc += PcgOp<T>::norm2(acc[d]);
         }
         return true;
     }
 };
-// congrad's updates without fused multiply-add, as the reference rounds them;
-// the FP32 correction's with
-__device__ __forceinline__ double2 pcg_axpy(double s, double2 a, double2 b) {
-    return zadd(b, zscal(s, a));
-}
-__device__ __forceinline__ cpair pcg_axpy(float s, const cpair& a, const cpair& b) {
-    return zaxpy(s, a, b);
-}
-template <class V, class Real>
+template <class T>
 struct PcgEpi2 {
+    typedef typename unit_of<T>::type V;
+    typedef typename real_of<T>::type Real;
     const V* p;
     V *r, *x;
     Real alpha, sigma;
@@ -145,19 +174,20 @@ struct PcgEpi2 {
     __device__ __forceinline__ bool operator()(V acc[4], int64_t e, int64_t cst, uint32_t o,
                                                bool act, int, uint32_t) {
         if (!act) return true;
-        constexpr bool SH = std::is_same<V, cpair>::value;
 #pragma unroll
         for (int d = 0; d < 4; d++) {
             const int64_t ed = e + d * cst;
             V a = acc[d];
-            if (SH || upd) {
+            if (!PcgOp<T>::kLateX && (PcgOp<T>::kShifted || upd)) {
                 const V pv = ld_unit(unit_at(p + ed, o));
-                if (SH) a = pcg_axpy(sigma, pv, a);
-                if (upd) st_unit(unit_at(x + ed, o), pcg_axpy(alpha, pv, ld_unit(unit_at(x + ed, o))));
+                if (PcgOp<T>::kShifted) a = PcgOp<T>::axpy(sigma, pv, a);
+                if (upd)
+                    st_unit(unit_at(x + ed, o),
+                            PcgOp<T>::axpy(alpha, pv, ld_unit(unit_at(x + ed, o))));
             }
-            const V rv = pcg_axpy(-alpha, a, ld_unit(unit_at(r + ed, o)));
+            const V rv = PcgOp<T>::axpy(-alpha, a, ld_unit(unit_at(r + ed, o)));
             st_unit(unit_at(r + ed, o), rv);
-            loc += unit_norm2(rv);
+            loc += PcgOp<T>::norm2(rv);
         }
         return true;
     }
@@ -168,8 +198,8 @@ __device__ __forceinline__ void pcg_sweep(const PcgArgs<T>& a, const PcgGeo<T>& 
                                           const typename unit_of<T>::type* in,
                                           const PlaneThread& th, Epi& epi) {
     for (uint32_t it = (uint32_t)b; it < G.pl.nitem; it += (uint32_t)G.nblk)
-        plane_item<DAG, IMASS, true, std::is_same<T, double2>::value || IMASS == 3>(
-            in, G.pl, th, it, a.chif + a.chi0[s], G.diag, G.hpin, G.apbc != 0, epi);
+        PcgOp<T>::template item<DAG, IMASS>(in, G.pl, th, it, a.chif + a.chi0[s], G.diag, G.hpin,
+                                            G.apbc != 0, epi);
 }
 template <class T>
 __device__ __forceinline__ int64_t pcg_units(const PlanePlan& pl) {
@@ -186,7 +216,7 @@ __global__ void __maxnreg__(kPlaneRegs) k_pcg1(const __grid_constant__ PcgArgs<T
     V* p = a.vec + a.vec0[s];
     pcg_wait();
     if (a.slot[2 * s + (k & 1)].done) return;
-    PcgEpi1<V> epi{p + 2 * pcg_units<T>(G.pl), 0.0};
+    PcgEpi1<T> epi{p + 2 * pcg_units<T>(G.pl), 0.0};
     pcg_sweep<false, IMASS>(a, G, s, b, p, th, epi);
     __shared__ double sh[32];
     const double loc = block_sum_any(epi.loc, sh);
@@ -203,17 +233,17 @@ __global__ void __maxnreg__(kPlaneRegs) k_pcg2(const __grid_constant__ PcgArgs<T
     const PlaneThread th = plane_thread(G.pl);
     V* p = a.vec + a.vec0[s];
     double* part = a.part + a.part0[s];
-    PcgEpi2<V, Real> epi{p, p + pcg_units<T>(G.pl), a.dyn[s].x, (Real)1, a.dyn[s].sigma, true, 0.0};
+    PcgEpi2<T> epi{p, p + pcg_units<T>(G.pl), a.dyn[s].x, (Real)1, a.dyn[s].sigma, true, 0.0};
     pcg_wait();
     const PcgSlot c = a.slot[2 * s + (k & 1)];
     if (c.done) return;
     const double tot = sum_partials_any(part, G.nblk);
-    if constexpr (std::is_same<T, double2>::value) {
+    if constexpr (!PcgOp<T>::kShifted) {
         // alphad = |x1|^2 ; alpha = alphan/alphad from the second iteration on
         // (:1093-1117)
         const int nx = a.run->base + k + 1;
         epi.upd = nx > 1;
-        if (nx > 1) epi.alpha = (double)(c.alphan / (float)tot);
+        if (nx > 1) epi.alpha = (Real)(c.alphan / (float)tot);
     } else {
         // p^dagger (M^dagger M + sigma) p = |M p|^2 + sigma |p|^2; a value that
         // is not positive ends the system in k_pcg3
@@ -221,6 +251,7 @@ __global__ void __maxnreg__(kPlaneRegs) k_pcg2(const __grid_constant__ PcgArgs<T
         const double pap = tot + (double)epi.sigma * sum_partials_any(part + 2 * G.nblk, G.neblk);
         epi.alpha = pap > 0.0 ? (float)(c.rr / pap) : 0.0f;
     }
+    if (PcgOp<T>::kLateX && b == 0 && threadIdx.x == 0) part[2 * G.nblk + G.neblk] = (double)epi.alpha;
     pcg_sweep<true, IMASS>(a, G, s, b, p + 2 * pcg_units<T>(G.pl), th, epi);
     __shared__ double sh[32];
     const double loc = block_sum_any(epi.loc, sh);
@@ -240,18 +271,37 @@ __global__ void __launch_bounds__(kPcgThreads) k_pcg3(const __grid_constant__ Pc
     const float resid = a.dyn[s].resid;
     const double rstop = a.dyn[s].rstop;
     const int niterc = a.dyn[s].niterc;
+    V* x = a.dyn[s].x;
+    constexpr bool LX = PcgOp<T>::kLateX;
+    constexpr int N = pcg_units_thread<T>();
+    const int64_t i0 = (int64_t)b * (kPcgThreads * N) + threadIdx.x;
+    V pv[N], rv[N], xv[LX ? N : 1];
+    auto load = [&] {
+#pragma unroll
+        for (int q = 0; q < N; q++) {
+            const int64_t i = i0 + q * kPcgThreads;
+            if (i >= nu) break;
+            pv[q] = ld_unit(p + i);
+            rv[q] = ld_unit(r + i);
+            if (LX) xv[q] = ld_unit(x + i);
+        }
+    };
     pcg_wait();
+    // hmc32: on their way while the sum is formed (12.2 -> 10.9 ms); the others'
+    // batches have blocks enough to hide it, and are 5% slower so
+    if (LX) load();
     const PcgSlot c = a.slot[2 * s + (k & 1)];
     PcgSlot* next = a.slot + 2 * s + ((k + 1) & 1);
     if (c.done) {
         if (b == 0 && threadIdx.x == 0) *next = c;
         return;
     }
+    const Real alpha = LX ? (Real)part[2 * G.nblk + G.neblk] : (Real)0;
     const double tot = sum_partials_any(part + G.nblk, G.nblk);
     const int nx = a.run->base + k + 1;
     PcgSlot n = c;
     Real beta;
-    if constexpr (std::is_same<T, double2>::value) {
+    if constexpr (!PcgOp<T>::kShifted) {
         const float betan = (float)tot;                    // :1133-1141
         float bt = betan / c.betad;
         n.betad = betan;
@@ -260,7 +310,7 @@ __global__ void __launch_bounds__(kPcgThreads) k_pcg3(const __grid_constant__ Pc
         if (betan < resid) n.done = 1;
         else if (nx >= niterc) n.done = 2;
         if (!(betan == betan)) n.done = 3;
-        beta = (double)bt;
+        beta = (Real)bt;
     } else {
         n.rr = tot;
         beta = (float)(tot / c.rr);
@@ -276,19 +326,25 @@ __global__ void __launch_bounds__(kPcgThreads) k_pcg3(const __grid_constant__ Pc
             __threadfence_system();
         }
     }
-    if (n.done) return;
-    // p = r + beta p (:1147-1150)
-    const int64_t i0 = (int64_t)b * (kPcgThreads * kPcgUnits) + threadIdx.x;
+    if (!LX) {
+        if (n.done) return;
+        load();
+    }
+    // x += alpha p (from the second iteration on), p = r + beta p (:1121-1127,
+    // :1147-1150)
     double loc = 0.0;
 #pragma unroll
-    for (int q = 0; q < kPcgUnits; q++) {
+    for (int q = 0; q < N; q++) {
         const int64_t i = i0 + q * kPcgThreads;
         if (i >= nu) break;
-        const V v = pcg_axpy(beta, ld_unit(p + i), ld_unit(r + i));
+        if (LX && nx > 1) st_unit(x + i, PcgOp<T>::axpy(alpha, pv[q], xv[q]));
+        if (n.done) continue;
+        const V v = PcgOp<T>::axpy(beta, pv[q], rv[q]);
         st_unit(p + i, v);
-        if (std::is_same<T, float2>::value) loc += unit_norm2(v);
+        if (PcgOp<T>::kShifted) loc += PcgOp<T>::norm2(v);
     }
-    if constexpr (std::is_same<T, float2>::value) {
+    if (n.done) return;
+    if constexpr (PcgOp<T>::kShifted) {
         __shared__ double sh[32];
         loc = block_sum_any(loc, sh);
         if (threadIdx.x == 0) part[2 * G.nblk + b] = loc;
@@ -317,6 +373,7 @@ inline int pcg_sms() {
 template <class T>
 struct PcgBatch {
     typedef typename real_of<T>::type Real;
+    static constexpr bool kPair = std::is_same<typename unit_of<T>::type, cpair>::value;
     PcgArgs<T> a;                     // layout; the pointers are set when it runs
     int imass = 1;
     int64_t units = 0;
@@ -327,13 +384,14 @@ struct PcgBatch {
         if (a.nsys == kPcgSys || (a.nsys > 0 && im != imass)) return false;
         PcgGeo<T> G;
         memset(&G, 0, sizeof(G));
-        G.pl = plane_plan(g, std::is_same<T, float2>::value, nsm, kPcgThreads);
+        G.pl = plane_plan(g, kPair, nsm, kPcgThreads);
         G.diag = diag;
         G.hpin = hpin;
         G.apbc = apbc;
         G.nblk = G.pl.nitem < (uint32_t)kPcgMaxBlocks ? (int)G.pl.nitem : kPcgMaxBlocks;
         const int64_t nu = 8 * (int64_t)G.pl.U * g.kvol;
-        const int64_t ne = (nu + kPcgThreads * kPcgUnits - 1) / (kPcgThreads * kPcgUnits);
+        const int per = kPcgThreads * pcg_units_thread<T>();
+        const int64_t ne = (nu + per - 1) / per;
         if (ne > (int64_t)1 << 30) return false;
         G.neblk = (int)ne;
         int id = 0;
@@ -353,7 +411,7 @@ struct PcgBatch {
         a.eblk0[s + 1] = a.eblk0[s] + G.neblk;
         units += (3 + extra) * nu;
         chis += 3 * g.kvol;
-        parts += 2 * G.nblk + G.neblk;
+        parts += 2 * G.nblk + G.neblk + 1;
         return true;
     }
     const PcgGeo<T>& geo(int s) const { return a.geo[a.gid[s]]; }

@@ -302,17 +302,58 @@ __device__ __forceinline__ void plane_kappa(cpair acc[4], const cpair cur[4], fl
     for (int d = 0; d < 4; d++) acc[d] = zaxpy(-0.5f, acc[d], zscal2(hd, cur[d]));
 }
 
+struct PlaneThread { int x, y, t; };   // the thread's place in its tile
+__device__ __forceinline__ PlaneThread plane_thread(const PlanePlan& pl) {
+    const int tid = threadIdx.x, r = tid / pl.nx, t = r / pl.ny;
+    return PlaneThread{tid - r * pl.nx, r - t * pl.ny, t};
+}
+// Where a work item puts the thread: flavour, run of units, site, and the byte
+// offsets in a plane of the site and its neighbours.  Threads without a site
+// (act false) stand at the tile's corner; with SKIP `none` says that no thread
+// of the warp has one.
+struct PlanePlace {
+    int f, u0, u1, t;
+    bool act, none;
+    uint32_t site, o_0, o_xp, o_xm, o_yp, o_ym, o_tp, o_tm;
+};
+template <bool SKIP, uint32_t W>
+__device__ __forceinline__ PlanePlace plane_place(const PlanePlan& pl, const PlaneThread& th,
+                                                  uint32_t item) {
+    PlanePlace p;
+    const int L = pl.L, Lt = pl.Lt, U = pl.U;
+    // item -> (run, flavour, tile); tile -> corner
+    const uint32_t rf = fdiv(item, pl.dtile), tile = item - rf * pl.ntile;
+    const int run = (int)(rf >> 1);
+    p.f = (int)(rf & 1);
+    const uint32_t tyt = fdiv(tile, pl.dtx), tix = tile - tyt * (uint32_t)pl.tx;
+    const uint32_t tit = fdiv(tyt, pl.dty), tiy = tyt - tit * (uint32_t)pl.ty;
+    p.u0 = run * U / pl.nrun;
+    p.u1 = (run + 1) * U / pl.nrun;
+    int x = (int)tix * pl.nx + th.x, y = (int)tiy * pl.ny + th.y, t = (int)tit * pl.nt + th.t;
+    p.act = th.t < pl.nt && x < L && y < L && t < Lt;
+    // whole warps only: behind a branch of single threads nothing is kept in
+    // uniform registers
+    p.none = SKIP && !__any_sync(0xffffffffu, p.act);
+    if (!p.act) { x = (int)tix * pl.nx; y = (int)tiy * pl.ny; t = (int)tit * pl.nt; }
+    p.t = t;
+    const uint32_t uL = (uint32_t)L, LL = uL * uL;
+    p.site = (uint32_t)x + uL * ((uint32_t)y + uL * (uint32_t)t);
+    const uint32_t o_0 = p.o_0 = p.site * W;
+    p.o_xp = x + 1 == L ? o_0 - (uL - 1) * W : o_0 + W;
+    p.o_xm = x == 0 ? o_0 + (uL - 1) * W : o_0 - W;
+    p.o_yp = y + 1 == L ? o_0 - uL * (uL - 1) * W : o_0 + uL * W;
+    p.o_ym = y == 0 ? o_0 + uL * (uL - 1) * W : o_0 - uL * W;
+    p.o_tp = t + 1 == Lt ? o_0 - LL * (uint32_t)(Lt - 1) * W : o_0 + LL * W;
+    p.o_tm = t == 0 ? o_0 + LL * (uint32_t)(Lt - 1) * W : o_0 - LL * W;
+    return p;
+}
+
 // One work item: the thread's site, flavour and run of units.  For every
 // unit of the run epi(acc, off) is called by every thread of the block with
 // the four Dirac components of M R or M^dagger R: component d belongs at unit
 // e + d*cst of an output vector, byte offset o0 (the thread's site) from
 // there; act tells whether the thread holds a site, u is the unit.  It
 // returns whether to go on (the same for the whole block).
-struct PlaneThread { int x, y, t; };   // the thread's place in its tile
-__device__ __forceinline__ PlaneThread plane_thread(const PlanePlan& pl) {
-    const int tid = threadIdx.x, r = tid / pl.nx, t = r / pl.ny;
-    return PlaneThread{tid - r * pl.nx, r - t * pl.ny, t};
-}
 // SKIP: warps without a site return at once (no block barrier in epi).
 // S_LATE: the units above and below are loaded behind the diagonal term, which
 // suits kernels that would spill otherwise (CG in FP64 207 -> 193 ms for 32
@@ -324,30 +365,13 @@ __device__ __forceinline__ void plane_item(const V* in, const PlanePlan& pl, con
                                            Epi& epi) {
     constexpr int SF = DAG ? -1 : 1;
     constexpr int UP = DAG ? 0 : 2, DN = DAG ? 2 : 0;
-    const int L = pl.L, Lt = pl.Lt, U = pl.U;
-    // item -> (run, flavour, tile); tile -> corner
-    const uint32_t rf = fdiv(item, pl.dtile), tile = item - rf * pl.ntile;
-    const int f = (int)(rf & 1), run = (int)(rf >> 1);
-    const uint32_t tyt = fdiv(tile, pl.dtx), tix = tile - tyt * (uint32_t)pl.tx;
-    const uint32_t tit = fdiv(tyt, pl.dty), tiy = tyt - tit * (uint32_t)pl.ty;
-    const int u0 = run * U / pl.nrun, u1 = (run + 1) * U / pl.nrun;
-    const int lx = th.x, ly = th.y, lt = th.t;
-    int x = (int)tix * pl.nx + lx, y = (int)tiy * pl.ny + ly, t = (int)tit * pl.nt + lt;
-    const bool act = lt < pl.nt && x < L && y < L && t < Lt;
-    // whole warps only: behind a branch of single threads nothing is kept in
-    // uniform registers
-    if (SKIP && !__any_sync(0xffffffffu, act)) return;
-    if (!act) { x = (int)tix * pl.nx; y = (int)tiy * pl.ny; t = (int)tit * pl.nt; }
-    const uint32_t uL = (uint32_t)L, kv = pl.kvol, LL = uL * uL;
-    const uint32_t site = (uint32_t)x + uL * ((uint32_t)y + uL * (uint32_t)t);
-    constexpr uint32_t W = sizeof(V);
-    const uint32_t o_0 = site * W;
-    const uint32_t o_xp = x + 1 == L ? o_0 - (uL - 1) * W : o_0 + W;
-    const uint32_t o_xm = x == 0 ? o_0 + (uL - 1) * W : o_0 - W;
-    const uint32_t o_yp = y + 1 == L ? o_0 - uL * (uL - 1) * W : o_0 + uL * W;
-    const uint32_t o_ym = y == 0 ? o_0 + uL * (uL - 1) * W : o_0 - uL * W;
-    const uint32_t o_tp = t + 1 == Lt ? o_0 - LL * (uint32_t)(Lt - 1) * W : o_0 + LL * W;
-    const uint32_t o_tm = t == 0 ? o_0 + LL * (uint32_t)(Lt - 1) * W : o_0 - LL * W;
+    const int U = pl.U, Lt = pl.Lt;
+    const PlanePlace w0 = plane_place<SKIP, sizeof(V)>(pl, th, item);
+    if (SKIP && w0.none) return;
+    const bool act = w0.act;
+    const int f = w0.f, u0 = w0.u0, u1 = w0.u1, t = w0.t;
+    const uint32_t kv = pl.kvol, site = w0.site, o_0 = w0.o_0, o_xp = w0.o_xp, o_xm = w0.o_xm,
+                   o_yp = w0.o_yp, o_ym = w0.o_ym, o_tp = w0.o_tp, o_tm = w0.o_tm;
     const int64_t cst = (int64_t)U * kv;             // component stride
     const int64_t e0 = 4 * f * cst + (int64_t)u0 * kv;
     const V *p0 = in + e0, *p1 = p0 + cst, *p2 = p1 + cst, *p3 = p2 + cst;
