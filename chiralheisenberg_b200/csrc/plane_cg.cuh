@@ -37,6 +37,7 @@
 #include <cstring>
 #include <vector>
 
+#include "chunk_graph.h"
 #include "planes.cuh"
 #include "row_stage.cuh"
 
@@ -115,10 +116,6 @@ __device__ __forceinline__ int pcg_find(const int* first, int nsys, int b) {
 static __global__ void k_pcg_tick(PcgRun* run, int chunk) {
     run->base = run->next;
     run->next += chunk;
-}
-__device__ __forceinline__ void pcg_wait() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 // What a kind of system brings: its stencil, and s*a + b of its updates.
@@ -214,7 +211,7 @@ __global__ void __maxnreg__(kPlaneRegs) k_pcg1(const __grid_constant__ PcgArgs<T
     const int b = (int)blockIdx.x - a.blk0[s];
     const PlaneThread th = plane_thread(G.pl);
     V* p = a.vec + a.vec0[s];
-    pcg_wait();
+    pdl_wait();
     if (a.slot[2 * s + (k & 1)].done) return;
     PcgEpi1<T> epi{p + 2 * pcg_units<T>(G.pl), 0.0};
     pcg_sweep<false, IMASS>(a, G, s, b, p, th, epi);
@@ -234,7 +231,7 @@ __global__ void __maxnreg__(kPlaneRegs) k_pcg2(const __grid_constant__ PcgArgs<T
     V* p = a.vec + a.vec0[s];
     double* part = a.part + a.part0[s];
     PcgEpi2<T> epi{p, p + pcg_units<T>(G.pl), a.dyn[s].x, (Real)1, a.dyn[s].sigma, true, 0.0};
-    pcg_wait();
+    pdl_wait();
     const PcgSlot c = a.slot[2 * s + (k & 1)];
     if (c.done) return;
     const double tot = sum_partials_any(part, G.nblk);
@@ -286,7 +283,7 @@ __global__ void __launch_bounds__(kPcgThreads) k_pcg3(const __grid_constant__ Pc
             if (LX) xv[q] = ld_unit(x + i);
         }
     };
-    pcg_wait();
+    pdl_wait();
     // hmc32: on their way while the sum is formed (12.2 -> 10.9 ms); the others'
     // batches have blocks enough to hide it, and are 5% slower so
     if (LX) load();
@@ -446,50 +443,6 @@ void pcg_launch_chunk(const PcgArgs<T>& a, int imass, int chunk, cudaStream_t st
     }
 }
 
-// A chunk of iterations as a CUDA graph.  Every launch of the loop is the
-// same (the iteration state is on the device), so one capture serves every
-// chunk of this and later batches of the same layout: the key is the kernels'
-// arguments.  At most kPcgGraphs are kept.
-constexpr size_t kPcgGraphs = 16;
-struct PcgGraphs {
-    struct G {
-        std::vector<unsigned char> key;
-        cudaGraphExec_t exec = nullptr;
-    };
-    std::vector<G> g;
-    void release() {
-        for (G& x : g)
-            if (x.exec) cudaGraphExecDestroy(x.exec);
-        g.clear();
-    }
-    ~PcgGraphs() { release(); }
-    template <class T>
-    cudaGraphExec_t get(const PcgArgs<T>& a, int imass, int chunk, cudaStream_t st) {
-        std::vector<unsigned char> key(sizeof(a) + sizeof(int));
-        memcpy(key.data(), &a, sizeof(a));
-        memcpy(key.data() + sizeof(a), &imass, sizeof(int));
-        for (const G& x : g)
-            if (x.key == key) return x.exec;
-        cudaGraph_t graph = nullptr;
-        cudaGraphExec_t exec = nullptr;
-        if (cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-            pcg_launch_chunk(a, imass, chunk, st);
-            if (cudaStreamEndCapture(st, &graph) == cudaSuccess && graph) {
-                if (cudaGraphInstantiate(&exec, graph, 0) != cudaSuccess) exec = nullptr;
-                cudaGraphDestroy(graph);
-            }
-        }
-        cudaGetLastError();
-        if (!exec) return nullptr;
-        if (g.size() >= kPcgGraphs) {
-            if (g[0].exec) cudaGraphExecDestroy(g[0].exec);
-            g.erase(g.begin());
-        }
-        g.push_back(G{key, exec});
-        return exec;
-    }
-};
-
 // Vectors and device state of a batch, kept between solves and grown when a
 // larger batch arrives.
 template <class T>
@@ -504,7 +457,7 @@ struct PcgWork {
     PcgSlot* slot = nullptr;
     PcgRun* run = nullptr;
     int *hflag_host = nullptr, *hflag_dev = nullptr;
-    PcgGraphs graphs;
+    ChunkGraphs graphs;
     void release() {
         graphs.release();
         cudaFree(vec); cudaFree(chif); cudaFree(part); cudaFree(dyn); cudaFree(slot); cudaFree(run);
@@ -562,7 +515,8 @@ struct PcgWork {
             return e;
         *hflag_host = 0;
         constexpr int kChunk = 16;
-        cudaGraphExec_t ge = graphs.get(b.a, b.imass, kChunk, st);
+        const cudaGraphExec_t ge =
+            graphs.get(b.a, b.imass, st, [&] { pcg_launch_chunk(b.a, b.imass, kChunk, st); });
         cudaEvent_t ev[2];
         cudaEventCreateWithFlags(&ev[0], cudaEventDisableTiming);
         cudaEventCreateWithFlags(&ev[1], cudaEventDisableTiming);

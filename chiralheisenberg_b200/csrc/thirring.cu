@@ -10,10 +10,10 @@
 // evaluation bit for bit.  derivs gives one thread to each link (site, mu)
 // and adds its 8*kthird terms in the reference's order into a REAL*4
 // register, also bit for bit.  The multi-shift solver and congrad run
-// their scalar recurrences on the device, in the last block of each
-// reduction, with the reference's implicit REAL*4 / REAL*8 types; the sums
-// are FP64 block partials added in block order, and the host polls a stop
-// flag once every 16 iterations instead of reading every scalar.
+// their scalar recurrences on the device with the reference's implicit
+// REAL*4 / REAL*8 types; the sums are FP64 block partials added in one order,
+// and the host polls a stop flag once a chunk of iterations instead of reading
+// every scalar.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -21,9 +21,12 @@
 #include <vector>
 
 #include "chdwf_thirring.h"
+#include "chunk_graph.h"
 #include "common.cuh"
 #include "internal.h"
+#include "planes.cuh"
 #include "rng.h"
+#include "row_stage.cuh"
 
 namespace chdwf {
 namespace {
@@ -160,7 +163,13 @@ __global__ void __launch_bounds__(kThreads) k_thr_dslash(double2* __restrict__ o
 
 // derivs (:820-878), one thread per link (i, mu): for Dirac d and s in the
 // reference's order, the Wilson term then the Dirac term, each rounded to
-// REAL*4 as it is added.
+// REAL*4 as it is added.  The sum is a serial chain; the operands of the next
+// kDerivS values of s are loaded while those before are added (12^3x12: 32 ->
+// 15 us).
+constexpr int kDerivS = 4;
+struct DerivBatch {
+    double2 ri[kDerivS], ru[kDerivS], xi[kDerivS], xu[kDerivS], yi[kDerivS], yu[kDerivS];
+};
 __global__ void __launch_bounds__(kThreads) k_thr_derivs(const double2* __restrict__ R,
                                                          const double2* __restrict__ X2, TGeom g,
                                                          double tz, int iflag,
@@ -177,22 +186,43 @@ __global__ void __launch_bounds__(kThreads) k_thr_derivs(const double2* __restri
     tnbr(g, x, y, t, mu, &up, &dn);
     const double2 tzi = make_double2(0.0, tz);
     float f = dS[j];
-    for (int d = 0; d < 4; d++) {
-        const int dg = c_tgi[mu][d];
+    const int per = (Ls + kDerivS - 1) / kDerivS, nb = 4 * per;      // batches
+    auto load = [&](DerivBatch& v, int b) {
+        const int bb = b < nb ? b : nb - 1, d = bb / per, s0 = (bb - d * per) * kDerivS;
+        const int64_t ei = Ls * (i + kvol * d), eu = Ls * (up + kvol * d);
+        const int64_t gi = Ls * (i + kvol * c_tgi[mu][d]), gu = Ls * (up + kvol * c_tgi[mu][d]);
+#pragma unroll
+        for (int q = 0; q < kDerivS; q++) {
+            const int s = s0 + q < Ls ? s0 + q : Ls - 1;
+            v.ri[q] = zconj(R[ei + s]);
+            v.ru[q] = zconj(R[eu + s]);
+            v.xi[q] = X2[ei + s];
+            v.xu[q] = X2[eu + s];
+            v.yi[q] = X2[gi + s];
+            v.yu[q] = X2[gu + s];
+        }
+    };
+    auto add = [&](const DerivBatch& v, int b) {
+        if (b >= nb) return;
+        const int d = b / per, ns = Ls - (b - d * per) * kDerivS;
         const double2 tg = zmul(tzi, c_tgv[mu][d]);
-        for (int s = 0; s < Ls; s++) {
-            const double2 ri = zconj(R[s + (int64_t)Ls * (i + kvol * d)]);
-            const double2 ru = zconj(R[s + (int64_t)Ls * (up + kvol * d)]);
-            const double2 a = zmul(ri, X2[s + (int64_t)Ls * (up + kvol * d)]);
-            const double2 b = zmul(ru, X2[s + (int64_t)Ls * (i + kvol * d)]);
-            const double2 w = zmul(tzi, zsub(a, b));
+#pragma unroll
+        for (int q = 0; q < kDerivS; q++) {
+            if (q >= ns) break;
+            const double2 w = zmul(tzi, zsub(zmul(v.ri[q], v.xu[q]), zmul(v.ru[q], v.xi[q])));
             f = __double2float_rn(__dsub_rn((double)f, __dmul_rn(0.5, w.x)));     // :843-850
-            const double2 a2 = zmul(ri, X2[s + (int64_t)Ls * (up + kvol * dg)]);
-            const double2 b2 = zmul(ru, X2[s + (int64_t)Ls * (i + kvol * dg)]);
-            const double2 w2 = zmul(tg, zadd(a2, b2));
+            const double2 w2 = zmul(tg, zadd(zmul(v.ri[q], v.yu[q]), zmul(v.ru[q], v.yi[q])));
             f = __double2float_rn(iflag == 0 ? __dsub_rn((double)f, w2.x)             // :851-868
                                              : __dadd_rn((double)f, w2.x));
         }
+    };
+    DerivBatch v0, v1;
+    load(v0, 0);
+    for (int b = 0; b < nb; b += 2) {
+        load(v1, b + 1);
+        add(v0, b);
+        load(v0, b + 2);
+        add(v1, b + 1);
     }
     dS[j] = f;
 }
@@ -212,20 +242,341 @@ struct PoleCoef {
     double rho[kThrMaxPoles], amu[kThrMaxPoles];
 };
 
-// The solver's scalar recurrences run on the device, in thread 0 of the
-// block that finishes a reduction last, with the reference's implicit types
-// and the same operation order as a sequential host evaluation (no fused
-// multiply-adds), so the iterates do not depend on where the scalars are
-// formed.  The host only polls the stop flag every few iterations.
+// One iteration is two kernels, one thread a point (s, site) with its four
+// Dirac components, so a neighbour and a link serve all four:
+//   k_thr_m    vt = M R, |vt|^2
+//   k_thr_md   q = R/beta, R' = M^dagger vt/beta - alphatild q - beta q', |R'|^2
+// with alphatild = q^dagger M^dagger M q = |vt|^2/beta^2, so that the vector
+// enters M before beta = |R| is known and neither sum needs a kernel of its
+// own: a block leaves its partial and k_thr_md's blocks add both sums' partials
+// themselves.  One block more forms the pole recurrences with the reference's
+// implicit types.  The q of a chunk of iterations are kept, and k_thr_poles
+// takes p_k and x_k through all of them at once, so the 2*ndiag vectors are read
+// and written once a chunk instead of once an iteration.
+// At 12^3x12 with 12 poles (162 blocks: launches and latency) k_thr_m takes 6 us
+// and k_thr_md 9, k_thr_poles 28 for 16 iterations; a solve with its 12 link
+// forces 2.3 ms, against 10.2 with seven kernels an iteration, two of which
+// ended in a serial sum over 592 partials, and p_k and x_k updated every time.
+constexpr int kThrBlock = 128;
+constexpr int kThrChunk = 16;                  // q kept, at most
 struct ThrQCtl {
-    ThrRun run;
+    ThrRun run[2];                             // by parity of the iteration
+    int base, next;                            // iterations before this chunk, before the next
     int niterc, ndiag;
-    float phimod, resid, alphatild, pad_;
-    double beta;                                   // REAL*8 beta of :684-704
+    float phimod, resid;
     double aden[kThrMaxPoles], d[kThrMaxPoles], rhom1[kThrMaxPoles];
-    double rho[kThrMaxPoles], amu[kThrMaxPoles];
-    unsigned count1, count2;
+    double rho[kThrChunk][kThrMaxPoles], amu[kThrChunk][kThrMaxPoles];
 };
+struct ThrQArgs {
+    TGeom g;
+    int nblk, chunk;                           // blocks, iterations a chunk (even)
+    double2 *rr, *vt, *ring;                   // R, M R, the chunk's q
+    const double2* u;
+    double diag;
+    double2 zk, zkd;
+    double* part;                              // |vt|^2, |R|^2 of even and odd iterations
+    double2 *p, *x1;
+    ThrQCtl* c;
+    int* hflag;
+};
+
+__device__ __forceinline__ double2 zfma(double2 a, double2 b, double2 c) {   // a b + c
+    return make_double2(__fma_rn(a.x, b.x, __fma_rn(-a.y, b.y, c.x)),
+                        __fma_rn(a.x, b.y, __fma_rn(a.y, b.x, c.y)));
+}
+
+// The four components of M R or M^dagger R at (s, site i): thr_element's terms,
+// the two hops of a direction together.
+template <bool DAG, int IMASS>
+__device__ __forceinline__ void thr_point(double2 phi[4], const double2* R,
+                                          const double2* __restrict__ u, const TGeom& g, int s,
+                                          int i, double diag, double2 zk) {
+    const int L = g.L, Ls = g.Ls;
+    const int64_t kvol = g.kvol, cs = (int64_t)Ls * kvol;
+    const double2* r0 = R + s + (int64_t)Ls * i;
+    int x, y, t;
+    tsite_xyt(L, i, &x, &y, &t);
+#pragma unroll
+    for (int d = 0; d < 4; d++) phi[d] = zscal(diag, r0[cs * d]);
+#pragma unroll
+    for (int mu = 0; mu < 3; mu++) {
+        int64_t up, dn;
+        tnbr(g, x, y, t, mu, &up, &dn);
+        const double2 uu = __ldg(u + i + kvol * mu), ud = zconj(__ldg(u + dn + kvol * mu));
+        const double2 *ru = R + s + Ls * up, *rd = R + s + Ls * dn;
+        double2 a[4], b[4];
+#pragma unroll
+        for (int d = 0; d < 4; d++) {
+            a[d] = ru[cs * d];
+            b[d] = rd[cs * d];
+        }
+#pragma unroll
+        for (int d = 0; d < 4; d++) {
+            const double2 z = make_double2(0.0, 0.0);
+            a[d] = zfma(uu, a[d], z);
+            b[d] = zfma(ud, b[d], z);
+        }
+        // gamval(mu, d) is +-1/2 (mu 1) or +-i/2 (mu 0, 2), gamin(mu, d): d' = 3-d, 3-d, d^2
+        constexpr double sg[3][4] = {{-.5, -.5, .5, .5}, {-.5, .5, .5, -.5}, {-.5, .5, .5, -.5}};
+#pragma unroll
+        for (int d = 0; d < 4; d++) {
+            const int dg = mu == 2 ? d ^ 2 : 3 - d;
+            const double h = DAG ? -sg[mu][d] : sg[mu][d];
+            const double2 w = zadd(a[d], b[d]), v = zsub(a[dg], b[dg]);
+            phi[d].x = __fma_rn(-0.5, w.x, phi[d].x);
+            phi[d].y = __fma_rn(-0.5, w.y, phi[d].y);
+            phi[d].x = mu == 1 ? __fma_rn(h, v.x, phi[d].x) : __fma_rn(-h, v.y, phi[d].x);
+            phi[d].y = mu == 1 ? __fma_rn(h, v.y, phi[d].y) : __fma_rn(h, v.x, phi[d].y);
+        }
+    }
+    constexpr int UP = DAG ? 0 : 2, DN = DAG ? 2 : 0;   // pair that takes s+1, s-1
+#pragma unroll
+    for (int d = 0; d < 2; d++) {
+        if (s < Ls - 1) phi[UP + d] = zsub(phi[UP + d], r0[cs * (UP + d) + 1]);
+        if (s > 0) phi[DN + d] = zsub(phi[DN + d], r0[cs * (DN + d) - 1]);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const bool grpA = k < 2;
+        if (grpA ? s != Ls - 1 : s != 0) continue;
+        const int d = grpA ? UP + k : DN + k - 2;
+        if (IMASS == 5) phi[d] = zsub(phi[d], zmul(zk, r0[cs * (d ^ 2)]));
+        else {
+            const double2 tt = zmul(zk, r0[cs * d + (grpA ? 1 - Ls : Ls - 1)]);
+            phi[d] = IMASS == 3 && grpA == !DAG ? zsub(phi[d], tt) : zadd(phi[d], tt);
+        }
+    }
+}
+__device__ __forceinline__ double znorm2(double2 v) { return v.x * v.x + v.y * v.y; }
+
+// Points of the block's threads: (s, site) = j, s fastest.
+template <class F>
+__device__ __forceinline__ void thr_points(const TGeom& g, F&& f) {
+    const int64_t n = (int64_t)g.kvol * g.Ls, step = (int64_t)gridDim.x * kThrBlock;
+    for (int64_t j = (int64_t)blockIdx.x * kThrBlock + threadIdx.x; j < n; j += step) {
+        int64_t i;
+        if (n <= (int64_t)0xffffffffLL) i = (uint32_t)j / (uint32_t)g.Ls;
+        else i = j / g.Ls;
+        f(j, (int)(j - i * g.Ls), (int)i);
+    }
+}
+
+__global__ void k_thr_tick(ThrQCtl* c, int chunk) {
+    c->base = c->next;
+    c->next += chunk;
+}
+
+// R = Phi, partials of |R|^2
+__global__ void __launch_bounds__(kThrBlock) k_thr_start(ThrQArgs a,
+                                                         const double2* __restrict__ Phi) {
+    __shared__ double sh[32];
+    double loc = 0.0;
+    for (int64_t j = (int64_t)blockIdx.x * kThrBlock + threadIdx.x; j < a.g.kferm;
+         j += (int64_t)gridDim.x * kThrBlock) {
+        const double2 v = Phi[j];
+        a.rr[j] = v;
+        loc += znorm2(v);
+    }
+    loc = block_sum_any(loc, sh);
+    if (threadIdx.x == 0) a.part[a.nblk + blockIdx.x] = loc;
+}
+
+template <int IMASS>
+__global__ void __launch_bounds__(kThrBlock, 4) k_thr_m(ThrQArgs a, int k) {
+    __shared__ double sh[32];
+    pdl_wait();
+    if (a.c->run[k & 1].done) return;
+    double loc = 0.0;
+    thr_points(a.g, [&](int64_t j, int s, int i) {
+        double2 phi[4];
+        thr_point<false, IMASS>(phi, a.rr, a.u, a.g, s, i, a.diag, a.zk);
+#pragma unroll
+        for (int d = 0; d < 4; d++) {
+            a.vt[j + (int64_t)a.g.Ls * a.g.kvol * d] = phi[d];
+            loc += znorm2(phi[d]);
+        }
+    });
+    loc = block_sum_any(loc, sh);
+    if (threadIdx.x == 0) a.part[blockIdx.x] = loc;
+}
+
+// The pole recurrences of iteration it (:712-747) and the stopping test
+// (:750-757), by the threads of a block of their own.
+__device__ __forceinline__ void thr_scalars(const ThrQArgs& a, int k, int it, double beta,
+                                            float alphat) {
+    __shared__ float rm[kThrMaxPoles];
+    ThrQCtl* c = a.c;
+    const int nd = c->ndiag, p = threadIdx.x;
+    const float beta0 = (float)beta;
+    const float phimod = it == 1 ? beta0 : c->phimod;
+    if (p < nd) {
+        const double alpha = __dadd_rn((double)alphat, c->aden[p]);
+        double rho, amu = 0.0;
+        if (it == 1) {
+            c->d[p] = alpha;
+            rho = __ddiv_rn((double)beta0, alpha);
+        } else {
+            const double dm1 = c->d[p];
+            amu = __ddiv_rn((double)beta0, dm1);
+            const double dk = __dsub_rn(alpha, __dmul_rn((double)beta0, amu));
+            rho = -__ddiv_rn(__dmul_rn(__dmul_rn(amu, dm1), c->rhom1[p]), dk);
+            c->d[p] = dk;
+            rm[p] = (float)fabs(__dmul_rn((double)phimod, rho));
+        }
+        c->rho[k][p] = rho;
+        c->amu[k][p] = amu;
+        c->rhom1[p] = rho;
+    }
+    __syncthreads();
+    if (p != 0) return;
+    if (it == 1) c->phimod = phimod;
+    float rhomax = rm[0];
+    for (int q = 1; q < nd; q++)
+        if (rm[q] > rhomax) rhomax = rm[q];
+    ThrRun r{0, 0};
+    const float arelax = 2.0f;
+    if (it > 1 && rhomax < __fmul_rn(arelax, c->resid)) r = ThrRun{1, it};
+    else if (it >= c->niterc) r = ThrRun{2, it};
+    c->run[(k + 1) & 1] = r;
+    if (r.done && a.hflag) {
+        *(volatile int*)a.hflag = r.done;
+        __threadfence_system();
+    }
+}
+
+// Sums of two runs of n <= kRedBlocks partials, the same in every block.
+struct ThrSum2 {
+    static constexpr int N = (kRedBlocks + kThrBlock - 1) / kThrBlock;
+    double a[N], b[N];
+    __device__ __forceinline__ void load(const double* pa, const double* pb, int n) {
+#pragma unroll
+        for (int q = 0; q < N; q++) {
+            const int i = threadIdx.x + q * kThrBlock;
+            a[q] = i < n ? __ldcg(pa + i) : 0.0;
+            b[q] = i < n ? __ldcg(pb + i) : 0.0;
+        }
+    }
+    __device__ __forceinline__ void sum(double* ta, double* tb) {
+        __shared__ double sa[kThrBlock / 32], sb[kThrBlock / 32];
+        double x = 0.0, y = 0.0;
+#pragma unroll
+        for (int q = 0; q < N; q++) {
+            x += a[q];
+            y += b[q];
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            x += __shfl_xor_sync(0xffffffffu, x, o);
+            y += __shfl_xor_sync(0xffffffffu, y, o);
+        }
+        if ((threadIdx.x & 31) == 0) {
+            sa[threadIdx.x >> 5] = x;
+            sb[threadIdx.x >> 5] = y;
+        }
+        __syncthreads();
+        x = y = 0.0;
+#pragma unroll
+        for (int w = 0; w < kThrBlock / 32; w++) {
+            x += sa[w];
+            y += sb[w];
+        }
+        *ta = x;
+        *tb = y;
+    }
+};
+
+template <int IMASS>
+__global__ void __launch_bounds__(kThrBlock, 4) k_thr_md(ThrQArgs a, int k) {
+    __shared__ double sh[32];
+    pdl_wait();
+    const ThrRun run = a.c->run[k & 1];
+    const bool scalars = blockIdx.x == (unsigned)a.nblk;      // the block behind the points'
+    if (run.done) {
+        if (scalars && threadIdx.x == 0) a.c->run[(k + 1) & 1] = run;
+        return;
+    }
+    const int it = a.c->base + k + 1;
+    ThrSum2 sums;
+    sums.load(a.part, a.part + (size_t)a.nblk * (1 + (k & 1)), a.nblk);
+    // the first point's hops while the partials are on their way
+    const int64_t n = (int64_t)a.g.kvol * a.g.Ls, cs = n;
+    int64_t j = (int64_t)blockIdx.x * kThrBlock + threadIdx.x;
+    double2 phi[4];
+    auto point = [&] {
+        const int64_t i = n <= (int64_t)0xffffffffLL ? (uint32_t)j / (uint32_t)a.g.Ls : j / a.g.Ls;
+        thr_point<true, IMASS>(phi, a.vt, a.u, a.g, (int)(j - i * a.g.Ls), (int)i, a.diag, a.zkd);
+    };
+    bool act = !scalars && j < n;
+    if (act) point();
+    double v2, b2;
+    sums.sum(&v2, &b2);
+    const double beta = __dsqrt_rn(b2), inv = 1.0 / beta;               // :684-694
+    const float alphat = (float)(v2 / b2);
+    if (scalars) {
+        thr_scalars(a, k, it, beta, alphat);
+        return;
+    }
+    const double2* qm1 = a.ring + a.g.kferm * (int64_t)(k > 0 ? k - 1 : a.chunk - 1);
+    double2* q = a.ring + a.g.kferm * (int64_t)k;
+    double loc = 0.0;
+    while (act) {
+#pragma unroll
+        for (int d = 0; d < 4; d++) {
+            const int64_t e = j + cs * d;
+            const double2 qj = zscal(inv, a.rr[e]);
+            double2 r = zsub(zscal(inv, phi[d]), zscal((double)alphat, qj));
+            if (it > 1) r = zsub(r, zscal(beta, qm1[e]));
+            q[e] = qj;
+            a.rr[e] = r;
+            loc += znorm2(r);
+        }
+        j += (int64_t)a.nblk * kThrBlock;
+        act = j < n;
+        if (act) point();
+    }
+    loc = block_sum_any(loc, sh);
+    if (threadIdx.x == 0) a.part[(size_t)a.nblk * (2 - (k & 1)) + blockIdx.x] = loc;
+}
+
+// p_k = q - amu_k p_k, x_k += rho_k p_k for the chunk's iterations (first
+// iteration of a solve: p_k = q, x_k = rho_k q; :712-747, pm1 equals p), four
+// poles a thread: q is read ndiag/4 times.
+constexpr int kThrPoles = 4;
+__global__ void __launch_bounds__(kThreads) k_thr_poles(ThrQArgs a) {
+    const ThrQCtl* c = a.c;
+    const ThrRun run = c->run[0];              // a chunk is an even number of iterations
+    const int base = c->base;
+    const int nit = run.done ? run.iters - base : a.chunk;
+    const int64_t n = a.g.kferm, j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (nit <= 0 || j >= n) return;
+    const int k0 = (int)blockIdx.y * kThrPoles, nk = min(kThrPoles, c->ndiag - k0);
+    double2 p[kThrPoles], x[kThrPoles];
+#pragma unroll
+    for (int k = 0; k < kThrPoles; k++) {
+        p[k] = x[k] = make_double2(0.0, 0.0);
+        if (k < nk && base > 0) {
+            p[k] = a.p[j + n * (k0 + k)];
+            x[k] = a.x1[j + n * (k0 + k)];
+        }
+    }
+#pragma unroll 4
+    for (int it = 0; it < nit; it++) {
+        const double2 q = a.ring[j + n * it];
+#pragma unroll
+        for (int k = 0; k < kThrPoles; k++) {
+            if (k >= nk) continue;
+            const double rho = c->rho[it][k0 + k], amu = c->amu[it][k0 + k];
+            p[k] = base + it == 0 ? q : zsub(q, zscal(amu, p[k]));
+            x[k] = zadd(x[k], zscal(rho, p[k]));
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < kThrPoles; k++) {
+        if (k >= nk) continue;
+        a.p[j + n * (k0 + k)] = p[k];
+        a.x1[j + n * (k0 + k)] = x[k];
+    }
+}
 
 // Grid sum of one double per thread with the block partials added in block
 // order by one thread (the order of a host loop over the partials).  The
@@ -257,15 +608,6 @@ __device__ __forceinline__ bool last_block_seq(double v, double* part, unsigned*
     return true;
 }
 
-// q = R/beta (:684-686)
-__global__ void k_thr_q(double2* __restrict__ q, const double2* __restrict__ R,
-                        const ThrQCtl* __restrict__ c, int it, int64_t n) {
-    if (thr_skip(&c->run, it)) return;
-    const double beta = c->beta;
-    const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (j < n) q[j] = make_double2(__ddiv_rn(R[j].x, beta), __ddiv_rn(R[j].y, beta));
-}
-
 // block partials of sum Re(conjg(a)*b); the host adds them in block order
 __global__ void __launch_bounds__(kThreads) k_thr_dot(const double2* __restrict__ a,
                                                       const double2* __restrict__ b, int64_t n,
@@ -277,106 +619,6 @@ __global__ void __launch_bounds__(kThreads) k_thr_dot(const double2* __restrict_
         loc += zmul(zconj(a[j]), b[j]).x;
     loc = block_sum<kThreads>(loc, sh);
     if (threadIdx.x == 0) part[blockIdx.x] = loc;
-}
-
-// alphatild = sum Re(conjg(q)*x3), rounded once to REAL*4 (:688-694)
-__global__ void __launch_bounds__(kThreads) k_thr_alpha(const double2* __restrict__ q,
-                                                        const double2* __restrict__ x3, int64_t n,
-                                                        double* __restrict__ part,
-                                                        ThrQCtl* __restrict__ c, int it) {
-    if (thr_skip(&c->run, it)) return;
-    double loc = 0.0;
-    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < n;
-         j += (int64_t)gridDim.x * blockDim.x)
-        loc += zmul(zconj(q[j]), x3[j]).x;
-    double tot;
-    if (!last_block_seq<kThreads, kRedBlocks>(loc, part, &c->count1, &tot)) return;
-    if (threadIdx.x == 0) c->alphatild = (float)tot;
-}
-
-// R = x3 - alphatild q - beta qm1 ; qm1 = q ; beta = |R| (:696-704), then
-// the pole recurrences and the stopping test (:712-757) in the last block
-__global__ void __launch_bounds__(kThreads) k_thr_lanczos(double2* __restrict__ R,
-                                                          double2* __restrict__ qm1,
-                                                          const double2* __restrict__ q,
-                                                          const double2* __restrict__ x3, int64_t n,
-                                                          double* __restrict__ part,
-                                                          ThrQCtl* __restrict__ c, int it) {
-    if (thr_skip(&c->run, it)) return;
-    const double alphat = (double)c->alphatild, beta = c->beta;
-    double loc = 0.0;
-    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < n;
-         j += (int64_t)gridDim.x * blockDim.x) {
-        const double2 qj = q[j];
-        const double2 r = zsub(zsub(x3[j], zscal(alphat, qj)), zscal(beta, qm1[j]));
-        R[j] = r;
-        qm1[j] = qj;
-        loc += zmul(zconj(r), r).x;
-    }
-    double b2;
-    if (!last_block_seq<kThreads, kRedBlocks>(loc, part, &c->count2, &b2)) return;
-    if (threadIdx.x != 0) return;
-    const float beta0 = (float)beta;
-    c->beta = __dsqrt_rn(b2);
-    const int nd = c->ndiag;
-    float rhomax = 0.0f;
-    for (int k = 0; k < nd; k++) {
-        const double alpha = __dadd_rn((double)c->alphatild, c->aden[k]);
-        if (it == 1) {                                                     // :712-724
-            c->d[k] = alpha;
-            c->rho[k] = __ddiv_rn((double)beta0, alpha);
-            c->rhom1[k] = c->rho[k];
-        } else {                                                           // :725-747
-            const double amu = __ddiv_rn((double)beta0, c->d[k]);
-            const double dm1 = c->d[k];
-            const double dk = __dsub_rn(alpha, __dmul_rn((double)beta0, amu));
-            const double rho = -__ddiv_rn(__dmul_rn(__dmul_rn(amu, dm1), c->rhom1[k]), dk);
-            c->amu[k] = amu;
-            c->d[k] = dk;
-            c->rho[k] = rho;
-            const double rm = fabs(__dmul_rn((double)c->phimod, rho));
-            if (k == 0) rhomax = (float)rm;
-            else if (rm > (double)rhomax) rhomax = (float)rm;
-            c->rhom1[k] = rho;
-        }
-    }
-    const float arelax = 2.0f;                                             // :750-757
-    if (it > 1 && rhomax < __fmul_rn(arelax, c->resid)) {
-        c->run.iters = it;
-        c->run.done = 1;
-    } else if (it >= c->niterc) {
-        c->run.iters = it;
-        c->run.done = 2;
-    }
-}
-
-// all poles at once: first iteration p_k = q, x_k = rho_k q; later
-// p_k = q - amu_k p_k, x_k += rho_k p_k (:712-747; pm1 equals p).  Runs in
-// the iteration that stopped the solve too.
-__global__ void k_thr_poles(double2* __restrict__ p, double2* __restrict__ x1,
-                            const double2* __restrict__ q, const ThrQCtl* __restrict__ c,
-                            int it, int64_t n, int* hflag) {
-    if (thr_skip(&c->run, it)) return;
-    const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (j == 0 && c->run.done && hflag) {
-        *(volatile int*)hflag = c->run.done;
-        __threadfence_system();
-    }
-    if (j >= n) return;
-    const double2 qj = q[j];
-    const int nd = c->ndiag;
-    for (int k = 0; k < nd; k++) {
-        const int64_t e = j + n * k;
-        const double rho = c->rho[k];
-        if (it == 1) {
-            p[e] = qj;
-            x1[e] = zscal(rho, qj);
-        } else {
-            const double2 pk = zsub(qj, zscal(c->amu[k], p[e]));
-            p[e] = pk;
-            x1[e] = zadd(x1[e], zscal(rho, pk));
-        }
-    }
 }
 
 // x = anum0 Phi, then x += anum_k x_k in pole order (:666, :766-772)
@@ -549,7 +791,10 @@ struct chdwf_thr {
     float *theta = nullptr, *thetat = nullptr, *pp = nullptr, *dS = nullptr, *gauss = nullptr;
     double2 *ut = nullptr, *uio = nullptr;
     double2 *Phi = nullptr, *X1 = nullptr, *R = nullptr, *X2 = nullptr, *Phi0 = nullptr;
-    double2 *q = nullptr, *qm1 = nullptr, *vt = nullptr, *x3 = nullptr, *rr = nullptr;
+    double2 *vt = nullptr, *rr = nullptr;
+    double2* ring = nullptr;              // chunk vectors: the q of a chunk of iterations
+    int chunk = 0;
+    chdwf::ChunkGraphs graphs;
     double2 *p = nullptr, *x1 = nullptr;
     double* part = nullptr;
     std::vector<double> hpart;
@@ -577,11 +822,37 @@ thread_local std::string g_thr_create_err;
 template <class T>
 cudaError_t talloc(T** p, size_t n) { return cudaMalloc((void**)p, sizeof(T) * n); }
 
+double2 thr_mass(float am, int imass, bool dag) {
+    return imass == 1 ? make_double2((double)am, 0.0)
+                      : make_double2(0.0, dag ? (double)am : (double)(-am));
+}
+
+// The launches of a chunk of qmrherm's iterations.
+template <int IMASS>
+void thr_launch_chunk(const chdwf::ThrQArgs& a, int ndiag, cudaStream_t st) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.blockDim = dim3(chdwf::kThrBlock);
+    c.stream = st;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    chdwf::k_thr_tick<<<1, 1, 0, st>>>(a.c, a.chunk);
+    for (int k = 0; k < a.chunk; k++) {
+        c.gridDim = dim3((unsigned)a.nblk);
+        cudaLaunchKernelEx(&c, chdwf::k_thr_m<IMASS>, a, k);
+        c.gridDim = dim3((unsigned)a.nblk + 1);
+        cudaLaunchKernelEx(&c, chdwf::k_thr_md<IMASS>, a, k);
+    }
+    const dim3 grid(chdwf::tblk(a.g.kferm), (unsigned)((ndiag + chdwf::kThrPoles - 1) / chdwf::kThrPoles));
+    chdwf::k_thr_poles<<<grid, chdwf::kThreads, 0, st>>>(a);
+}
+
 void thr_dslash(chdwf_thr* h, bool dag, float am, int imass, double2* out, const double2* in,
                 const double2* u, const chdwf::ThrRun* run = nullptr, int it = 0) {
     const unsigned nb = chdwf::tblk(h->g.kferm);
-    double2 zk = imass == 1 ? make_double2((double)am, 0.0)
-                            : make_double2(0.0, dag ? (double)am : (double)(-am));
+    const double2 zk = thr_mass(am, imass, dag);
     const double dg = h->diag();
 #define THR_LAUNCH(D, I) chdwf::k_thr_dslash<D, I><<<nb, chdwf::kThreads, 0, h->st>>>(out, in, u, h->g, dg, zk, run, it)
     if (dag) {
@@ -595,7 +866,9 @@ void thr_dslash(chdwf_thr* h, bool dag, float am, int imass, double2* out, const
 
 void thr_derivs(chdwf_thr* h, const double2* R, const double2* X2, double anum, int iflag) {
     const double tz = (double)(float)(2.0 * anum);                         // tzi, :839
-    chdwf::k_thr_derivs<<<chdwf::tblk(3 * (int64_t)h->g.kvol), chdwf::kThreads, 0, h->st>>>(
+    // small blocks: few links, each a long chain
+    const unsigned nb = (unsigned)((3 * (int64_t)h->g.kvol + 31) / 32);
+    chdwf::k_thr_derivs<<<nb, 32, 0, h->st>>>(
         R, X2, h->g, tz, iflag, h->dS);
     chdwf::count_launches(1);
 }
@@ -611,13 +884,13 @@ cudaError_t thr_sum(chdwf_thr* h, double* out) {
     return e;
 }
 
-// Launches iterations 1, 2, ... of a solve in chunks of 16 until the
-// device raises the stop flag or cap iterations are queued.  The flag is
-// read one chunk behind, so up to two chunks are in flight; the kernels of
-// iterations past the stopping one return at once.
+// Launches a solve in chunks of iterations until the device raises the stop
+// flag or cap iterations are queued: launch(first) queues the chunk that
+// begins with iteration first.  The flag is read one chunk behind, so up to two
+// chunks are in flight; the kernels of iterations past the stopping one return
+// at once.
 template <class F>
-cudaError_t thr_run_chunks(chdwf_thr* h, int64_t cap, F&& launch_iteration) {
-    const int chunk = 16;
+cudaError_t thr_run_chunks(chdwf_thr* h, int64_t cap, int chunk, F&& launch) {
     cudaEvent_t ev[2];
     cudaError_t e = cudaEventCreateWithFlags(&ev[0], cudaEventDisableTiming);
     if (e) return e;
@@ -625,10 +898,9 @@ cudaError_t thr_run_chunks(chdwf_thr* h, int64_t cap, F&& launch_iteration) {
         cudaEventDestroy(ev[0]);
         return e;
     }
-    int64_t launched = 0;
     int nchunk = 0;
-    while (launched < cap) {
-        for (int c = 0; c < chunk && launched < cap; c++) launch_iteration((int)++launched);
+    for (int64_t first = 1; first <= cap; first += chunk) {
+        launch((int)first);
         if ((e = cudaGetLastError())) break;
         cudaEventRecord(ev[nchunk & 1], h->st);
         if (nchunk >= 1) {
@@ -652,16 +924,8 @@ int thr_qmrherm(chdwf_thr* h, const double2* Phi, float res, int* itercg, float 
     const int niterc = 7500;                                             // :635
     const float resid = std::sqrt((float)n * res * res);                // :660
     cudaError_t e;
-    cudaMemcpyAsync(h->rr, Phi, sizeof(double2) * n, cudaMemcpyDeviceToDevice, h->st);   // :662-667
-    cudaMemsetAsync(h->qm1, 0, sizeof(double2) * n, h->st);
-    chdwf::k_thr_dot<<<chdwf::kRedBlocks, chdwf::kThreads, 0, h->st>>>(h->rr, h->rr, n, h->part);
-    chdwf::count_launches(1);
-    double b0;
-    if ((e = thr_sum(h, &b0))) return h->fail(e, "thr_qmrherm");
     chdwf::ThrQCtl hc;
     memset(&hc, 0, sizeof(hc));
-    hc.beta = std::sqrt(b0);
-    hc.phimod = (float)hc.beta;
     hc.resid = resid;
     hc.niterc = niterc;
     hc.ndiag = ndiag;
@@ -669,23 +933,38 @@ int thr_qmrherm(chdwf_thr* h, const double2* Phi, float res, int* itercg, float 
     if ((e = cudaMemcpyAsync(h->qctl, &hc, sizeof(hc), cudaMemcpyHostToDevice, h->st)))
         return h->fail(e, "thr_qmrherm");
     *h->hflag_host = 0;
-    chdwf::ThrQCtl* c = h->qctl;
-    const chdwf::ThrRun* run = &c->run;
-    e = thr_run_chunks(h, niterc, [&](int it) {
-        chdwf::k_thr_q<<<nb, chdwf::kThreads, 0, h->st>>>(h->q, h->rr, c, it, n);
-        thr_dslash(h, false, am, imass, h->vt, h->q, u, run, it);
-        thr_dslash(h, true, am, imass, h->x3, h->vt, u, run, it);
-        chdwf::k_thr_alpha<<<chdwf::kRedBlocks, chdwf::kThreads, 0, h->st>>>(h->q, h->x3, n,
-                                                                            h->part, c, it);
-        chdwf::k_thr_lanczos<<<chdwf::kRedBlocks, chdwf::kThreads, 0, h->st>>>(
-            h->rr, h->qm1, h->q, h->x3, n, h->part, c, it);
-        chdwf::k_thr_poles<<<nb, chdwf::kThreads, 0, h->st>>>(h->p, h->x1, h->q, c, it, n,
-                                                               h->hflag_dev);
-        chdwf::count_launches(4);
+    chdwf::ThrQArgs a;
+    memset(&a, 0, sizeof(a));
+    a.g = h->g;
+    const int64_t pts = (int64_t)h->g.kvol * h->g.Ls;
+    a.nblk = (int)std::min<int64_t>((pts + chdwf::kThrBlock - 1) / chdwf::kThrBlock,
+                                    chdwf::kRedBlocks);
+    a.chunk = h->chunk;
+    a.rr = h->rr; a.vt = h->vt; a.ring = h->ring;
+    a.u = u;
+    a.diag = h->diag();
+    a.zk = thr_mass(am, imass, false);
+    a.zkd = thr_mass(am, imass, true);
+    a.part = h->part;
+    a.p = h->p; a.x1 = h->x1;
+    a.c = h->qctl;
+    a.hflag = h->hflag_dev;
+    chdwf::k_thr_start<<<a.nblk, chdwf::kThrBlock, 0, h->st>>>(a, Phi);   // :662-667
+    chdwf::count_launches(1);
+    auto chunk = [&] {
+        if (imass == 1) thr_launch_chunk<1>(a, ndiag, h->st);
+        else if (imass == 3) thr_launch_chunk<3>(a, ndiag, h->st);
+        else thr_launch_chunk<5>(a, ndiag, h->st);
+    };
+    const cudaGraphExec_t ge = h->graphs.get(a, imass + 8 * ndiag, h->st, chunk);
+    e = thr_run_chunks(h, niterc, a.chunk, [&](int) {
+        if (ge) cudaGraphLaunch(ge, h->st);
+        else chunk();
+        chdwf::count_launches(2 * a.chunk + 2);
     });
     if (e) return h->fail(e, "thr_qmrherm");
     chdwf::ThrRun hr;
-    if ((e = cudaMemcpyAsync(&hr, run, sizeof(hr), cudaMemcpyDeviceToHost, h->st)) ||
+    if ((e = cudaMemcpyAsync(&hr, &h->qctl->run[0], sizeof(hr), cudaMemcpyDeviceToHost, h->st)) ||
         (e = cudaStreamSynchronize(h->st)))
         return h->fail(e, "thr_qmrherm");
     *itercg = hr.iters;
@@ -788,7 +1067,7 @@ int thr_congrad(chdwf_thr* h, const double2* Phi, float res, int* itercg, float 
     const unsigned nb = chdwf::tblk(n);
     const int64_t niterc = h->g.Ls * (int64_t)h->g.kvol;                 // :934
     const float resid = (float)n * res * res;                            // :947
-    double2 *p = h->q, *r = h->rr, *x1 = h->vt, *x2 = h->x3;
+    double2 *p = h->ring, *r = h->rr, *x1 = h->vt, *x2 = h->ring + n;
     cudaMemcpyAsync(p, x, sizeof(double2) * n, cudaMemcpyDeviceToDevice, h->st);   // :956-959
     cudaMemcpyAsync(r, Phi, sizeof(double2) * n, cudaMemcpyDeviceToDevice, h->st);
     chdwf::ThrCgCtl hc;
@@ -804,7 +1083,8 @@ int thr_congrad(chdwf_thr* h, const double2* Phi, float res, int* itercg, float 
     *h->hflag_host = 0;
     chdwf::ThrCgCtl* c = h->cgctl;
     const chdwf::ThrRun* run = &c->run;
-    e = thr_run_chunks(h, niterc, [&](int it) {
+    e = thr_run_chunks(h, niterc, 16, [&](int first) {
+      for (int it = first; it < first + 16 && it <= niterc; it++) {
         thr_dslash(h, false, am, imass, x1, p, u, run, it);               // :966
         if (it != 1) {                                                    // :970-983
             chdwf::k_thr_cg_alpha<<<chdwf::kRedBlocks, chdwf::kThreads, 0, h->st>>>(x1, n, h->part,
@@ -817,6 +1097,7 @@ int thr_congrad(chdwf_thr* h, const double2* Phi, float res, int* itercg, float 
                                                                           it, h->hflag_dev);
         chdwf::k_thr_xpay<<<nb, chdwf::kThreads, 0, h->st>>>(p, r, c, it, n);
         chdwf::count_launches(2);
+      }
     });
     if (e) return h->fail(e, "thr_congrad");
     chdwf::ThrRun hr;
@@ -963,12 +1244,20 @@ int chdwf_thr_create(chdwf_thr** out, int ksize, int ksizet, int kthird, float d
     if (!e) e = talloc(&h->gauss, 8 * (size_t)h->g.kvol * kthird);
     if (!e) e = talloc(&h->ut, n3);
     if (!e) e = talloc(&h->uio, n3);
-    for (double2** v : {&h->Phi, &h->X1, &h->R, &h->X2, &h->q, &h->qm1, &h->vt, &h->x3, &h->rr})
+    for (double2** v : {&h->Phi, &h->X1, &h->R, &h->X2, &h->vt, &h->rr})
         if (!e) e = talloc(v, n);
     if (!e) e = talloc(&h->Phi0, n * np);
     if (!e) e = talloc(&h->p, n * np);
     if (!e) e = talloc(&h->x1, n * np);
-    if (!e) e = talloc(&h->part, chdwf::kRedBlocks);
+    // a longer chunk is an option: where memory is short, a shorter one
+    for (h->chunk = chdwf::kThrChunk; !e && !h->ring; h->chunk /= 2) {
+        e = talloc(&h->ring, n * h->chunk);
+        if (!e) break;
+        if (h->chunk == 2) break;
+        cudaGetLastError();
+        e = cudaSuccess;
+    }
+    if (!e) e = talloc(&h->part, 3 * chdwf::kRedBlocks);
     if (!e) e = talloc(&h->qctl, 1);
     if (!e) e = talloc(&h->cgctl, 1);
     if (!e) e = cudaHostAlloc((void**)&h->hflag_host, sizeof(int), cudaHostAllocMapped);
@@ -992,9 +1281,10 @@ void chdwf_thr_destroy(chdwf_thr* h) {
     cudaSetDevice(h->device);
     if (h->st) cudaStreamSynchronize(h->st);
     for (float* v : {h->theta, h->thetat, h->pp, h->dS, h->gauss}) if (v) cudaFree(v);
-    for (double2* v : {h->ut, h->uio, h->Phi, h->X1, h->R, h->X2, h->Phi0, h->q, h->qm1, h->vt,
-                       h->x3, h->rr, h->p, h->x1})
+    for (double2* v : {h->ut, h->uio, h->Phi, h->X1, h->R, h->X2, h->Phi0, h->ring, h->vt,
+                       h->rr, h->p, h->x1})
         if (v) cudaFree(v);
+    h->graphs.release();
     if (h->part) cudaFree(h->part);
     if (h->qctl) cudaFree(h->qctl);
     if (h->cgctl) cudaFree(h->cgctl);
