@@ -202,7 +202,7 @@ static int dslash_host(Ctx* c, double* Phi, const double* R, const double* chi, 
     if ((e = c->upload_chi(chi))) return c->status_of(e, "dslash: chi upload");
     if ((e = cudaMemcpyAsync(c->spin[0], R, bytes, cudaMemcpyHostToDevice, c->stream)))
         return c->status_of(e, "dslash: R upload");
-    launch_dslash64(dag, imass, c->spin[1], c->spin[0], c->chif, c->g, c->am3, hpin, c->ibound,
+    launch_dslash64(dag, imass, c->spin[1], c->spin[0], {c->chid, c->chif}, c->g, c->am3, hpin, c->ibound,
                     c->stream);
     if ((e = cudaMemcpyAsync(Phi, c->spin[1], bytes, cudaMemcpyDeviceToHost, c->stream)))
         return c->status_of(e, "dslash: Phi download");
@@ -231,9 +231,8 @@ int chdwf_dslash_dev(chdwf_ctx* ctx, void* Phi, const void* R, const void* chi, 
     if (!c || !Phi || !R || !chi) return CHDWF_BAD_ARG;
     cudaSetDevice(c->device);
     cudaStream_t st = stream ? (cudaStream_t)stream : c->stream;
-    launch_round_chi((const double*)chi, c->chif, c->g.kvol, st);
-    launch_dslash64(dagger != 0, imass, (double2*)Phi, (const double2*)R, c->chif, c->g, c->am3,
-                    hpin, c->ibound, st);
+    launch_dslash64(dagger != 0, imass, (double2*)Phi, (const double2*)R,
+                    {(const double*)chi, c->chif}, c->g, c->am3, hpin, c->ibound, st);
     return c->status_of(cudaGetLastError(), "dslash_dev");
 }
 
@@ -243,9 +242,8 @@ int chdwf_dslash_dev_lp(chdwf_ctx* ctx, void* Phi, const void* R, const void* ch
     if (!c || !Phi || !R || !chi || (prec != 1 && prec != 2)) return CHDWF_BAD_ARG;
     cudaSetDevice(c->device);
     cudaStream_t st = stream ? (cudaStream_t)stream : c->stream;
-    launch_round_chi((const double*)chi, c->chif, c->g.kvol, st);
-    launch_dslash_lp(dagger != 0, imass, prec == 2, Phi, R, c->chif, c->g, c->am3, hpin, c->ibound,
-                     st);
+    launch_dslash_lp(dagger != 0, imass, prec == 2, Phi, R, {(const double*)chi, c->chif}, c->g,
+                     c->am3, hpin, c->ibound, st);
     return c->status_of(cudaGetLastError(), "dslash_dev_lp");
 }
 

@@ -5,6 +5,7 @@
 #include <cstdlib>
 #include <cstring>
 
+#include "chunk_graph.h"
 #include "dwf_stencil.cuh"
 #include "internal.h"
 #include "row_stage.cuh"
@@ -16,20 +17,68 @@ struct LdF64 {
     __device__ __forceinline__ double2 operator()(int64_t j) const { return __ldg(p + j); }
 };
 
-// Flavour-split: two threads per point (split_point / split_flavour); OCC
-// blocks a SM (the register budget).
+// The operator on the ABI's spinors takes chi as the callers have it, REAL*8,
+// and rounds it to REAL*4 where a wall reads it, and is launched with
+// programmatic serialisation: its blocks are scheduled while the kernel before
+// it drains.  At 8^3x8 a call takes 4.7 us (5.3 without the latter),
+// against 7.7 with a rounding kernel in front of it.
+
+// chi of a wall point on its way while the hops are formed: it comes from HBM
+// where the rounded copy used to be in L2.
+__device__ __forceinline__ void prefetch_chi(const double* chi, const Geom& g, const PointIdx& q,
+                                             int pt) {
+    if (q.s == 0 || q.s + pt == g.Ls) {
+#pragma unroll
+        for (int k = 0; k < 3; k++)
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(chi + (int64_t)k * g.kvol + q.site));
+    }
+}
+
+// A block covers kOpPoints consecutive units (of one, two or four points) of
+// both flavours, the first half of its threads flavour 0.  128 threads rather
+// than 256 at the same registers: 24^3x24 FP64 23.5 -> 22.7 us, 48^3x32 FP32
+// 120 -> 114 (a finer grain where the walls make warps uneven); 64 gain nothing
+// more.  Tiles of sites in place of consecutive points, which read the y and t
+// neighbours from L1, are slower: 24^3x24 FP64 26, 48^3x32 FP32 143-162.
+constexpr int kOpThreads = 128, kOpPoints = kOpThreads / 2;
+__device__ __forceinline__ int op_flavour() { return threadIdx.x >= kOpPoints; }
+template <int PT> __device__ __forceinline__ int64_t op_point() {
+    return PT * ((int64_t)blockIdx.x * kOpPoints + (threadIdx.x & (kOpPoints - 1)));
+}
+static unsigned op_blocks(int64_t npts, int pt) {
+    return (unsigned)((npts + pt * kOpPoints - 1) / (pt * kOpPoints));
+}
+
+// Flavour-split: two threads per point; OCC blocks a SM (the register budget).
 template <bool DAG, int IMASS, int OCC>
-__global__ void __launch_bounds__(kSplitThreads, OCC)
+__global__ void __launch_bounds__(kOpThreads, OCC)
     k_dslash64(double2* __restrict__ out, const double2* __restrict__ in,
-               const float* __restrict__ chif, Geom g, double diag, double hpin, int apbc) {
-    const int64_t p = split_point();
-    const int f = split_flavour();
+               const double* __restrict__ chi, Geom g, double diag, double hpin, int apbc) {
+    pdl_wait();
+    const int64_t p = op_point<1>();
+    const int f = op_flavour();
     if (p >= g.npts) return;
     const PointIdx q = point_of(g, p);
+    prefetch_chi(chi, g, q, 1);
     double2 acc[4];
-    dwf_apply_flavour<DAG, IMASS>(acc, LdF64{in}, g, q, f, chif, diag, hpin, apbc != 0);
+    dwf_apply_flavour<DAG, IMASS>(acc, LdF64{in}, g, q, f, chi, diag, hpin, apbc != 0);
 #pragma unroll
     for (int d = 0; d < 4; d++) out[p + g.cs * (d + 4 * f)] = acc[d];
+}
+
+template <class... P, class... A>
+static void launch_op(void (*k)(P...), unsigned nb, unsigned threads, cudaStream_t st, A... a) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(nb);
+    c.blockDim = dim3(threads);
+    c.stream = st;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    cudaLaunchKernelEx(&c, k, a...);
+    count_launches(1);
 }
 
 static inline float diag_of(float am3) { return 2.0f * ((3.0f - am3) + 1.0f); }  // :2652
@@ -195,32 +244,30 @@ bool op_rows_launchable(const Geom& g, int elem) {
                        : op_rows_setup<__half2, float2, false, 1, 1>(g, rp, &nb);
 }
 
-void launch_dslash64(bool dag, int imass, double2* out, const double2* in, const float* chif,
+void launch_dslash64(bool dag, int imass, double2* out, const double2* in, OpChi chi,
                      const Geom& g, float am3, float hpin, int ibound, cudaStream_t st,
                      int variant) {
-    const unsigned nb = split_blocks(g.npts);
+    const unsigned nb = op_blocks(g.npts, 1);
     const double diag = (double)diag_of(am3), hp = (double)hpin;
     const int apbc = ibound == -1;
     const int shape = variant < 0 ? stencil_choice(g, 16, st) : variant;
-    if (shape == kStencilRows &&
-        launch_op_rows_any<double2, double2>(dag, imass, out, in, chif, g, diag, hp, apbc, st)) {
-        note_stencil(kStencilRows, 1);
-        return;
+    if (shape == kStencilRows) {
+        launch_round_chi(chi.chi, chi.scratch, g.kvol, st);
+        if (launch_op_rows_any<double2, double2>(dag, imass, out, in, chi.scratch, g, diag, hp,
+                                                 apbc, st)) {
+            note_stencil(kStencilRows, 1);
+            return;
+        }
     }
     note_stencil(shape == kStencilGather4 ? kStencilGather4 : kStencilGather3, 1);
 #define LAUNCH(D, I)                                                                          \
-    do {                                                                                      \
-        if (shape == kStencilGather4)                                                         \
-            k_dslash64<D, I, 4><<<nb, kSplitThreads, 0, st>>>(out, in, chif, g, diag, hp, apbc); \
-        else                                                                                  \
-            k_dslash64<D, I, 3><<<nb, kSplitThreads, 0, st>>>(out, in, chif, g, diag, hp, apbc); \
-    } while (0)
+    launch_op(shape == kStencilGather4 ? k_dslash64<D, I, 8> : k_dslash64<D, I, 6>, nb,       \
+              kOpThreads, st, out, in, chi.chi, g, diag, hp, apbc)
     if (!dag) {
         if (imass == 1) LAUNCH(false, 1); else if (imass == 3) LAUNCH(false, 3); else LAUNCH(false, 0);
     } else {
         if (imass == 1) LAUNCH(true, 1); else if (imass == 3) LAUNCH(true, 3); else LAUNCH(true, 0);
     }
-    count_launches(1);
 #undef LAUNCH
 }
 
@@ -240,14 +287,15 @@ struct LdF16 {
 template <bool DAG, int IMASS, int HALF>
 __global__ void __launch_bounds__(kThreads) k_dslash_lp(void* __restrict__ out,
                                                        const void* __restrict__ in,
-                                                       const float* __restrict__ chif, Geom g,
+                                                       const double* __restrict__ chi, Geom g,
                                                        float diag, float hpin, int apbc) {
+    pdl_wait();
     const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (p >= g.npts) return;
     const PointIdx q = point_of(g, p);
     float2 acc[2][4];
-    if (HALF) dwf_apply_point<DAG, IMASS>(acc, LdF16{(const __half2*)in}, g, q, chif, diag, hpin, apbc != 0);
-    else dwf_apply_point<DAG, IMASS>(acc, LdF32{(const float2*)in}, g, q, chif, diag, hpin, apbc != 0);
+    if (HALF) dwf_apply_point<DAG, IMASS>(acc, LdF16{(const __half2*)in}, g, q, chi, diag, hpin, apbc != 0);
+    else dwf_apply_point<DAG, IMASS>(acc, LdF32{(const float2*)in}, g, q, chi, diag, hpin, apbc != 0);
 #pragma unroll
     for (int f = 0; f < 2; f++)
 #pragma unroll
@@ -259,19 +307,19 @@ __global__ void __launch_bounds__(kThreads) k_dslash_lp(void* __restrict__ out,
 }
 
 // FP32 storage with Ls even: a thread takes two adjacent points of one
-// flavour with 16-byte loads (dwf_apply_flavour_pair); a block covers 128
-// point pairs of both flavours.
+// flavour with 16-byte loads (dwf_apply_flavour_pair).
 template <bool DAG, int IMASS, int OCC>
-__global__ void __launch_bounds__(kSplitThreads, OCC)
+__global__ void __launch_bounds__(kOpThreads, OCC)
     k_dslash_f32_pair(float2* __restrict__ out, const float2* __restrict__ in,
-                      const float* __restrict__ chif, Geom g, float diag, float hpin, int apbc) {
-    const int64_t p = (int64_t)blockIdx.x * (2 * kSplitPoints) +
-                      2 * (threadIdx.x & (kSplitPoints - 1));
-    const int f = split_flavour();
+                      const double* __restrict__ chi, Geom g, float diag, float hpin, int apbc) {
+    pdl_wait();
+    const int64_t p = op_point<2>();
+    const int f = op_flavour();
     if (p >= g.npts) return;
     const PointIdx q = point_of(g, p);
+    prefetch_chi(chi, g, q, 2);
     float2 acc[2][4];
-    dwf_apply_flavour_pair<DAG, IMASS>(acc, in, g, q, f, chif, diag, hpin, apbc != 0);
+    dwf_apply_flavour_pair<DAG, IMASS>(acc, in, g, q, f, chi, diag, hpin, apbc != 0);
 #pragma unroll
     for (int d = 0; d < 4; d++) {
         const int64_t e = p + g.cs * (d + 4 * f);
@@ -318,7 +366,7 @@ template <> struct Quad<__half2> {
 template <bool DAG, int IMASS, class S>
 __device__ __forceinline__ void dwf_apply_flavour_quad(float2 acc[4][4], const S* __restrict__ in,
                                                        const Geom& g, const PointIdx& q, int f,
-                                                       const float* __restrict__ chif,
+                                                       const double* __restrict__ chi,
                                                        float diag, float hpin, bool apbc) {
     constexpr int SF = DAG ? -1 : 1;
     const int L = g.L, Lt = g.Lt, Ls = g.Ls;
@@ -395,8 +443,8 @@ __device__ __forceinline__ void dwf_apply_flavour_quad(float2 acc[4][4], const S
     // both for Ls = 4)
     const bool atL = (q.s + 4 == Ls), at0 = (q.s == 0);
     if (!(atL || at0)) return;
-    const float c1f = __ldg(chif + q.site), c2f = __ldg(chif + g.kvol + q.site),
-                c3f = __ldg(chif + 2 * g.kvol + q.site);
+    const float c1f = (float)__ldg(chi + q.site), c2f = (float)__ldg(chi + g.kvol + q.site),
+                c3f = (float)__ldg(chi + 2 * g.kvol + q.site);
     const bool pin = (q.site == 0);
     if (atL && at0) {
         constexpr int WA = DAG ? 0 : 2;
@@ -419,16 +467,17 @@ __device__ __forceinline__ void dwf_apply_flavour_quad(float2 acc[4][4], const S
 }
 
 template <bool DAG, int IMASS, class S>
-__global__ void __launch_bounds__(kSplitThreads, 2)
-    k_dslash_quad(S* __restrict__ out, const S* __restrict__ in, const float* __restrict__ chif,
+__global__ void __launch_bounds__(kOpThreads, 4)
+    k_dslash_quad(S* __restrict__ out, const S* __restrict__ in, const double* __restrict__ chi,
                   Geom g, float diag, float hpin, int apbc) {
-    const int64_t p = (int64_t)blockIdx.x * (4 * kSplitPoints) +
-                      4 * (threadIdx.x & (kSplitPoints - 1));
-    const int f = split_flavour();
+    pdl_wait();
+    const int64_t p = op_point<4>();
+    const int f = op_flavour();
     if (p >= g.npts) return;
     const PointIdx q = point_of(g, p);
+    prefetch_chi(chi, g, q, 4);
     float2 acc[4][4];
-    dwf_apply_flavour_quad<DAG, IMASS, S>(acc, in, g, q, f, chif, diag, hpin, apbc != 0);
+    dwf_apply_flavour_quad<DAG, IMASS, S>(acc, in, g, q, f, chi, diag, hpin, apbc != 0);
 #pragma unroll
     for (int d = 0; d < 4; d++) {
         const float2 v[4] = {acc[0][d], acc[1][d], acc[2][d], acc[3][d]};
@@ -436,13 +485,15 @@ __global__ void __launch_bounds__(kSplitThreads, 2)
     }
 }
 
-void launch_dslash_lp(bool dag, int imass, int half, void* out, const void* in, const float* chif,
+void launch_dslash_lp(bool dag, int imass, int half, void* out, const void* in, OpChi chi,
                       const Geom& g, float am3, float hpin, int ibound, cudaStream_t st,
                       int variant) {
     const int shape = variant < 0 ? stencil_choice(g, half ? 4 : 8, st) : variant;
     if (shape == kStencilRows) {
         const float diag = diag_of(am3);
         const int apbc = ibound == -1;
+        const float* chif = chi.scratch;
+        launch_round_chi(chi.chi, chi.scratch, g.kvol, st);
         if (half ? launch_op_rows_any<__half2, float2>(dag, imass, (__half2*)out,
                                                        (const __half2*)in, chif, g, diag, hpin,
                                                        apbc, st)
@@ -455,43 +506,35 @@ void launch_dslash_lp(bool dag, int imass, int half, void* out, const void* in, 
     }
     note_stencil(shape == kStencilGather4 && !half ? kStencilGather4 : kStencilGather3, 1);
     if (half && g.Ls % 4 == 0) {
-        const unsigned nb4 = (unsigned)((g.npts + 4 * kSplitPoints - 1) / (4 * kSplitPoints));
+        const unsigned nb4 = op_blocks(g.npts, 4);
         const float diag = diag_of(am3);
         const int apbc = ibound == -1;
         __half2* o = (__half2*)out;
         const __half2* i = (const __half2*)in;
-#define PQ(D, I) k_dslash_quad<D, I, __half2><<<nb4, kSplitThreads, 0, st>>>(o, i, chif, g, diag, hpin, apbc)
+#define PQ(D, I) launch_op(k_dslash_quad<D, I, __half2>, nb4, kOpThreads, st, o, i, chi.chi, g, diag, hpin, apbc)
         if (!dag) { if (imass == 3) PQ(false, 3); else PQ(false, 1); }
         else { if (imass == 3) PQ(true, 3); else PQ(true, 1); }
 #undef PQ
-        count_launches(1);
         return;
     }
     if (!half && pair_ok(g)) {
-        const unsigned nb2 = (unsigned)((g.npts + 2 * kSplitPoints - 1) / (2 * kSplitPoints));
+        const unsigned nb2 = op_blocks(g.npts, 2);
         const float diag = diag_of(am3);
         const int apbc = ibound == -1;
         float2* o = (float2*)out;
         const float2* i = (const float2*)in;
-#define PR(D, I)                                                                             \
-    do {                                                                                     \
-        if (shape == kStencilGather4)                                                        \
-            k_dslash_f32_pair<D, I, 4><<<nb2, kSplitThreads, 0, st>>>(o, i, chif, g, diag, hpin, \
-                                                                     apbc);                  \
-        else                                                                                 \
-            k_dslash_f32_pair<D, I, 3><<<nb2, kSplitThreads, 0, st>>>(o, i, chif, g, diag, hpin, \
-                                                                     apbc);                  \
-    } while (0)
+#define PR(D, I)                                                                              \
+    launch_op(shape == kStencilGather4 ? k_dslash_f32_pair<D, I, 8> : k_dslash_f32_pair<D, I, 6>, \
+              nb2, kOpThreads, st, o, i, chi.chi, g, diag, hpin, apbc)
         if (!dag) { if (imass == 3) PR(false, 3); else PR(false, 1); }
         else { if (imass == 3) PR(true, 3); else PR(true, 1); }
 #undef PR
-        count_launches(1);
         return;
     }
     const unsigned nb = (unsigned)((g.npts + kThreads - 1) / kThreads);
     const float diag = diag_of(am3);
     const int apbc = ibound == -1;
-#define LP(D, I, H) k_dslash_lp<D, I, H><<<nb, kThreads, 0, st>>>(out, in, chif, g, diag, hpin, apbc)
+#define LP(D, I, H) launch_op(k_dslash_lp<D, I, H>, nb, kThreads, st, out, in, chi.chi, g, diag, hpin, apbc)
     if (half) {
         if (!dag) { if (imass == 3) LP(false, 3, 1); else LP(false, 1, 1); }
         else { if (imass == 3) LP(true, 3, 1); else LP(true, 1, 1); }
@@ -500,7 +543,6 @@ void launch_dslash_lp(bool dag, int imass, int half, void* out, const void* in, 
         else { if (imass == 3) LP(true, 3, 0); else LP(true, 1, 0); }
     }
 #undef LP
-    count_launches(1);
 }
 
 // M on npole stacked two-slice lattices: blockIdx.y = pole.

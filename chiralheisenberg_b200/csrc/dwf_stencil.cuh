@@ -187,11 +187,11 @@ __device__ __forceinline__ void wall_terms(T acc[4], const Ld& ld, int64_t cs, i
 // chi is passed pre-rounded to REAL*4: the reference builds the wall
 // coupling with cmplx(chi, ...) without a KIND, i.e. in default (single)
 // precision (cheisdwf.f:2914, :2962, :2998, :3034).  chif holds (chi1, chi2,
-// chi3) as three planes of kvol floats.
-template <bool DAG, int IMASS, class T, class Ld>
+// chi3) as three planes of kvol floats, or of doubles that are rounded here.
+template <bool DAG, int IMASS, class T, class Ld, class C>
 __device__ __forceinline__ void dwf_apply_flavour(T acc[4], const Ld& ld, const Geom& g,
                                                   const PointIdx& q, int f,
-                                                  const float* __restrict__ chif,
+                                                  const C* __restrict__ chif,
                                                   typename real_of<T>::type diag,
                                                   typename real_of<T>::type hpin, bool apbc) {
     typedef typename real_of<T>::type R;
@@ -241,17 +241,17 @@ __device__ __forceinline__ void dwf_apply_flavour(T acc[4], const Ld& ld, const 
     // wall coupling: the pair at s=Ls reads s=1, the pair at s=1 reads s=Ls
     const bool atL = (q.s == Ls - 1), at0 = (q.s == 0);
     if (!(atL || at0)) return;
-    const float c1f = __ldg(chif + q.site), c2f = __ldg(chif + g.kvol + q.site),
-                c3f = __ldg(chif + 2 * g.kvol + q.site);
+    const float c1f = (float)__ldg(chif + q.site), c2f = (float)__ldg(chif + g.kvol + q.site),
+                c3f = (float)__ldg(chif + 2 * g.kvol + q.site);
     const int64_t other = atL ? LsI * q.site : LsI * q.site + Ls - 1;
     const bool pin = (q.site == 0);
     wall_terms_rt<DAG, IMASS>(acc, ld, cs, other, atL, f, c1f, c2f, c3f, pin, hpin);
 }
 
 // All eight components of one output point (one thread per point).
-template <bool DAG, int IMASS, class T, class Ld>
+template <bool DAG, int IMASS, class T, class Ld, class C>
 __device__ __forceinline__ void dwf_apply_point(T acc[2][4], const Ld& ld, const Geom& g,
-                                                const PointIdx& q, const float* __restrict__ chif,
+                                                const PointIdx& q, const C* __restrict__ chif,
                                                 typename real_of<T>::type diag,
                                                 typename real_of<T>::type hpin, bool apbc) {
     dwf_apply_flavour<DAG, IMASS>(acc[0], ld, g, q, 0, chif, diag, hpin, apbc);
@@ -272,11 +272,11 @@ struct LdF2 {
 // address arithmetic of its 34 loads.
 inline bool pair_ok(const Geom& g) { return g.Ls % 2 == 0 && g.kferm < (int64_t(1) << 31); }
 
-template <bool DAG, int IMASS>
+template <bool DAG, int IMASS, class C>
 __device__ __forceinline__ void dwf_apply_flavour_pair(float2 acc[2][4],
                                                        const float2* __restrict__ in,
                                                        const Geom& g, const PointIdx& q, int f,
-                                                       const float* __restrict__ chif, float diag,
+                                                       const C* __restrict__ chif, float diag,
                                                        float hpin, bool apbc) {
     constexpr int SF = DAG ? -1 : 1;
     const int L = g.L, Lt = g.Lt, Ls = g.Ls;
@@ -365,8 +365,8 @@ __device__ __forceinline__ void dwf_apply_flavour_pair(float2 acc[2][4],
     constexpr int WB = DAG ? 2 : 0;
     const bool atL = (q.s + 2 == Ls), at0 = (q.s == 0);
     if (!(atL || at0)) return;
-    const float c1f = __ldg(chif + q.site), c2f = __ldg(chif + g.kvol + q.site),
-                c3f = __ldg(chif + 2 * g.kvol + q.site);
+    const float c1f = (float)__ldg(chif + q.site), c2f = (float)__ldg(chif + g.kvol + q.site),
+                c3f = (float)__ldg(chif + 2 * g.kvol + q.site);
     const bool pin = (q.site == 0);
     if (atL && at0) {   // Ls = 2: one pair holds both walls
         wall_terms<DAG, IMASS, WA, 0>(acc[1], LdF2{in}, cs, LsI * q.site, f, c1f, c2f, c3f, pin, hpin);
@@ -399,11 +399,11 @@ struct LdSp {
 // and three-term step done as packed FP32x2 operations on both points at
 // once.  The s hops and the wall terms act on one point of the pair and stay
 // per point.  Needs pair_ok(g).
-template <bool DAG, int IMASS>
+template <bool DAG, int IMASS, class C>
 __device__ __forceinline__ void dwf_apply_flavour_pair_sp(cpair acc[4],
                                                           const float2* __restrict__ in,
                                                           const Geom& g, const PointIdx& q, int f,
-                                                          const float* __restrict__ chif,
+                                                          const C* __restrict__ chif,
                                                           float diag, float hpin, bool apbc) {
     constexpr int SF = DAG ? -1 : 1;
     const int L = g.L, Lt = g.Lt, Ls = g.Ls;
@@ -475,8 +475,8 @@ __device__ __forceinline__ void dwf_apply_flavour_pair_sp(cpair acc[4],
     constexpr int WB = DAG ? 2 : 0;
     const bool atL = (q.s + 2 == Ls), at0 = (q.s == 0);
     if (!(atL || at0)) return;
-    const float c1f = __ldg(chif + q.site), c2f = __ldg(chif + g.kvol + q.site),
-                c3f = __ldg(chif + 2 * g.kvol + q.site);
+    const float c1f = (float)__ldg(chif + q.site), c2f = (float)__ldg(chif + g.kvol + q.site),
+                c3f = (float)__ldg(chif + 2 * g.kvol + q.site);
     const bool pin = (q.site == 0);
     if (atL && at0) {   // Ls = 2: one pair holds both walls
         float2 w0[4], w1[4];
@@ -521,11 +521,5 @@ __device__ __forceinline__ void dwf_apply_flavour_pair_sp(cpair acc[4],
 constexpr int kSplitThreads = 256;
 constexpr int kSplitPoints = kSplitThreads / 2;
 __device__ __forceinline__ int split_flavour() { return threadIdx.x >= kSplitPoints; }
-__device__ __forceinline__ int64_t split_point() {
-    return (int64_t)blockIdx.x * kSplitPoints + (threadIdx.x & (kSplitPoints - 1));
-}
-inline unsigned split_blocks(int64_t npts) {
-    return (unsigned)((npts + kSplitPoints - 1) / kSplitPoints);
-}
 
 }  // namespace chdwf

@@ -60,18 +60,24 @@ struct LzHist {
 // Operator launchers (FP64, exact evaluation order).
 // variant: -1 the tuned choice (stencil_choice), or one of the kStencil*
 // shapes below (the row-staged one wherever its shared memory fits).
-void launch_dslash64(bool dag, int imass, double2* out, const double2* in, const float* chif,
+// chi on the device: REAL*8, rounded to REAL*4 by the kernels; scratch (3*kvol
+// floats) holds the rounded copy that the row-staged shape reads.
+struct OpChi {
+    const double* chi;
+    float* scratch;
+};
+void launch_dslash64(bool dag, int imass, double2* out, const double2* in, OpChi chi,
                      const Geom& g, float am3, float hpin, int ibound, cudaStream_t st,
                      int variant = -1);
 
 // Operator on FP32 (half=0, complex64) or FP16 (half=1, two halves per
 // complex) storage with FP32 arithmetic.
-void launch_dslash_lp(bool dag, int imass, int half, void* out, const void* in, const float* chif,
+void launch_dslash_lp(bool dag, int imass, int half, void* out, const void* in, OpChi chi,
                       const Geom& g, float am3, float hpin, int ibound, cudaStream_t st,
                       int variant = -1);
 
-// Stencil kernel shapes: the point-gather kernels with 3 blocks of 256 a SM
-// (80 registers a thread) or 4 (64 registers), or the row-staged kernels.
+// Stencil kernel shapes: the point-gather kernels with 80 registers a thread
+// or 64, or the row-staged kernels.
 constexpr int kStencilGather3 = 0, kStencilRows = 1, kStencilGather4 = 2;
 
 // Autotuner (tune.cu): the stencil shape for this lattice and element size

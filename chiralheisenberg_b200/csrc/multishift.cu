@@ -101,11 +101,11 @@ struct MsWork {
 
 // Residual vector Phi - (M^dag M + sigma) x into r, block partials of its
 // square into part (FP64)
-void true_residual(Ctx* c, MsWork& w, const double2* phi, const double2* x, double sigma,
-                   float hpin, int imass, double2* r, double* part) {
+void true_residual(Ctx* c, MsWork& w, const double* chi, const double2* phi, const double2* x,
+                   double sigma, float hpin, int imass, double2* r, double* part) {
     const Geom& g = c->g;
-    launch_dslash64(false, imass, w.t, x, c->chif, g, c->am3, hpin, c->ibound, c->stream);
-    launch_dslash64(true, imass, c->spin[3], w.t, c->chif, g, c->am3, hpin, c->ibound, c->stream);
+    launch_dslash64(false, imass, w.t, x, {chi, c->chif}, g, c->am3, hpin, c->ibound, c->stream);
+    launch_dslash64(true, imass, c->spin[3], w.t, {chi, c->chif}, g, c->am3, hpin, c->ibound, c->stream);
     k_ms_resid<<<reduce_blocks(g.kferm), kThreads, 0, c->stream>>>(r, phi, c->spin[3], x, sigma,
                                                                   g.kferm, part);
     count_launches(1);
@@ -129,7 +129,8 @@ constexpr double kMsInner = 1e-5;      // least relative residual of an inner so
 
 // Defect correction of the shifts k0..k0+n-1 together, until each one's true
 // residual is at most res or stops falling.
-cudaError_t correct_part(Ctx* c, MsWork& w, PcgWork<float2>& P, const double2* phi, double phin,
+cudaError_t correct_part(Ctx* c, MsWork& w, PcgWork<float2>& P, const double* chi,
+                         const double2* phi, double phin,
                          float res, float hpin, int imass, int k0, int n, const double* sigma,
                          void* const* x, double* true_res, int* iters) {
     const Geom& g = c->g;
@@ -143,7 +144,7 @@ cudaError_t correct_part(Ctx* c, MsWork& w, PcgWork<float2>& P, const double2* p
     for (int round = 0; !run.empty(); round++) {
         for (size_t a = 0; a < run.size(); a++) {
             const int i = run[a];
-            true_residual(c, w, phi, (const double2*)x[k0 + i], sigma[k0 + i], hpin, imass,
+            true_residual(c, w, chi, phi, (const double2*)x[k0 + i], sigma[k0 + i], hpin, imass,
                           w.r + g.kferm * (int64_t)a, w.part + (size_t)nb * a);
         }
         if ((e = run_sums(w.part, (int)run.size(), nb, r2.data(), st))) return e;
@@ -267,14 +268,14 @@ extern "C" int chdwf_multishift_dev(chdwf_ctx* ctx, const void* Phi, float res, 
         if ((e = P.reserve(B.units, 0, B.parts))) return c->status_of(e, "multishift: workspace");
         for (int k0 = 0; k0 < n; k0 += np) {
             const int m = n - k0 < np ? n - k0 : np;
-            if ((e = correct_part(c, w, P, (const double2*)Phi, phin, res, hpin, imass, k0, m, sigma,
+            if ((e = correct_part(c, w, P, (const double*)chi, (const double2*)Phi, phin, res, hpin, imass, k0, m, sigma,
                                   x, true_res, refine_iters)))
                 return c->status_of(e, "multishift refinement");
         }
     } else {
         for (int k = 0; k < n; k++) {
             double r2 = 0.0;
-            true_residual(c, w, (const double2*)Phi, (const double2*)x[k], sigma[k], hpin, imass, w.r,
+            true_residual(c, w, (const double*)chi, (const double2*)Phi, (const double2*)x[k], sigma[k], hpin, imass, w.r,
                           w.part);
             if ((e = run_sums(w.part, 1, reduce_blocks(g.kferm), &r2, st)))
                 return c->status_of(e, "multishift residual");

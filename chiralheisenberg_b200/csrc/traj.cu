@@ -325,7 +325,7 @@ int chdwf_traj_propagator(chdwf_ctx* ctx, int ittt, int idsource, float res, flo
     k_wall_source<<<nblk(ksize2), kThreads, 0, c->stream>>>(xi, g, (int64_t)(ittt - 1) * ksize2,
                                                              idsource, val); count_launches(1);
     launch_round_chi(c->chit, c->chif, g.kvol, c->stream);
-    launch_dslash64(true, imass, Phi, xi, c->chif, g, c->am3, hpin, c->ibound, c->stream);  // :979
+    launch_dslash64(true, imass, Phi, xi, {c->chit, c->chif}, g, c->am3, hpin, c->ibound, c->stream);  // :979
     cudaMemcpyAsync(xi, Phi, sizeof(double2) * g.kferm, cudaMemcpyDeviceToDevice, c->stream);  // :983-991
     int st = 0;
     cudaError_t e = cg_solve(c->cg, g, Phi, res, c->chif, c->am3, hpin, imass, c->ibound, xi,
@@ -370,7 +370,7 @@ int chdwf_traj_propagators(chdwf_ctx* ctx, int nsrc, const int* ittt, const int*
         k_wall_source<<<nblk(ksize2), kThreads, 0, c->stream>>>(
             xi, g, (int64_t)(ittt[i] - 1) * ksize2, idsource[i], val);
         count_launches(1);
-        launch_dslash64(true, imass, Phi, xi, c->chif, g, c->am3, hpin, c->ibound,
+        launch_dslash64(true, imass, Phi, xi, {c->chit, c->chif}, g, c->am3, hpin, c->ibound,
                         c->stream);                                                // :979
         cudaMemcpyAsync(xi, Phi, sizeof(double2) * g.kferm, cudaMemcpyDeviceToDevice,
                         c->stream);                                                // :983-991
@@ -409,7 +409,7 @@ int chdwf_traj_noise_solve(chdwf_ctx* ctx, const float* eta, int swall, int idir
     k_noise_source<<<nblk(2 * (int64_t)g.kvol), kThreads, 0, c->stream>>>(
         xi, g, eta_d, swall - 1, idirac - 1); count_launches(1);
     launch_round_chi(c->chit, c->chif, g.kvol, c->stream);
-    launch_dslash64(true, imass, Phi, xi, c->chif, g, c->am3, hpin, c->ibound, c->stream);  // :1273
+    launch_dslash64(true, imass, Phi, xi, {c->chit, c->chif}, g, c->am3, hpin, c->ibound, c->stream);  // :1273
     cudaMemcpyAsync(xi, Phi, sizeof(double2) * g.kferm, cudaMemcpyDeviceToDevice, c->stream);  // :1277-1282
     int st = 0;
     cudaError_t e = cg_solve(c->cg, g, Phi, res, c->chif, c->am3, hpin, imass, c->ibound, xi,

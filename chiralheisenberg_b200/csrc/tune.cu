@@ -2,15 +2,15 @@
 //
 // The domain-wall operator has three kernel shapes: the point-gather kernels
 // (dwf_stencil.cuh: one thread per point and flavour, every neighbour read
-// through L1/L2) at a register budget of 80 a thread (3 blocks of 256 a
-// SM) or 64 (4 blocks, more warps in flight, some spills), and the
+// through L1/L2) at a register budget of 80 a thread (24 warps a SM, the
+// shape called gather3) or 64 (gather4: 32 warps, some spills), and the
 // row-staged kernels (row_stage.cuh: rows y-1..y+1 and t-1, t+1 staged in
 // shared memory by bulk copies), where they can launch.  Which is fastest
 // depends on the lattice and the precision.  On the first use of a (L, Lt,
 // Ls, element size) the tuner applies M in every shape to scratch vectors on
 // the caller's stream -- 2 warm-up and 5 timed applications each, CUDA
 // events, L2 not flushed (all see the same cache state) -- and keeps the
-// fastest, the 3-block point-gather kernel unless another shape is faster
+// fastest, the 80-register point-gather kernel unless another shape is faster
 // by more than kTuneMargin (10%).  The choice holds for the operator on
 // spinors in the ABI's layout; the multi-shift solver's vectors are planes
 // (planes.cuh), whose launch plan is a rule of its own.  The table is per
@@ -39,7 +39,7 @@ const char* shape_name(int k) {
     return k == kStencilRows ? "rows" : (k == kStencilGather4 ? "gather4" : "gather3");
 }
 
-// Another shape replaces the 3-block point-gather kernels only when the probe
+// Another shape replaces the 80-register point-gather kernels only when the probe
 // finds it faster by more than 10%: the probe's spread from box to box is 5%.
 constexpr float kTuneMargin = 0.10f;
 
@@ -47,14 +47,14 @@ std::mutex g_tune_mu;
 std::vector<TuneEntry> g_tune;
 
 // median microseconds of 5 applications (after 2) of variant v
-float time_variant(const Geom& g, int elem, int v, void* out, const void* in, const float* chif,
+float time_variant(const Geom& g, int elem, int v, void* out, const void* in, OpChi chi,
                    cudaStream_t st) {
     auto apply = [&] {
         if (elem == 16)
-            launch_dslash64(false, 1, (double2*)out, (const double2*)in, chif, g, 1.0f, 0.0f, -1,
+            launch_dslash64(false, 1, (double2*)out, (const double2*)in, chi, g, 1.0f, 0.0f, -1,
                             st, v);
         else
-            launch_dslash_lp(false, 1, elem == 4 ? 1 : 0, out, in, chif, g, 1.0f, 0.0f, -1, st,
+            launch_dslash_lp(false, 1, elem == 4 ? 1 : 0, out, in, chi, g, 1.0f, 0.0f, -1, st,
                              v);
     };
     for (int k = 0; k < 2; k++) apply();
@@ -96,20 +96,20 @@ int stencil_choice(const Geom& g, int elem, cudaStream_t st) {
     }
     // measure on scratch vectors (zeros: the same memory traffic)
     void *in = nullptr, *out = nullptr;
-    float* chif = nullptr;
+    double* chi = nullptr;            // and the rounded copy behind it
     const size_t bytes = (size_t)elem * g.kferm;
     TuneEntry t{g.L, g.Lt, g.Ls, elem, dev, kStencilGather3, {0.0f, 0.0f, 0.0f}};
     if (cudaMalloc(&in, bytes) == cudaSuccess && cudaMalloc(&out, bytes) == cudaSuccess &&
-        cudaMalloc(&chif, sizeof(float) * 3 * (size_t)g.kvol) == cudaSuccess) {
+        cudaMalloc(&chi, sizeof(double) * 6 * (size_t)g.kvol) == cudaSuccess) {
         cudaMemsetAsync(in, 0, bytes, st);
-        cudaMemsetAsync(chif, 0, sizeof(float) * 3 * (size_t)g.kvol, st);
-        // another shape replaces the point-gather kernel at 3 blocks a SM
+        cudaMemsetAsync(chi, 0, sizeof(double) * 6 * (size_t)g.kvol, st);
+        // another shape replaces the 80-register point-gather kernel
         // only if it is faster by more than kTuneMargin
         float best = 0.0f;
         for (int k : {kStencilGather3, kStencilGather4, kStencilRows}) {
             if (k == kStencilRows && !(rows_fit && op_rows_launchable(g, elem))) continue;
             if (k == kStencilGather4 && elem == 4) continue;   // one FP16 gather kernel
-            t.us[k] = time_variant(g, elem, k, out, in, chif, st);
+            t.us[k] = time_variant(g, elem, k, out, in, {chi, (float*)(chi + 3 * (size_t)g.kvol)}, st);
             if (best == 0.0f || t.us[k] < best * (1.0f - kTuneMargin)) {
                 best = t.us[k];
                 t.choice = k;
@@ -119,7 +119,7 @@ int stencil_choice(const Geom& g, int elem, cudaStream_t st) {
     cudaGetLastError();
     cudaFree(in);
     cudaFree(out);
-    cudaFree(chif);
+    cudaFree(chi);
     std::lock_guard<std::mutex> lk(g_tune_mu);
     g_tune.push_back(t);
     return t.choice;
