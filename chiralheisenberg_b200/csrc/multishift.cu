@@ -15,7 +15,7 @@
 //
 // The corrections of several shifts run as one batch (plane_cg.cuh): their
 // scalars stay on the device and each iteration is three launches for all of
-// them: 20 shifts at 16^3x16 to 1e-10 take 98 ms.  One shift at a time, with
+// them: 20 shifts at 16^3x16 to 1e-10 take 91 ms.  One shift at a time, with
 // the scalars on the host (two round trips an iteration), they took 615 ms.
 #include <cmath>
 #include <cstring>
@@ -125,7 +125,8 @@ cudaError_t run_sums(const double* part_dev, int n, int len, double* out, cudaSt
 }
 
 constexpr int kMsRounds = 20;          // corrections of one shift at most
-constexpr double kMsInner = 1e-5;      // least relative residual of an inner solve
+constexpr double kMsInner = 1e-5;      // relative residual of an inner solve, least
+constexpr double kMsOuter = 1e-4;      // and largest
 
 // Defect correction of the shifts k0..k0+n-1 together, until each one's true
 // residual is at most res or stops falling.
@@ -180,11 +181,11 @@ cudaError_t correct_part(Ctx* c, MsWork& w, PcgWork<float2>& P, const double* ch
         }
         for (size_t a = 0; a < run.size(); a++) {
             if ((e = run_sums(P.part + B.a.part0[a] + 2 * nblk, 1, neblk, &rr[a], st))) return e;
-            // one round to a tenth of res where FP32 can reach it: x is then
-            // 1.5e-10 from 64 bits (a quarter of res: 3.8e-10; rounds of a
-            // fixed 1e-4: 2.6e-10)
+            // one round to a tenth of res where FP32 can reach it, and never
+            // less than four digits: x is then 1.5e-10 from 64 bits at res
+            // 1e-10 (a quarter of res: 3.8e-10; a fixed 1e-4: 2.6e-10)
             double tol = 0.1 * (double)res / rel[run[a]];
-            tol = tol < kMsInner ? kMsInner : (tol > 0.5 ? 0.5 : tol);
+            tol = tol < kMsInner ? kMsInner : (tol > kMsOuter ? kMsOuter : tol);
             memset(&slots[a], 0, sizeof(PcgSlot));
             slots[a].rr = rr[a];
             PcgDyn<float2> d;
