@@ -124,6 +124,7 @@ cudaError_t run_sums(const double* part_dev, int n, int len, double* out, cudaSt
     return e;
 }
 
+constexpr double kMsBytes = 90e6;      // FP32 vectors of a part: they stay in L2
 constexpr int kMsRounds = 20;          // corrections of one shift at most
 constexpr double kMsInner = 1e-5;      // relative residual of an inner solve, least
 constexpr double kMsOuter = 1e-4;      // and largest
@@ -233,7 +234,7 @@ extern "C" int chdwf_multishift_dev(chdwf_ctx* ctx, const void* Phi, float res, 
     // shifts that are corrected together: as many as keep their four FP32
     // vectors in L2
     const size_t ve = (size_t)plane_elems<float2>(g) / 2;
-    int np = prec == CHDWF_PREC_F32 ? (int)(90e6 / (64.0 * (double)ve)) : 1;
+    int np = prec == CHDWF_PREC_F32 ? (int)(kMsBytes / (64.0 * (double)ve)) : 1;
     np = np < 1 ? 1 : (np > n ? n : np);
     if ((e = cudaMalloc(&w.t, sizeof(double2) * g.kferm)) ||
         (e = cudaMalloc(&w.r, sizeof(double2) * g.kferm * np)) ||
@@ -273,6 +274,8 @@ extern "C" int chdwf_multishift_dev(chdwf_ctx* ctx, const void* Phi, float res, 
                                   x, true_res, refine_iters)))
                 return c->status_of(e, "multishift refinement");
         }
+        // kept for the next call while it is small beside what a solve holds
+        if (64.0 * (double)ve > kMsBytes) P.release();
     } else {
         for (int k = 0; k < n; k++) {
             double r2 = 0.0;
