@@ -13,15 +13,17 @@
 namespace chdwf {
 
 struct LdF64 {
-    const double2* __restrict__ p;
-    __device__ __forceinline__ double2 operator()(int64_t j) const { return __ldg(p + j); }
+    const double2* p;
+    __device__ __forceinline__ double2 operator()(int64_t j) const { return p[j]; }
 };
 
 // The operator on the ABI's spinors takes chi as the callers have it, REAL*8,
 // and rounds it to REAL*4 where a wall reads it, and is launched with
 // programmatic serialisation: its blocks are scheduled while the kernel before
-// it drains.  At 8^3x8 a call takes 4.7 us (5.3 without the latter),
-// against 7.7 with a rounding kernel in front of it.
+// it drains.  What that kernel writes may be what this one reads, so in and chi
+// are read by coherent loads only, behind pdl_wait.  At 8^3x8 a call takes 4.7 us
+// (5.3 without programmatic serialisation), against 7.7 with a rounding kernel in
+// front of it.
 
 // chi of a wall point on its way while the hops are formed: it comes from HBM
 // where the rounded copy used to be in L2.
@@ -52,8 +54,8 @@ static unsigned op_blocks(int64_t npts, int pt) {
 // Flavour-split: two threads per point; OCC blocks a SM (the register budget).
 template <bool DAG, int IMASS, int OCC>
 __global__ void __launch_bounds__(kOpThreads, OCC)
-    k_dslash64(double2* __restrict__ out, const double2* __restrict__ in,
-               const double* __restrict__ chi, Geom g, double diag, double hpin, int apbc) {
+    k_dslash64(double2* out, const double2* in, const double* chi, Geom g, double diag,
+               double hpin, int apbc) {
     pdl_wait();
     const int64_t p = op_point<1>();
     const int f = op_flavour();
@@ -274,20 +276,19 @@ void launch_dslash64(bool dag, int imass, double2* out, const double2* in, OpChi
 // ---- reduced-precision storage: FP32 spinors (complex64) and FP16 spinors
 // (two halves per complex), FP32 arithmetic ----------------------------------
 struct LdF32 {
-    const float2* __restrict__ p;
-    __device__ __forceinline__ float2 operator()(int64_t j) const { return __ldg(p + j); }
+    const float2* p;
+    __device__ __forceinline__ float2 operator()(int64_t j) const { return p[j]; }
 };
 struct LdF16 {
-    const __half2* __restrict__ p;
-    __device__ __forceinline__ float2 operator()(int64_t j) const { return __half22float2(__ldg(p + j)); }
+    const __half2* p;
+    __device__ __forceinline__ float2 operator()(int64_t j) const { return __half22float2(p[j]); }
 };
 
 // One thread per point and both flavours: with FP32 arithmetic the registers
 // already allow full occupancy, and this shape is the faster one there.
 template <bool DAG, int IMASS, int HALF>
-__global__ void __launch_bounds__(kThreads) k_dslash_lp(void* __restrict__ out,
-                                                       const void* __restrict__ in,
-                                                       const double* __restrict__ chi, Geom g,
+__global__ void __launch_bounds__(kThreads) k_dslash_lp(void* out, const void* in,
+                                                       const double* chi, Geom g,
                                                        float diag, float hpin, int apbc) {
     pdl_wait();
     const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -310,8 +311,8 @@ __global__ void __launch_bounds__(kThreads) k_dslash_lp(void* __restrict__ out,
 // flavour with 16-byte loads (dwf_apply_flavour_pair).
 template <bool DAG, int IMASS, int OCC>
 __global__ void __launch_bounds__(kOpThreads, OCC)
-    k_dslash_f32_pair(float2* __restrict__ out, const float2* __restrict__ in,
-                      const double* __restrict__ chi, Geom g, float diag, float hpin, int apbc) {
+    k_dslash_f32_pair(float2* out, const float2* in, const double* chi, Geom g, float diag,
+                      float hpin, int apbc) {
     pdl_wait();
     const int64_t p = op_point<2>();
     const int f = op_flavour();
@@ -348,7 +349,7 @@ template <class S> struct Quad;
 template <> struct Quad<__half2> {
     uint4 v;
     __device__ __forceinline__ void load(const __half2* p, int64_t n) {
-        v = __ldg(reinterpret_cast<const uint4*>(p + n));
+        v = *reinterpret_cast<const uint4*>(p + n);
     }
     __device__ __forceinline__ float2 get(int k) const {
         return h2_get(k == 0 ? v.x : (k == 1 ? v.y : (k == 2 ? v.z : v.w)));
@@ -364,9 +365,9 @@ template <> struct Quad<__half2> {
     typedef LdF16 Elem;
 };
 template <bool DAG, int IMASS, class S>
-__device__ __forceinline__ void dwf_apply_flavour_quad(float2 acc[4][4], const S* __restrict__ in,
+__device__ __forceinline__ void dwf_apply_flavour_quad(float2 acc[4][4], const S* in,
                                                        const Geom& g, const PointIdx& q, int f,
-                                                       const double* __restrict__ chi,
+                                                       const double* chi,
                                                        float diag, float hpin, bool apbc) {
     constexpr int SF = DAG ? -1 : 1;
     const int L = g.L, Lt = g.Lt, Ls = g.Ls;
@@ -443,8 +444,8 @@ __device__ __forceinline__ void dwf_apply_flavour_quad(float2 acc[4][4], const S
     // both for Ls = 4)
     const bool atL = (q.s + 4 == Ls), at0 = (q.s == 0);
     if (!(atL || at0)) return;
-    const float c1f = (float)__ldg(chi + q.site), c2f = (float)__ldg(chi + g.kvol + q.site),
-                c3f = (float)__ldg(chi + 2 * g.kvol + q.site);
+    const float c1f = (float)chi[q.site], c2f = (float)chi[g.kvol + q.site],
+                c3f = (float)chi[2 * g.kvol + q.site];
     const bool pin = (q.site == 0);
     if (atL && at0) {
         constexpr int WA = DAG ? 0 : 2;
@@ -468,8 +469,8 @@ __device__ __forceinline__ void dwf_apply_flavour_quad(float2 acc[4][4], const S
 
 template <bool DAG, int IMASS, class S>
 __global__ void __launch_bounds__(kOpThreads, 4)
-    k_dslash_quad(S* __restrict__ out, const S* __restrict__ in, const double* __restrict__ chi,
-                  Geom g, float diag, float hpin, int apbc) {
+    k_dslash_quad(S* out, const S* in, const double* chi, Geom g, float diag, float hpin,
+                  int apbc) {
     pdl_wait();
     const int64_t p = op_point<4>();
     const int f = op_flavour();

@@ -10,6 +10,12 @@
 //   s hop; chi3 wall term; pinning term; chi1/chi2 wall term.
 // With the exact (non-contracted) FP64 helpers the result is bit-identical to
 // the sweep-by-sweep evaluation.
+//
+// The element functions read their input and chi by plain, coherent loads
+// (no __ldg, no __restrict__ on what is read): the operator kernels are
+// launched with programmatic serialisation and may be resident while the
+// kernel before them still writes the vector that they will read, which the
+// non-coherent path does not allow.
 #pragma once
 #include "common.cuh"
 
@@ -191,7 +197,7 @@ __device__ __forceinline__ void wall_terms(T acc[4], const Ld& ld, int64_t cs, i
 template <bool DAG, int IMASS, class T, class Ld, class C>
 __device__ __forceinline__ void dwf_apply_flavour(T acc[4], const Ld& ld, const Geom& g,
                                                   const PointIdx& q, int f,
-                                                  const C* __restrict__ chif,
+                                                  const C* chif,
                                                   typename real_of<T>::type diag,
                                                   typename real_of<T>::type hpin, bool apbc) {
     typedef typename real_of<T>::type R;
@@ -241,8 +247,8 @@ __device__ __forceinline__ void dwf_apply_flavour(T acc[4], const Ld& ld, const 
     // wall coupling: the pair at s=Ls reads s=1, the pair at s=1 reads s=Ls
     const bool atL = (q.s == Ls - 1), at0 = (q.s == 0);
     if (!(atL || at0)) return;
-    const float c1f = (float)__ldg(chif + q.site), c2f = (float)__ldg(chif + g.kvol + q.site),
-                c3f = (float)__ldg(chif + 2 * g.kvol + q.site);
+    const float c1f = (float)chif[q.site], c2f = (float)chif[g.kvol + q.site],
+                c3f = (float)chif[2 * g.kvol + q.site];
     const int64_t other = atL ? LsI * q.site : LsI * q.site + Ls - 1;
     const bool pin = (q.site == 0);
     wall_terms_rt<DAG, IMASS>(acc, ld, cs, other, atL, f, c1f, c2f, c3f, pin, hpin);
@@ -251,7 +257,7 @@ __device__ __forceinline__ void dwf_apply_flavour(T acc[4], const Ld& ld, const 
 // All eight components of one output point (one thread per point).
 template <bool DAG, int IMASS, class T, class Ld, class C>
 __device__ __forceinline__ void dwf_apply_point(T acc[2][4], const Ld& ld, const Geom& g,
-                                                const PointIdx& q, const C* __restrict__ chif,
+                                                const PointIdx& q, const C* chif,
                                                 typename real_of<T>::type diag,
                                                 typename real_of<T>::type hpin, bool apbc) {
     dwf_apply_flavour<DAG, IMASS>(acc[0], ld, g, q, 0, chif, diag, hpin, apbc);
@@ -259,8 +265,8 @@ __device__ __forceinline__ void dwf_apply_point(T acc[2][4], const Ld& ld, const
 }
 
 struct LdF2 {
-    const float2* __restrict__ p;
-    __device__ __forceinline__ float2 operator()(int64_t j) const { return __ldg(p + j); }
+    const float2* p;
+    __device__ __forceinline__ float2 operator()(int64_t j) const { return p[j]; }
 };
 
 // Two adjacent points (s, s+1), s even, of flavour f on FP32 storage.  Each
@@ -274,16 +280,16 @@ inline bool pair_ok(const Geom& g) { return g.Ls % 2 == 0 && g.kferm < (int64_t(
 
 template <bool DAG, int IMASS, class C>
 __device__ __forceinline__ void dwf_apply_flavour_pair(float2 acc[2][4],
-                                                       const float2* __restrict__ in,
+                                                       const float2* in,
                                                        const Geom& g, const PointIdx& q, int f,
-                                                       const C* __restrict__ chif, float diag,
+                                                       const C* chif, float diag,
                                                        float hpin, bool apbc) {
     constexpr int SF = DAG ? -1 : 1;
     const int L = g.L, Lt = g.Lt, Ls = g.Ls;
     const uint32_t LsI = (uint32_t)Ls, cs = (uint32_t)g.cs, fo = cs * (uint32_t)(4 * f);
     const uint32_t qp = (uint32_t)q.p;
     auto ld2 = [&](uint32_t n, float2& r0, float2& r1) {
-        const float4 v = __ldg(reinterpret_cast<const float4*>(in + n));
+        const float4 v = *reinterpret_cast<const float4*>(in + n);
         r0 = make_float2(v.x, v.y);
         r1 = make_float2(v.z, v.w);
     };
@@ -365,8 +371,8 @@ __device__ __forceinline__ void dwf_apply_flavour_pair(float2 acc[2][4],
     constexpr int WB = DAG ? 2 : 0;
     const bool atL = (q.s + 2 == Ls), at0 = (q.s == 0);
     if (!(atL || at0)) return;
-    const float c1f = (float)__ldg(chif + q.site), c2f = (float)__ldg(chif + g.kvol + q.site),
-                c3f = (float)__ldg(chif + 2 * g.kvol + q.site);
+    const float c1f = (float)chif[q.site], c2f = (float)chif[g.kvol + q.site],
+                c3f = (float)chif[2 * g.kvol + q.site];
     const bool pin = (q.site == 0);
     if (atL && at0) {   // Ls = 2: one pair holds both walls
         wall_terms<DAG, IMASS, WA, 0>(acc[1], LdF2{in}, cs, LsI * q.site, f, c1f, c2f, c3f, pin, hpin);
