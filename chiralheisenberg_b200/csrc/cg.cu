@@ -20,7 +20,7 @@ void CgWork::release() {
     w = nullptr;
 }
 
-static bool cg_batch(PcgBatch<double2>& b, const Geom& g, float am3, float hpin, int imass,
+static bool cg_batch(PcgBatch<double2, 1>& b, const Geom& g, float am3, float hpin, int imass,
                      int ibound) {
     return plane_ok(g) && b.add(g, (double)(2.0f * ((3.0f - am3) + 1.0f)), (double)hpin,
                                 ibound == -1, imass, 0, pcg_sms());
@@ -31,16 +31,14 @@ cudaError_t cg_solve(CgWork& w, const Geom& g, const double2* phi, float res, co
                      int* status, cudaStream_t st) {
     if (!w.w) w.w = new PcgWork<double2>();
     PcgWork<double2>& W = *w.w;
-    PcgBatch<double2> b;
+    PcgBatch<double2, 1> b;
     if (!cg_batch(b, g, am3, hpin, imass, ibound)) return cudaErrorInvalidValue;
     cudaError_t e = W.reserve(b.units, 0, b.parts);
     if (e) return e;
     W.bind(b, chif);
-    pcg_congrad_enter(g, W.vec, x, phi, st);
-    std::vector<PcgDyn<double2>> dyn(1, pcg_congrad_dyn(g, res, x));
+    std::vector<PcgDyn<double2>> dyn(1, pcg_congrad_dyn(g, res, x, phi));
     std::vector<PcgSlot> slots(1, pcg_congrad_slot());
-    if ((e = W.solve(b, dyn, slots, st))) return e;
-    pcg_congrad_leave(g, W.vec, x, st);
+    if ((e = pcg_congrad(W, b, dyn, slots, st))) return e;
     if ((e = cudaStreamSynchronize(st))) return e;
     *itercg = slots[0].iters;
     *status = pcg_status(slots[0]);
@@ -117,22 +115,21 @@ extern "C" int chdwf_congrad_static(const void* Phi, void* x, const void* chi, i
     double2* vec = reinterpret_cast<double2*>(base + kStaticCtl + 64 * 1024 +
                                               3 * kStaticMaxKvol * sizeof(float));
     cudaStream_t st = (cudaStream_t)stream;
-    PcgBatch<double2> b;
+    PcgBatch<double2, 1> b;
     if (!cg_batch(b, g, am3, hpin, imass, ibound)) return 4;
     b.a.vec = vec;
-    b.a.chif = chif;
+    b.a.chif = b.a.chi_out = chif;
     b.a.part = part;
     b.a.dyn = &ctl->dyn;
     b.a.slot = ctl->slot;
     b.a.run = &ctl->run;
     StaticCtl hc;
     memset(&hc, 0, sizeof(hc));
-    hc.dyn = pcg_congrad_dyn(g, res, (double2*)x);
+    hc.dyn = pcg_congrad_dyn(g, res, (double2*)x, (const double2*)Phi, (const double*)chi);
     hc.slot[0] = hc.slot[1] = pcg_congrad_slot();
     hc.run.active = 1;
     if (cudaMemcpyAsync(ctl, &hc, sizeof(hc), cudaMemcpyHostToDevice, st) != cudaSuccess) return 3;
-    launch_round_chi((const double*)chi, chif, g.kvol, st);
-    pcg_congrad_enter(g, vec, (double2*)x, (const double2*)Phi, st);
+    pcg_congrad_enter(b.a, st);
     // chunks of 16 iterations; the scalars are copied into a host stack
     // variable after each chunk (launches after convergence return at once)
     const int64_t cap = hc.dyn.niterc;
@@ -153,7 +150,7 @@ extern "C" int chdwf_congrad_static(const void* Phi, void* x, const void* chi, i
         hr = hs[0].done ? hs[0] : hs[1];
         if (hr.done) break;
     }
-    pcg_congrad_leave(g, vec, (double2*)x, st);
+    pcg_congrad_leave(b.a, st);
     if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess) return 3;
     *itercg = hr.iters;
     if (hr.done == 2) {

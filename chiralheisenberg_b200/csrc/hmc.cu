@@ -398,7 +398,7 @@ cudaError_t hcg_solve(chdwf_hmc* h, const float2* phi, float res, int imass, con
                       float2* x, int* itercg, int* status) {
     using namespace chdwf;
     const Geom& g = h->g;
-    PcgBatch<hmc32> B;
+    PcgBatch<hmc32, 1> B;
     if (!B.add(g, h->diag(), 0.0f, 1, imass, 0, pcg_sms())) return cudaErrorInvalidValue;
     h->cg.bind(B, chi);
     const unsigned nb = nblk(g.kferm);
@@ -522,7 +522,7 @@ int chdwf_hmc_create(chdwf_hmc** out, int ksize, int ksizet, int kthird, float d
     if (!e) e = dalloc(&h->X0, nf);
     if (!e) e = dalloc(&h->X1, nf);
     if (!e) e = dalloc(&h->R, nf);
-    chdwf::PcgBatch<chdwf::hmc32> B;
+    chdwf::PcgBatch<chdwf::hmc32, 1> B;
     if (!e && (!chdwf::plane_ok(h->g) || !B.add(h->g, h->diag(), 0.0f, 1, imass, 0, chdwf::pcg_sms())))
         e = cudaErrorInvalidValue;
     if (!e) e = h->cg.reserve(B.units, 0, B.parts);

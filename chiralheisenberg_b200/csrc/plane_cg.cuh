@@ -24,8 +24,9 @@
 // system writes the other.  All systems of a batch start together, so the
 // iteration number is common; finished systems' blocks return at once.
 //
-// A system's blocks and the order of its sums depend on its lattice alone,
-// so a system's solution has the same bits alone and in any batch.
+// A system's blocks (of its sums: a block of the launch may hold several, see
+// PcgTile) and the order of its sums depend on its lattice alone, so a system's
+// solution has the same bits alone and in any batch.
 //
 // The batch's layout (lattices, plans, where each system's blocks and vectors
 // start) is a kernel argument: a block finds its system by a search over
@@ -43,7 +44,8 @@
 
 namespace chdwf {
 
-constexpr int kPcgThreads = 192;      // a block; 4 an SM at kPlaneRegs
+constexpr int kPcgThreads = 192;      // a block
+constexpr int kPcgPerSm = 4;          // stencil blocks an SM holds at kPlaneRegs
 constexpr int kPcgMaxBlocks = 2048;   // stencil blocks of one system
 // bytes of a vector a thread takes in k_pcg3
 constexpr int kPcgBytes = 64;
@@ -57,22 +59,26 @@ struct PcgSlot {
     int done, iters;
 };
 
-constexpr int kPcgSys = 32;           // systems of one set of launches
-constexpr int kPcgGeo = 6;            // distinct lattices and parameters among them
+// Systems of one set of launches, at most, and the same of chdwf_congrad_batch for
+// sets that are wider.  Their arguments take 17 KB a kernel, which the first pass on a
+// layout pays for (graph of 49 kernels: 5 to 10 ms more).
+constexpr int kPcgSys = 32, kPcgSysBatch = 256;
+// distinct lattices among NS systems
+constexpr int pcg_geos(int NS) { return NS / 8 + 2; }
 
 template <class T>
-struct PcgGeo {
-    typedef typename real_of<T>::type Real;
+struct alignas(8) PcgGeo {        // with 4 the stencil kernels spill 30 to 50 bytes more
     PlanePlan pl;
-    Real diag, hpin;
-    int apbc;
-    int nblk, neblk;                  // stencil blocks, element blocks (k_pcg3)
+    int nblk, neblk;                  // blocks of the stencil's sums, element blocks (k_pcg3)
+    int pack;                         // of the former in a block of the launch
 };
 // What may change from call to call in a batch of the same layout (device).
 template <class T>
 struct PcgDyn {
     typedef typename unit_of<T>::type V;
     V* x;
+    const V* phi;                     // congrad: right-hand side,
+    const double* chi;                // and chi to be rounded (null: it is already)
     typename real_of<T>::type sigma;
     float resid;                      // congrad: stop when betan < resid
     double rstop;                     // shifted: stop when |r|^2 <= rstop
@@ -83,18 +89,24 @@ struct PcgRun {                       // iterations before this chunk, before th
     int active;                       // systems still running
 };
 
-template <class T>
+template <class T_, int NS>
 struct PcgArgs {
+    typedef T_ T;
     typedef typename unit_of<T>::type V;
-    PcgGeo<T> geo[kPcgGeo];
-    int64_t vec0[kPcgSys];            // system's vectors p, r, x1 (units from vec)
-    int chi0[kPcgSys];                // its REAL*4 chi (from chif)
-    int part0[kPcgSys];               // its partials of |x1|^2, |r|^2, |p|^2, and alpha (from part)
-    int blk0[kPcgSys + 1], eblk0[kPcgSys + 1];
-    unsigned char gid[kPcgSys];
-    int nsys, ngeo;
+    typedef typename real_of<T>::type Real;
+    static constexpr int kMost = NS;
+    PcgGeo<T> geo[pcg_geos(NS)];
+    int64_t vec0[NS];                 // system's vectors p, r, x1 (units from vec)
+    Real diag[NS], hpin[NS];          // its parameters
+    int apbc[NS];
+    int chi0[NS];                     // its REAL*4 chi (from chif)
+    int part0[NS];                    // its partials of |x1|^2, |r|^2, |p|^2, and alpha (from part)
+    int blk0[NS + 1], eblk0[NS + 1];  // its first block in the launches
+    unsigned char gid[NS];            // its lattice's entry of geo
+    int nsys, ngeo, packed;
     V* vec;
     const float* chif;
+    float* chi_out;                   // the same where the batch holds it
     double* part;
     const PcgDyn<T>* dyn;
     PcgSlot* slot;                    // [nsys][2]
@@ -190,44 +202,85 @@ struct PcgEpi2 {
     }
 };
 
-template <bool DAG, int IMASS, class T, class Epi>
-__device__ __forceinline__ void pcg_sweep(const PcgArgs<T>& a, const PcgGeo<T>& G, int s, int b,
-                                          const typename unit_of<T>::type* in,
-                                          const PlaneThread& th, Epi& epi) {
-    for (uint32_t it = (uint32_t)b; it < G.pl.nitem; it += (uint32_t)G.nblk)
-        PcgOp<T>::template item<DAG, IMASS>(in, G.pl, th, it, a.chif + a.chi0[s], G.diag, G.hpin,
-                                            G.apbc != 0, epi);
+// The thread's place among a system's blocks.  With PACK a block of the launch
+// holds G.pack of them: warps g*kw to g*kw + kw - 1 (kw: a tile's warps) are block
+// b = pack * (block of the launch) + g; warps behind the last tile hold no site.
+// g is the same for a warp, and the shuffle lets the compiler know, so that what
+// hangs on b stays in uniform registers.  It costs k_pcg1 64 bytes of spills all
+// the same (FP64, 24^3x24: 107 ms a solve instead of 103), so launches that are
+// not packed have kernels without it.
+struct PcgTile {
+    int b, w0;                        // block, its first warp
+    PlaneThread th;
+};
+template <bool PACK, class T>
+__device__ __forceinline__ PcgTile pcg_tile(const PcgGeo<T>& G, int blk) {
+    if (!PACK) return PcgTile{blk, 0, plane_thread(G.pl)};
+    const int kw = G.pl.threads >> 5;
+    int g = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0) / kw;
+    g = g < G.pack ? g : G.pack - 1;
+    return PcgTile{blk * G.pack + g, g * kw,
+                   plane_thread(G.pl, (int)threadIdx.x - g * G.pl.threads)};
+}
+template <bool DAG, int IMASS, bool PACK, class A, class T, class Epi>
+__device__ __forceinline__ void pcg_sweep(const A& a, const PcgGeo<T>& G, int s,
+                                          const PcgTile& t, const typename unit_of<T>::type* in,
+                                          Epi& epi) {
+    if (PACK && t.b >= G.nblk) return;
+    for (uint32_t it = (uint32_t)t.b; it < G.pl.nitem; it += (uint32_t)G.nblk)
+        PcgOp<T>::template item<DAG, IMASS>(in, G.pl, t.th, it, a.chif + a.chi0[s], a.diag[s],
+                                            a.hpin[s], a.apbc[s] != 0, epi);
+}
+// Block b's partial, its warps' sums added in order: the same however many
+// blocks share a block of the launch.
+template <class T>
+__device__ __forceinline__ void pcg_partial(const PcgGeo<T>& G, const PcgTile& t, double loc,
+                                            double* part) {
+    __shared__ double sh[kPcgThreads / 32];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) loc += __shfl_down_sync(0xffffffffu, loc, o);
+    const int w = (int)threadIdx.x >> 5;
+    if ((threadIdx.x & 31) == 0) sh[w] = loc;
+    __syncthreads();
+    if ((int)threadIdx.x != 32 * t.w0 || t.b >= G.nblk) return;
+    double r = 0.0;
+    for (int i = 0; i < G.pl.threads >> 5; i++) r += sh[w + i];
+    part[t.b] = r;
 }
 template <class T>
 __device__ __forceinline__ int64_t pcg_units(const PlanePlan& pl) {
     return 8 * (int64_t)pl.U * pl.kvol;
 }
 
-template <class T, int IMASS>
-__global__ void __maxnreg__(kPlaneRegs) k_pcg1(const __grid_constant__ PcgArgs<T> a, int k) {
+template <class A, int IMASS, bool PACK>
+__global__ void __maxnreg__(kPlaneRegs) k_pcg1(const __grid_constant__ A a, int k) {
+    typedef typename A::T T;
     typedef typename unit_of<T>::type V;
     const int s = pcg_find(a.blk0, a.nsys, (int)blockIdx.x);
     const PcgGeo<T>& G = a.geo[a.gid[s]];
-    const int b = (int)blockIdx.x - a.blk0[s];
-    const PlaneThread th = plane_thread(G.pl);
+    const PcgTile t = pcg_tile<PACK>(G, (int)blockIdx.x - a.blk0[s]);
     V* p = a.vec + a.vec0[s];
     pdl_wait();
     if (a.slot[2 * s + (k & 1)].done) return;
     PcgEpi1<T> epi{p + 2 * pcg_units<T>(G.pl), 0.0};
-    pcg_sweep<false, IMASS>(a, G, s, b, p, th, epi);
-    __shared__ double sh[32];
-    const double loc = block_sum_any(epi.loc, sh);
-    if (threadIdx.x == 0) a.part[a.part0[s] + b] = loc;
+    pcg_sweep<false, IMASS, PACK>(a, G, s, t, p, epi);
+    if constexpr (PACK) {
+        pcg_partial(G, t, epi.loc, a.part + a.part0[s]);
+    } else {
+        __shared__ double sh[32];
+        const double loc = block_sum_any(epi.loc, sh);
+        if (threadIdx.x == 0) a.part[a.part0[s] + t.b] = loc;
+    }
 }
 
-template <class T, int IMASS>
-__global__ void __maxnreg__(kPlaneRegs) k_pcg2(const __grid_constant__ PcgArgs<T> a, int k) {
+template <class A, int IMASS, bool PACK>
+__global__ void __maxnreg__(kPlaneRegs) k_pcg2(const __grid_constant__ A a, int k) {
+    typedef typename A::T T;
     typedef typename unit_of<T>::type V;
     typedef typename real_of<T>::type Real;
     const int s = pcg_find(a.blk0, a.nsys, (int)blockIdx.x);
     const PcgGeo<T>& G = a.geo[a.gid[s]];
-    const int b = (int)blockIdx.x - a.blk0[s];
-    const PlaneThread th = plane_thread(G.pl);
+    const PcgTile t = pcg_tile<PACK>(G, (int)blockIdx.x - a.blk0[s]);
     V* p = a.vec + a.vec0[s];
     double* part = a.part + a.part0[s];
     PcgEpi2<T> epi{p, p + pcg_units<T>(G.pl), a.dyn[s].x, (Real)1, a.dyn[s].sigma, true, 0.0};
@@ -248,15 +301,21 @@ __global__ void __maxnreg__(kPlaneRegs) k_pcg2(const __grid_constant__ PcgArgs<T
         const double pap = tot + (double)epi.sigma * sum_partials_any(part + 2 * G.nblk, G.neblk);
         epi.alpha = pap > 0.0 ? (float)(c.rr / pap) : 0.0f;
     }
-    if (PcgOp<T>::kLateX && b == 0 && threadIdx.x == 0) part[2 * G.nblk + G.neblk] = (double)epi.alpha;
-    pcg_sweep<true, IMASS>(a, G, s, b, p + 2 * pcg_units<T>(G.pl), th, epi);
-    __shared__ double sh[32];
-    const double loc = block_sum_any(epi.loc, sh);
-    if (threadIdx.x == 0) part[G.nblk + b] = loc;
+    if (PcgOp<T>::kLateX && t.b == 0 && threadIdx.x == 0)
+        part[2 * G.nblk + G.neblk] = (double)epi.alpha;
+    pcg_sweep<true, IMASS, PACK>(a, G, s, t, p + 2 * pcg_units<T>(G.pl), epi);
+    if constexpr (PACK) {
+        pcg_partial(G, t, epi.loc, part + G.nblk);
+    } else {
+        __shared__ double sh[32];
+        const double loc = block_sum_any(epi.loc, sh);
+        if (threadIdx.x == 0) part[G.nblk + t.b] = loc;
+    }
 }
 
-template <class T>
-__global__ void __launch_bounds__(kPcgThreads) k_pcg3(const __grid_constant__ PcgArgs<T> a, int k) {
+template <class A>
+__global__ void __launch_bounds__(kPcgThreads) k_pcg3(const __grid_constant__ A a, int k) {
+    typedef typename A::T T;
     typedef typename unit_of<T>::type V;
     typedef typename real_of<T>::type Real;
     const int s = pcg_find(a.eblk0, a.nsys, (int)blockIdx.x);
@@ -348,15 +407,44 @@ __global__ void __launch_bounds__(kPcgThreads) k_pcg3(const __grid_constant__ Pc
     }
 }
 
-// ABI layout <-> planes of one system (FP64): p = x, r = Phi, and the solution
-// kept in planes in its own buffer while the solve runs.
-static __global__ void k_pcg_in(double2* __restrict__ out, const double2* __restrict__ in, Geom g) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i < g.kferm) out[i] = in[plane_unit_of<double2>(g, g.Ls, i).e];
-}
-static __global__ void k_pcg_out(double2* __restrict__ out, const double2* __restrict__ in, Geom g) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i < g.kferm) out[plane_unit_of<double2>(g, g.Ls, i).e] = in[i];
+// ABI layout <-> planes, congrad's systems (FP64), k_pcg3's blocks.  The solution
+// is kept in planes in its own buffer while the solve runs, so it passes through p
+// on the way in and through x1 on the way out:
+//   0  p = x, r = Phi (:1086-1089), chi rounded where the system brings it
+//   1  x = p
+//   2  x1 = x in the ABI's layout
+//   3  x = x1
+// One launch a step for all systems: launched one by one, a kernel or copy for
+// each, 128 solves on 4^4 spent 2.7 of their 4.5 ms there.
+template <int STEP, class A>
+__global__ void __launch_bounds__(kPcgThreads) k_pcg_move(const __grid_constant__ A a) {
+    typedef typename A::V V;
+    const int s = pcg_find(a.eblk0, a.nsys, (int)blockIdx.x);
+    const auto& G = a.geo[a.gid[s]];
+    const int64_t nu = pcg_units<typename A::T>(G.pl), kv = G.pl.kvol;
+    V *p = a.vec + a.vec0[s], *r = p + nu, *x1 = r + nu, *x = a.dyn[s].x;
+    const V* phi = a.dyn[s].phi;
+    const double* chi = a.dyn[s].chi;
+    float* chif = a.chi_out + a.chi0[s];
+    constexpr int N = pcg_units_thread<typename A::T>();
+    const int64_t i0 = (int64_t)((int)blockIdx.x - a.eblk0[s]) * (kPcgThreads * N) + threadIdx.x;
+#pragma unroll
+    for (int q = 0; q < N; q++) {
+        const int64_t i = i0 + q * kPcgThreads;
+        if (i >= nu) break;
+        if (STEP == 0 || STEP == 2) {
+            // unit (component c, s, site) of the planes; element s + Ls (site + kvol c)
+            const int64_t cs = (int64_t)((uint64_t)i / (uint64_t)kv), site = i - cs * kv;
+            const int c = (int)cs / G.pl.Ls;
+            const int64_t e = (cs - (int64_t)c * G.pl.Ls) + G.pl.Ls * (site + kv * c);
+            if (STEP == 0) {
+                p[i] = x[e];
+                r[i] = phi[e];
+                if (chi && i < 3 * kv) chif[i] = (float)chi[i];
+            } else x1[e] = x[i];
+        } else if (STEP == 1) x[i] = p[i];
+        else x[i] = x1[i];
+    }
 }
 
 // ---- host side ---------------------------------------------------------------------
@@ -367,49 +455,105 @@ inline int pcg_sms() {
     return nsm > 0 ? nsm : 1;
 }
 // A batch under construction: systems are added while they fit.
-template <class T>
+template <class T, int NS = kPcgSys>
 struct PcgBatch {
+    typedef PcgArgs<T, NS> Args;
     typedef typename real_of<T>::type Real;
     static constexpr bool kPair = std::is_same<typename unit_of<T>::type, cpair>::value;
-    PcgArgs<T> a;                     // layout; the pointers are set when it runs
+    static_assert(sizeof(Args) + 16 <= 32764, "beyond what kernel arguments may take");
+    Args a;                           // layout; the pointers are set when it runs
     int imass = 1;
     int64_t units = 0;
     int chis = 0, parts = 0;
     PcgBatch() { memset(&a, 0, sizeof(a)); }   // padding too: it is a graph's key
     // Vectors of a system: p, r, x1 and extra more.  False: the batch is full.
     bool add(const Geom& g, Real diag, Real hpin, int apbc, int im, int extra, int nsm) {
-        if (a.nsys == kPcgSys || (a.nsys > 0 && im != imass)) return false;
-        PcgGeo<T> G;
-        memset(&G, 0, sizeof(G));
-        G.pl = plane_plan(g, kPair, nsm, kPcgThreads);
-        G.diag = diag;
-        G.hpin = hpin;
-        G.apbc = apbc;
-        G.nblk = G.pl.nitem < (uint32_t)kPcgMaxBlocks ? (int)G.pl.nitem : kPcgMaxBlocks;
-        const int64_t nu = 8 * (int64_t)G.pl.U * g.kvol;
-        const int per = kPcgThreads * pcg_units_thread<T>();
-        const int64_t ne = (nu + per - 1) / per;
-        if (ne > (int64_t)1 << 30) return false;
-        G.neblk = (int)ne;
+        if (a.nsys == NS || (a.nsys > 0 && im != imass)) return false;
         int id = 0;
-        while (id < a.ngeo && memcmp(&a.geo[id], &G, sizeof(G)) != 0) id++;
-        if (id == kPcgGeo) return false;
-        if ((int64_t)a.eblk0[a.nsys] + ne > (int64_t)1 << 30 ||
+        while (id < a.ngeo &&
+               !(a.geo[id].pl.L == g.L && a.geo[id].pl.Lt == g.Lt && a.geo[id].pl.Ls == g.Ls))
+            id++;
+        if (id == pcg_geos(NS)) return false;
+        PcgGeo<T> G;
+        if (id < a.ngeo) G = a.geo[id];
+        else {
+            memset(&G, 0, sizeof(G));
+            G.pl = plane_plan(g, kPair, nsm, kPcgThreads);
+            G.nblk = G.pl.nitem < (uint32_t)kPcgMaxBlocks ? (int)G.pl.nitem : kPcgMaxBlocks;
+            const int per = kPcgThreads * pcg_units_thread<T>();
+            const int64_t ne = (8 * (int64_t)G.pl.U * g.kvol + per - 1) / per;
+            if (ne > (int64_t)1 << 30) return false;
+            G.neblk = (int)ne;
+            G.pack = 1;
+        }
+        if ((int64_t)a.eblk0[a.nsys] + G.neblk > (int64_t)1 << 30 ||
             (int64_t)chis + 3 * (int64_t)g.kvol > (int64_t)1 << 30)
             return false;
         if (id == a.ngeo) a.geo[a.ngeo++] = G;
         const int s = a.nsys++;
         imass = im;
         a.gid[s] = (unsigned char)id;
+        a.diag[s] = diag;
+        a.hpin[s] = hpin;
+        a.apbc[s] = apbc != 0;
         a.vec0[s] = units;
         a.chi0[s] = chis;
         a.part0[s] = parts;
         a.blk0[s + 1] = a.blk0[s] + G.nblk;
         a.eblk0[s + 1] = a.eblk0[s] + G.neblk;
-        units += (3 + extra) * nu;
+        units += (3 + extra) * vec_units(s);
         chis += 3 * g.kvol;
         parts += 2 * G.nblk + G.neblk + 1;
         return true;
+    }
+    // Packs a launch of more stencil blocks than fit the device at once (wave).  A
+    // small lattice's plan spreads tiles of one or two warps over the SMs, which
+    // suits one solve; in a batch each such block holds the place of six warps.
+    // Solves to 1e-6, ms not packed and packed: 5 on 8^4 (640 blocks, 320 packed) 3.5 and
+    // 2.8, 16 on 8^4 6.9 and 4.8, 32 on 6^4 9.8 and 3.8, 128 on 4^4 4.4 and 1.9.  Below
+    // one wave there is nothing to gain (4 on 8^4, 512 blocks: 2.7), and where only some
+    // lattices pack, the spills (PcgTile) cost 2% (20 lattices from 12^3 to 16^3: 76.7
+    // and 78.2), so a launch is packed where that takes a third of its blocks away.
+    void pack(int wave) {
+        if constexpr (NS > 1) {
+            const int before = a.blk0[a.nsys];
+            for (int m = 2; m <= kPcgThreads / 32 && a.blk0[a.nsys] > wave; m++) pack_by(m);
+            a.packed = a.blk0[a.nsys] <= before / 3 * 2;
+            if (!a.packed) pack_by(1);
+        }
+    }
+    // At most m blocks in one.
+    void pack_by(int m) {
+        for (int i = 0; i < a.ngeo; i++) {
+            const int most = kPcgThreads / a.geo[i].pl.threads;
+            a.geo[i].pack = m < most ? m : most;
+        }
+        for (int s = 0; s < a.nsys; s++)
+            a.blk0[s + 1] = a.blk0[s] + (geo(s).nblk + geo(s).pack - 1) / geo(s).pack;
+    }
+    // The same systems with room for M only: shorter kernel arguments.
+    template <int M> bool fits() const { return a.nsys <= M && a.ngeo <= pcg_geos(M); }
+    template <int M> PcgBatch<T, M> cut() const {
+        PcgBatch<T, M> b;
+        b.imass = imass;
+        b.units = units;
+        b.chis = chis;
+        b.parts = parts;
+        b.a.nsys = a.nsys;
+        b.a.ngeo = a.ngeo;
+        memcpy(b.a.geo, a.geo, sizeof(b.a.geo[0]) * a.ngeo);
+        for (int s = 0; s < a.nsys; s++) {
+            b.a.vec0[s] = a.vec0[s];
+            b.a.diag[s] = a.diag[s];
+            b.a.hpin[s] = a.hpin[s];
+            b.a.apbc[s] = a.apbc[s];
+            b.a.chi0[s] = a.chi0[s];
+            b.a.part0[s] = a.part0[s];
+            b.a.gid[s] = a.gid[s];
+            b.a.blk0[s + 1] = a.blk0[s + 1];
+            b.a.eblk0[s + 1] = a.eblk0[s + 1];
+        }
+        return b;
     }
     const PcgGeo<T>& geo(int s) const { return a.geo[a.gid[s]]; }
     int64_t vec_units(int s) const {
@@ -417,8 +561,8 @@ struct PcgBatch {
     }
 };
 
-template <class T>
-void pcg_launch_chunk(const PcgArgs<T>& a, int imass, int chunk, cudaStream_t st) {
+template <class A>
+void pcg_launch_chunk(const A& a, int imass, int chunk, cudaStream_t st) {
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
@@ -431,16 +575,22 @@ void pcg_launch_chunk(const PcgArgs<T>& a, int imass, int chunk, cudaStream_t st
     ce = c;
     ce.gridDim = dim3((unsigned)a.eblk0[a.nsys]);
     k_pcg_tick<<<1, 1, 0, st>>>(a.run, chunk);
-    for (int k = 0; k < chunk; k++) {
-        if (imass == 3) {
-            cudaLaunchKernelEx(&c, k_pcg1<T, 3>, a, k);
-            cudaLaunchKernelEx(&c, k_pcg2<T, 3>, a, k);
-        } else {
-            cudaLaunchKernelEx(&c, k_pcg1<T, 1>, a, k);
-            cudaLaunchKernelEx(&c, k_pcg2<T, 1>, a, k);
+    auto launch = [&](auto k1, auto k2) {
+        for (int k = 0; k < chunk; k++) {
+            cudaLaunchKernelEx(&c, k1, a, k);
+            cudaLaunchKernelEx(&c, k2, a, k);
+            cudaLaunchKernelEx(&ce, k_pcg3<A>, a, k);
         }
-        cudaLaunchKernelEx(&ce, k_pcg3<T>, a, k);
+    };
+    if constexpr (A::kMost > 1) {
+        if (a.packed) {
+            if (imass == 3) launch(k_pcg1<A, 3, true>, k_pcg2<A, 3, true>);
+            else launch(k_pcg1<A, 1, true>, k_pcg2<A, 1, true>);
+            return;
+        }
     }
+    if (imass == 3) launch(k_pcg1<A, 3, false>, k_pcg2<A, 3, false>);
+    else launch(k_pcg1<A, 1, false>, k_pcg2<A, 1, false>);
 }
 
 // Vectors and device state of a batch, kept between solves and grown when a
@@ -474,8 +624,8 @@ struct PcgWork {
         if ((e = cudaMalloc(&vec, sizeof(V) * (size_t)units)) ||
             (e = cudaMalloc(&chif, sizeof(float) * (size_t)(chis ? chis : 1))) ||
             (e = cudaMalloc(&part, sizeof(double) * (size_t)parts)) ||
-            (e = cudaMalloc(&dyn, sizeof(PcgDyn<T>) * kPcgSys)) ||
-            (e = cudaMalloc(&slot, sizeof(PcgSlot) * 2 * kPcgSys)) ||
+            (e = cudaMalloc(&dyn, sizeof(PcgDyn<T>) * kPcgSysBatch)) ||
+            (e = cudaMalloc(&slot, sizeof(PcgSlot) * 2 * kPcgSysBatch)) ||
             (e = cudaMalloc(&run, sizeof(PcgRun))) ||
             (e = cudaHostAlloc(&hflag_host, sizeof(int), cudaHostAllocMapped)) ||
             (e = cudaHostGetDevicePointer((void**)&hflag_dev, hflag_host, 0))) {
@@ -486,33 +636,50 @@ struct PcgWork {
         return cudaSuccess;
     }
     // chi: one field for all systems instead of the workspace's
-    void bind(PcgBatch<T>& b, const float* chi = nullptr) {
+    template <int NS> void bind(PcgBatch<T, NS>& b, const float* chi = nullptr) {
+        b.pack(pcg_sms() * kPcgPerSm);
         if (chi) memset(b.a.chi0, 0, sizeof(b.a.chi0));
         b.a.vec = vec;
         b.a.chif = chi ? chi : chif;
+        b.a.chi_out = chif;
         b.a.part = part;
         b.a.dyn = dyn;
         b.a.slot = slot;
         b.a.run = run;
         b.a.hflag = hflag_dev;
     }
-    // Runs a bound batch to its end.  Vectors initialised on st; dyn: the
-    // systems' solutions, scalars and caps; slots: their initial slots (FP32:
-    // |p|^2's partials as well), on return the final ones.
-    cudaError_t solve(const PcgBatch<T>& b, const std::vector<PcgDyn<T>>& hd,
+    // Runs a bound batch to its end.  Vectors initialised on st (congrad: by
+    // pcg_congrad_enter, between begin and run); dyn: the systems' solutions, scalars
+    // and caps; slots: their initial slots (FP32: |p|^2's partials as well), on return
+    // the final ones.
+    template <int NS>
+    cudaError_t solve(const PcgBatch<T, NS>& b, const std::vector<PcgDyn<T>>& hd,
                       std::vector<PcgSlot>& slots, cudaStream_t st) {
+        const cudaError_t e = begin(b, hd, slots, st);
+        return e ? e : run_to_end(b, hd, slots, st);
+    }
+    template <int NS>
+    cudaError_t begin(const PcgBatch<T, NS>& b, const std::vector<PcgDyn<T>>& hd,
+                      const std::vector<PcgSlot>& slots, cudaStream_t st) {
+        const int nsys = b.a.nsys;
+        std::vector<PcgSlot> s2(2 * nsys);
+        for (int i = 0; i < nsys; i++) s2[2 * i] = s2[2 * i + 1] = slots[i];
+        const PcgRun hr{0, 0, nsys};
+        cudaError_t e;
+        (void)((e = cudaMemcpyAsync(dyn, hd.data(), sizeof(PcgDyn<T>) * nsys, cudaMemcpyHostToDevice, st)) ||
+               (e = cudaMemcpyAsync(slot, s2.data(), sizeof(PcgSlot) * 2 * nsys, cudaMemcpyHostToDevice, st)) ||
+               (e = cudaMemcpyAsync(run, &hr, sizeof(hr), cudaMemcpyHostToDevice, st)));
+        return e;
+    }
+    template <int NS>
+    cudaError_t run_to_end(const PcgBatch<T, NS>& b, const std::vector<PcgDyn<T>>& hd,
+                           std::vector<PcgSlot>& slots, cudaStream_t st) {
         const int nsys = b.a.nsys;
         int cap = 0;
         for (const PcgDyn<T>& d : hd)
             if (d.niterc > cap) cap = d.niterc;
         std::vector<PcgSlot> s2(2 * nsys);
-        for (int i = 0; i < nsys; i++) s2[2 * i] = s2[2 * i + 1] = slots[i];
-        PcgRun hr{0, 0, nsys};
         cudaError_t e;
-        if ((e = cudaMemcpyAsync(dyn, hd.data(), sizeof(PcgDyn<T>) * nsys, cudaMemcpyHostToDevice, st)) ||
-            (e = cudaMemcpyAsync(slot, s2.data(), sizeof(PcgSlot) * 2 * nsys, cudaMemcpyHostToDevice, st)) ||
-            (e = cudaMemcpyAsync(run, &hr, sizeof(hr), cudaMemcpyHostToDevice, st)))
-            return e;
         *hflag_host = 0;
         constexpr int kChunk = 16;
         const cudaGraphExec_t ge =
@@ -553,29 +720,37 @@ inline PcgSlot pcg_congrad_slot() {
     s.betad = 1.0f;
     return s;
 }
-inline PcgDyn<double2> pcg_congrad_dyn(const Geom& g, float res, double2* x) {
+inline PcgDyn<double2> pcg_congrad_dyn(const Geom& g, float res, double2* x, const double2* phi,
+                                       const double* chi = nullptr) {
     PcgDyn<double2> d;
     memset(&d, 0, sizeof(d));
     d.x = x;
+    d.phi = phi;
+    d.chi = chi;
     d.resid = (float)g.kferm * res * res;                    // :1076
     d.niterc = (int)(g.Ls * (int64_t)g.kvol);
     return d;
 }
-// p = x ; r = Phi (:1086-1089) in planes, and x in planes in its own buffer
-inline void pcg_congrad_enter(const Geom& g, double2* p, double2* x, const double2* phi,
-                              cudaStream_t st) {
-    const unsigned nb = (unsigned)((g.kferm + kThreads - 1) / kThreads);
-    k_pcg_in<<<nb, kThreads, 0, st>>>(p, x, g);
-    k_pcg_in<<<nb, kThreads, 0, st>>>(p + g.kferm, phi, g);
-    cudaMemcpyAsync(x, p, sizeof(double2) * g.kferm, cudaMemcpyDeviceToDevice, st);
+// The systems' vectors set up from x and Phi, and x back in the ABI's layout.
+template <int STEP, class A>
+void pcg_move(const A& a, cudaStream_t st) {
+    k_pcg_move<STEP><<<(unsigned)a.eblk0[a.nsys], kPcgThreads, 0, st>>>(a);
+    k_pcg_move<STEP + 1><<<(unsigned)a.eblk0[a.nsys], kPcgThreads, 0, st>>>(a);
     count_launches(2);
 }
-// x back in the ABI's layout (through x1)
-inline void pcg_congrad_leave(const Geom& g, double2* p, double2* x, cudaStream_t st) {
-    double2* x1 = p + 2 * g.kferm;
-    k_pcg_out<<<(unsigned)((g.kferm + kThreads - 1) / kThreads), kThreads, 0, st>>>(x1, x, g);
-    cudaMemcpyAsync(x, x1, sizeof(double2) * g.kferm, cudaMemcpyDeviceToDevice, st);
-    count_launches(1);
+template <class A> void pcg_congrad_enter(const A& a, cudaStream_t st) { pcg_move<0>(a, st); }
+template <class A> void pcg_congrad_leave(const A& a, cudaStream_t st) { pcg_move<2>(a, st); }
+// A bound batch from begin to end.
+template <int NS>
+cudaError_t pcg_congrad(PcgWork<double2>& w, const PcgBatch<double2, NS>& b,
+                        const std::vector<PcgDyn<double2>>& dyn, std::vector<PcgSlot>& slots,
+                        cudaStream_t st) {
+    cudaError_t e = w.begin(b, dyn, slots, st);
+    if (e) return e;
+    pcg_congrad_enter(b.a, st);
+    if ((e = w.run_to_end(b, dyn, slots, st))) return e;
+    pcg_congrad_leave(b.a, st);
+    return cudaSuccess;
 }
 inline int pcg_status(const PcgSlot& s) { return s.done == 1 ? 0 : (s.done == 2 ? 1 : 2); }
 

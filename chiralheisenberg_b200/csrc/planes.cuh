@@ -303,9 +303,12 @@ __device__ __forceinline__ void plane_kappa(cpair acc[4], const cpair cur[4], fl
 }
 
 struct PlaneThread { int x, y, t; };   // the thread's place in its tile
-__device__ __forceinline__ PlaneThread plane_thread(const PlanePlan& pl) {
-    const int tid = threadIdx.x, r = tid / pl.nx, t = r / pl.ny;
+__device__ __forceinline__ PlaneThread plane_thread(const PlanePlan& pl, int tid) {
+    const int r = tid / pl.nx, t = r / pl.ny;
     return PlaneThread{tid - r * pl.nx, r - t * pl.ny, t};
+}
+__device__ __forceinline__ PlaneThread plane_thread(const PlanePlan& pl) {
+    return plane_thread(pl, (int)threadIdx.x);
 }
 // Where a work item puts the thread: flavour, run of units, site, and the byte
 // offsets in a plane of the site and its neighbours.  Threads without a site
