@@ -30,6 +30,7 @@
 #include <type_traits>
 #include <utility>
 
+#include "chunk_graph.h"
 #include "dwf_stencil.cuh"
 #include "lanczos.h"
 #include "planes.cuh"
@@ -421,6 +422,7 @@ __global__ void __maxnreg__(kPlaneRegs) k_lz1_M(LzArgsT<T> a, int k0) {
     constexpr int X = REGEN ? 0 : 1;
     const int nb = (int)gridDim.x - X, b = (int)blockIdx.x - X;
     const PlaneThread th = plane_thread(a.pp);
+    if (REGEN) pdl_wait();
     const int j = REGEN ? k0 : pass1_begin(ctl, k0, k0 == 0);
     PlaneM<T> em{reinterpret_cast<V*>(a.vt), REGEN ? 0 : *(volatile int*)&ctl->done, 0.0};
     if (!REGEN && b < 0) {
@@ -454,6 +456,7 @@ __global__ void __maxnreg__(kPlaneRegs) k_lz1_Md(LzArgsT<T> a, int k0) {
     constexpr int X = REGEN ? 0 : 1;
     const int nb = (int)gridDim.x - X, b = (int)blockIdx.x - X;
     const PlaneThread th = plane_thread(a.pp);
+    if (REGEN) pdl_wait();
     const int j = REGEN ? k0 : pass1_begin(ctl, k0, false);
     // M(j) ran if the solve had not stopped before iteration j: m is set with
     // done, by the scalar block of M^dagger(m)
@@ -492,38 +495,26 @@ __global__ void __maxnreg__(kPlaneRegs) k_lz1_Md(LzArgsT<T> a, int k0) {
     if (threadIdx.x == 0) a.part[nb + b] = loc;
 }
 
-// Regenerating pass 2: x += c_j q_j (iflag 0), or y_kj q_j on the two wall
-// slices of every pole's x_k (iflag 1), from r_j in planes.
-template <class T, int IFLAG>
-__global__ void __launch_bounds__(kThreads) k_lzp_acc(LzArgsT<T> a, int j) {
+// Regenerating pass 2, iflag 1: x_k += y_kj q_j on the two wall slices of every
+// pole's x_k, from r_j in planes.
+template <class T>
+__global__ void __launch_bounds__(kThreads) k_lzp_acc_walls(LzArgsT<T> a, int j) {
     typedef typename real_of<T>::type Real;
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const T* rj = ring(a, j);
+    const int64_t cs2 = 2 * (int64_t)a.g.kvol, kf2 = 8 * cs2;
+    if (t >= kf2) return;
     const Real ib = (Real)a.h.invbeta[j];
-    if (IFLAG == 0) {
-        if (t >= a.g.kferm) return;
-        const int64_t cs = t / a.g.kvol, site = t - cs * a.g.kvol;
-        const int c = (int)(cs / a.g.Ls), s = (int)(cs - (int64_t)c * a.g.Ls);
-        const double2 q = widen(zscal(ib, vget(a, rj, c, s, site)));
-        const double cj = a.h.c[j];
-        double2* x = a.x + s + (int64_t)a.g.Ls * site + a.g.cs * c;
-        x->x += cj * q.x;
-        x->y += cj * q.y;
-    } else {
-        const int64_t cs2 = 2 * (int64_t)a.g.kvol, kf2 = 8 * cs2;
-        if (t >= kf2) return;
-        const int c = (int)(t / cs2);
-        const int64_t r = t - c * cs2;
-        const double2 q =
-            widen(zscal(ib, vget(a, rj, c, (r & 1) ? a.g.Ls - 1 : 0, r >> 1)));
-        const int64_t H = kMaxIter + 2;
-        for (int k = 0; k < a.npole; k++) {
-            const double y = a.h.y[k * H + j];
-            double2 xv = a.xw[k * kf2 + t];
-            xv.x += y * q.x;
-            xv.y += y * q.y;
-            a.xw[k * kf2 + t] = xv;
-        }
+    const int c = (int)(t / cs2);
+    const int64_t r = t - c * cs2;
+    const double2 q =
+        widen(zscal(ib, vget(a, ring(a, j), c, (r & 1) ? a.g.Ls - 1 : 0, r >> 1)));
+    const int64_t H = kMaxIter + 2;
+    for (int k = 0; k < a.npole; k++) {
+        const double y = a.h.y[k * H + j];
+        double2 xv = a.xw[k * kf2 + t];
+        xv.x += y * q.x;
+        xv.y += y * q.y;
+        a.xw[k * kf2 + t] = xv;
     }
 }
 
@@ -777,6 +768,82 @@ __global__ void __launch_bounds__(kThreads, LzShape<T>::min_blocks)
     }
 }
 
+// ---- pass 2 from the stored basis ---------------------------------------
+// x += sum_j c_j q_j, q_j = r_j / beta_j, j = 1..m, in j order per element
+// (the same sequence of operations as the regenerating pass 2).  A thread
+// takes one 16-byte unit of the vectors (planes: one FP64 or two FP32
+// elements; the ABI's layout: one element), so the stored vectors, m of them
+// against one read and write of x, stream coalesced.  RING: the vectors are in
+// the residual ring (regenerating pass 2).
+template <class T> struct AccUnit;
+template <> struct AccUnit<double2> {
+    static constexpr int N = 1;
+    __device__ __forceinline__ static void get(const LzArgsT<double2>&, const double2* v,
+                                               int64_t i, double2* q) {
+        q[0] = __ldg(v + i);
+    }
+};
+template <> struct AccUnit<float2> {
+    static constexpr int N = 2;
+    __device__ __forceinline__ static void get(const LzArgsT<float2>& a, const float2* v,
+                                               int64_t i, float2* q) {
+        if (a.pl) {
+            const float4 f = __ldg(reinterpret_cast<const float4*>(v) + i);
+            const cpair p{make_float2(f.x, f.y), make_float2(f.z, f.w)};
+            q[0] = cpair_pt(p, 0);
+            q[1] = cpair_pt(p, 1);
+        } else {
+            q[0] = __ldg(v + i);
+            q[1] = make_float2(0.0f, 0.0f);
+        }
+    }
+};
+// Units of a stored vector, and the x elements of unit i: the first one's
+// index and the number of elements (x is in the ABI's layout, the elements
+// of a unit adjacent).
+template <class T>
+__host__ __device__ __forceinline__ int64_t acc_units(const LzArgsT<T>& a) {
+    return a.pl ? 8 * (int64_t)a.pp.U * a.g.kvol : a.g.kferm;
+}
+template <class T>
+__device__ __forceinline__ int64_t acc_elem(const LzArgsT<T>& a, int64_t i, int* n) {
+    constexpr int N = AccUnit<T>::N;
+    *n = 1;
+    if (!a.pl) return i;
+    const int64_t cu = i / a.g.kvol, site = i - cu * a.g.kvol;
+    const int c = (int)(cu / a.pp.U), u = (int)(cu - (int64_t)c * a.pp.U);
+    if (N == 2 && 2 * u + 1 < a.g.Ls) *n = 2;
+    return (int64_t)N * u + (int64_t)a.g.Ls * site + a.g.cs * c;
+}
+
+template <class T, bool RING>
+__global__ void __launch_bounds__(kThreads) k_lz_accum_x(LzArgsT<T> a, int j0, int j1) {
+    typedef typename real_of<T>::type Real;
+    constexpr int N = AccUnit<T>::N;
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= acc_units(a)) return;
+    int n;
+    const int64_t e = acc_elem(a, i, &n);
+    double2 xv[N];
+    xv[0] = a.x[e];
+    if (N == 2) xv[N - 1] = n == 2 ? a.x[e + 1] : make_double2(0.0, 0.0);
+#pragma unroll 4
+    for (int j = j0; j <= j1; j++) {
+        T q[N];
+        AccUnit<T>::get(a, RING ? ring(a, j) : a.basis + j * a.vs, i, q);
+        const Real ib = (Real)a.h.invbeta[j];
+        const double cj = a.h.c[j];
+#pragma unroll
+        for (int k = 0; k < N; k++) {
+            const double2 qj = widen(zscal(ib, q[k]));
+            xv[k].x += cj * qj.x;
+            xv[k].y += cj * qj.y;
+        }
+    }
+    a.x[e] = xv[0];
+    if (N == 2 && n == 2) a.x[e + 1] = xv[N - 1];
+}
+
 template <class T>
 static unsigned lz_direct_blocks(int64_t npts) {
     return (unsigned)((npts + LzShape<T>::unit - 1) / LzShape<T>::unit);
@@ -886,12 +953,12 @@ __global__ void k_lz_init(LzCtl* ctl, LzHist h, const double* part, int nb) {
 // vt, r_j, r_{j-1} and writes r_{j+1}; both read chi as REAL*4.
 // dep: programmatic dependent launch (see pass1_begin).
 template <class... P, class... A>
-static void launch_dep(bool dep, void (*k)(P...), unsigned nb, unsigned nt, cudaStream_t st,
-                       A... args) {
+static void launch_grid(bool dep, void (*k)(P...), unsigned grid, unsigned nt, size_t smem,
+                        cudaStream_t st, A... args) {
     cudaLaunchConfig_t c{};
-    c.gridDim = dim3(nb + 1);                        // nb workers and the scalar block
+    c.gridDim = dim3(grid);
     c.blockDim = dim3(nt);
-    c.dynamicSmemBytes = sizeof(double) * (nb + 3);
+    c.dynamicSmemBytes = smem;
     c.stream = st;
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -899,6 +966,12 @@ static void launch_dep(bool dep, void (*k)(P...), unsigned nb, unsigned nt, cuda
     c.attrs = &at;
     c.numAttrs = dep ? 1 : 0;
     cudaLaunchKernelEx(&c, k, P(args)...);
+}
+template <class... P, class... A>
+static void launch_dep(bool dep, void (*k)(P...), unsigned nb, unsigned nt, cudaStream_t st,
+                       A... args) {
+    // nb workers and the scalar block
+    launch_grid(dep, k, nb + 1, nt, sizeof(double) * (nb + 3), st, args...);
 }
 template <class T, int IMASS>
 static void launch_pass1_planes(const LzArgsT<T>& a, unsigned nb, int k0, int chunk, cudaStream_t st,
@@ -1119,15 +1192,26 @@ static void launch_pass2(const LzArgsT<T>& a, int j, int m, int iflag, cudaStrea
                          KernelTimer& tm) {
     const int apply = j < m;
     const double V = (double)a.g.kferm * sizeof(T), chi = 12.0 * a.g.kvol;
-    const double acc = iflag == 0 ? 2.0 * a.g.kferm * sizeof(double2) + V : 0.0;
+    // On planes x takes in three vectors at a time, while r_{j-2}, r_{j-1} and r_j are
+    // in the ring, in front of M^dagger(j), which writes over r_{j-2}.  x (FP64, the
+    // ABI's layout: elements Ls apart for neighbouring threads) is read and written
+    // once a triple, and the kernels are launched as pass 1's (launch_grid).  Solves to
+    // 1e-9 without a store: 12^3x8 11.8 ms, 20^3x20 68.7; 14.4 and 71.4 without the
+    // programmatic launches, 16.4 and 90 with x taken once a vector besides.
+    const bool take = iflag == 0 && (!a.pl || j % 3 == 0 || j == m);
+    const int j0 = j - (j - 1) % 3;
+    const double acc =
+        take ? 2.0 * a.g.kferm * sizeof(double2) + (a.pl ? j - j0 + 1 : 1) * V : 0.0;
     if (apply) tm.begin(timer_class<T>(3), st, 2 * V + chi + acc);
     if (a.pl) {
-        const int64_t n = iflag == 0 ? a.g.kferm : 16 * (int64_t)a.g.kvol;
-        const unsigned nbe = (unsigned)((n + kThreads - 1) / kThreads);
-        if (iflag == 0) k_lzp_acc<T, 0><<<nbe, kThreads, 0, st>>>(a, j);
-        else k_lzp_acc<T, 1><<<nbe, kThreads, 0, st>>>(a, j);
-        if (apply) k_lz1_M<T, IMASS, true><<<a.pp.nitem, a.pp.threads, 0, st>>>(a, j);
-        count_launches(1 + apply);
+        auto blocks = [](int64_t n) { return (unsigned)((n + kThreads - 1) / kThreads); };
+        if (iflag != 0)
+            k_lzp_acc_walls<T><<<blocks(16 * (int64_t)a.g.kvol), kThreads, 0, st>>>(a, j);
+        else if (take)
+            k_lz_accum_x<T, true><<<blocks(acc_units(a)), kThreads, 0, st>>>(a, j0, j);
+        if (apply)
+            launch_grid(!tm.enabled, k_lz1_M<T, IMASS, true>, a.pp.nitem, a.pp.threads, 0, st, a, j);
+        count_launches((iflag != 0 || take) + apply);
     } else {
         const unsigned nb = lz_direct_blocks<T>(a.g.npts);
         if (iflag == 0) k_lz2_M<T, IMASS, 0><<<nb, kThreads, 0, st>>>(a, j, apply);
@@ -1137,7 +1221,9 @@ static void launch_pass2(const LzArgsT<T>& a, int j, int m, int iflag, cudaStrea
     if (apply) {
         tm.end(st);
         tm.begin(timer_class<T>(3), st, 4 * V + chi);
-        if (a.pl) k_lz1_Md<T, IMASS, false, true><<<a.pp.nitem, a.pp.threads, 0, st>>>(a, j);
+        if (a.pl)
+            launch_grid(!tm.enabled, k_lz1_Md<T, IMASS, false, true>, a.pp.nitem, a.pp.threads, 0, st,
+                        a, j);
         else k_lz2_Md<T, IMASS><<<lz_direct_blocks<T>(a.g.npts), kThreads, 0, st>>>(a, j);
         tm.end(st);
         count_launches(1);
@@ -1501,81 +1587,6 @@ static void launch_accum_walls(const LzArgsT<T>& a, int m, int n, int64_t kvol, 
     }
 }
 
-// ---- pass 2 from the stored basis ---------------------------------------
-// x += sum_j c_j q_j, q_j = r_j / beta_j, j = 1..m, in j order per element
-// (the same sequence of operations as the regenerating pass 2).  A thread
-// takes one 16-byte unit of the vectors (planes: one FP64 or two FP32
-// elements; the ABI's layout: one element), so the stored vectors, m of them
-// against one read and write of x, stream coalesced.
-template <class T> struct AccUnit;
-template <> struct AccUnit<double2> {
-    static constexpr int N = 1;
-    __device__ __forceinline__ static void get(const LzArgsT<double2>&, const double2* v,
-                                               int64_t i, double2* q) {
-        q[0] = __ldg(v + i);
-    }
-};
-template <> struct AccUnit<float2> {
-    static constexpr int N = 2;
-    __device__ __forceinline__ static void get(const LzArgsT<float2>& a, const float2* v,
-                                               int64_t i, float2* q) {
-        if (a.pl) {
-            const float4 f = __ldg(reinterpret_cast<const float4*>(v) + i);
-            const cpair p{make_float2(f.x, f.y), make_float2(f.z, f.w)};
-            q[0] = cpair_pt(p, 0);
-            q[1] = cpair_pt(p, 1);
-        } else {
-            q[0] = __ldg(v + i);
-            q[1] = make_float2(0.0f, 0.0f);
-        }
-    }
-};
-// Units of a stored vector, and the x elements of unit i: the first one's
-// index and the number of elements (x is in the ABI's layout, the elements
-// of a unit adjacent).
-template <class T>
-__host__ __device__ __forceinline__ int64_t acc_units(const LzArgsT<T>& a) {
-    return a.pl ? 8 * (int64_t)a.pp.U * a.g.kvol : a.g.kferm;
-}
-template <class T>
-__device__ __forceinline__ int64_t acc_elem(const LzArgsT<T>& a, int64_t i, int* n) {
-    constexpr int N = AccUnit<T>::N;
-    *n = 1;
-    if (!a.pl) return i;
-    const int64_t cu = i / a.g.kvol, site = i - cu * a.g.kvol;
-    const int c = (int)(cu / a.pp.U), u = (int)(cu - (int64_t)c * a.pp.U);
-    if (N == 2 && 2 * u + 1 < a.g.Ls) *n = 2;
-    return (int64_t)N * u + (int64_t)a.g.Ls * site + a.g.cs * c;
-}
-
-template <class T>
-__global__ void __launch_bounds__(kThreads) k_lz_accum_x(LzArgsT<T> a, int j0, int j1) {
-    typedef typename real_of<T>::type Real;
-    constexpr int N = AccUnit<T>::N;
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= acc_units(a)) return;
-    int n;
-    const int64_t e = acc_elem(a, i, &n);
-    double2 xv[N];
-    xv[0] = a.x[e];
-    if (N == 2) xv[N - 1] = n == 2 ? a.x[e + 1] : make_double2(0.0, 0.0);
-#pragma unroll 4
-    for (int j = j0; j <= j1; j++) {
-        T q[N];
-        AccUnit<T>::get(a, a.basis + j * a.vs, i, q);
-        const Real ib = (Real)a.h.invbeta[j];
-        const double cj = a.h.c[j];
-#pragma unroll
-        for (int k = 0; k < N; k++) {
-            const double2 qj = widen(zscal(ib, q[k]));
-            xv[k].x += cj * qj.x;
-            xv[k].y += cj * qj.y;
-        }
-    }
-    a.x[e] = xv[0];
-    if (N == 2 && n == 2) a.x[e + 1] = xv[N - 1];
-}
-
 static constexpr int kAccumChunk = 64;
 
 // Per-shift solutions (iflag 2): x_k = sum_j y_kj q_j for poles k0..k0+7,
@@ -1798,7 +1809,7 @@ static cudaError_t lz_solve_t(LzWork& w, const Geom& g, const double2* phi, floa
             const unsigned nbx = (unsigned)((acc_units(a) + kThreads - 1) / kThreads);
             for (int j0 = 1; j0 <= m; j0 += kAccumChunk) {
                 const int j1 = j0 + kAccumChunk - 1 < m ? j0 + kAccumChunk - 1 : m;
-                k_lz_accum_x<T><<<nbx, kThreads, 0, st>>>(a, j0, j1);
+                k_lz_accum_x<T, false><<<nbx, kThreads, 0, st>>>(a, j0, j1);
                 count_launches(1);
             }
         } else if (a.wcap > 0) {
