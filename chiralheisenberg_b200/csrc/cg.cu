@@ -134,6 +134,7 @@ extern "C" int chdwf_congrad_static(const void* Phi, void* x, const void* chi, i
     // variable after each chunk (launches after convergence return at once)
     const int64_t cap = hc.dyn.niterc;
     int64_t launched = 0;
+    bool failed = false;
     PcgSlot hs[2];
     PcgSlot hr;
     memset(&hr, 0, sizeof(hr));
@@ -143,15 +144,19 @@ extern "C" int chdwf_congrad_static(const void* Phi, void* x, const void* chi, i
         count_launches(3 * 16 + 1);
         // a failed launch or copy ends the solve at once instead of launching
         // on until the iteration cap
-        if (cudaGetLastError() != cudaSuccess) return 3;
-        if (cudaMemcpyAsync(hs, ctl->slot, sizeof(hs), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-            cudaStreamSynchronize(st) != cudaSuccess)
-            return 3;
+        if (cudaGetLastError() != cudaSuccess ||
+            cudaMemcpyAsync(hs, ctl->slot, sizeof(hs), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+            cudaStreamSynchronize(st) != cudaSuccess) {
+            failed = true;
+            break;
+        }
         hr = hs[0].done ? hs[0] : hs[1];
         if (hr.done) break;
     }
     pcg_congrad_leave(b.a, st);
-    if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess) return 3;
+    failed |= cudaGetLastError() != cudaSuccess;
+    failed |= cudaStreamSynchronize(st) != cudaSuccess;
+    if (failed) return 3;
     *itercg = hr.iters;
     if (hr.done == 2) {
         fprintf(stdout, " # iterations of congrad exceeds niterc\n");   // :1151-1153

@@ -740,7 +740,8 @@ void pcg_move(const A& a, cudaStream_t st) {
 }
 template <class A> void pcg_congrad_enter(const A& a, cudaStream_t st) { pcg_move<0>(a, st); }
 template <class A> void pcg_congrad_leave(const A& a, cudaStream_t st) { pcg_move<2>(a, st); }
-// A bound batch from begin to end.
+// A bound batch from begin to end.  x is the solver's own in between, so it goes
+// back into the ABI's layout after an error too, and the GPU is done with it then.
 template <int NS>
 cudaError_t pcg_congrad(PcgWork<double2>& w, const PcgBatch<double2, NS>& b,
                         const std::vector<PcgDyn<double2>>& dyn, std::vector<PcgSlot>& slots,
@@ -748,9 +749,10 @@ cudaError_t pcg_congrad(PcgWork<double2>& w, const PcgBatch<double2, NS>& b,
     cudaError_t e = w.begin(b, dyn, slots, st);
     if (e) return e;
     pcg_congrad_enter(b.a, st);
-    if ((e = w.run_to_end(b, dyn, slots, st))) return e;
+    e = w.run_to_end(b, dyn, slots, st);
     pcg_congrad_leave(b.a, st);
-    return cudaSuccess;
+    if (e) cudaStreamSynchronize(st);
+    return e;
 }
 inline int pcg_status(const PcgSlot& s) { return s.done == 1 ? 0 : (s.done == 2 ? 1 : 2); }
 
