@@ -259,6 +259,14 @@ struct PoleCoef {
 // ended in a serial sum over 592 partials, and p_k and x_k updated every time.
 constexpr int kThrBlock = 128;
 constexpr int kThrChunk = 16;                  // q kept, at most
+// The q that a handle keeps: a longer chunk is an option, so it takes at most a
+// quarter of the memory that is free beside everything else, and else the two that
+// the solvers need (an even number of iterations).
+inline int thr_chunk(size_t vector_bytes, size_t free_bytes) {
+    int chunk = kThrChunk;
+    while (chunk > 2 && vector_bytes * chunk > free_bytes / 4) chunk /= 2;
+    return chunk;
+}
 struct ThrQCtl {
     ThrRun run[2];                             // by parity of the iteration
     int base, next;                            // iterations before this chunk, before the next
@@ -1249,19 +1257,15 @@ int chdwf_thr_create(chdwf_thr** out, int ksize, int ksizet, int kthird, float d
     if (!e) e = talloc(&h->Phi0, n * np);
     if (!e) e = talloc(&h->p, n * np);
     if (!e) e = talloc(&h->x1, n * np);
-    // a longer chunk is an option: where memory is short, a shorter one
-    for (h->chunk = chdwf::kThrChunk; !e && !h->ring; h->chunk /= 2) {
-        e = talloc(&h->ring, n * h->chunk);
-        if (!e) break;
-        if (h->chunk == 2) break;
-        cudaGetLastError();
-        e = cudaSuccess;
-    }
     if (!e) e = talloc(&h->part, 3 * chdwf::kRedBlocks);
     if (!e) e = talloc(&h->qctl, 1);
     if (!e) e = talloc(&h->cgctl, 1);
     if (!e) e = cudaHostAlloc((void**)&h->hflag_host, sizeof(int), cudaHostAllocMapped);
     if (!e) e = cudaHostGetDevicePointer((void**)&h->hflag_dev, h->hflag_host, 0);
+    size_t fr = 0, tot = 0;
+    if (!e) e = cudaMemGetInfo(&fr, &tot);
+    if (!e) h->chunk = chdwf::thr_chunk(sizeof(double2) * n, fr);
+    if (!e) e = talloc(&h->ring, n * h->chunk);
     if (!e) e = cudaMemsetAsync(h->theta, 0, sizeof(float) * n3, h->st);
     if (!e) e = cudaMemsetAsync(h->Phi0, 0, sizeof(double2) * n * np, h->st);
     if (!e) e = cudaStreamSynchronize(h->st);
