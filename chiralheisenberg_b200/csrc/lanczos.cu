@@ -236,7 +236,6 @@ __device__ __forceinline__ void wall_put(const LzArgsT<T>& a, int j1, int s, int
 // beta_j, a sum over the previous kernel's blocks, out of M.  Block b (of nb
 // workers) takes the items b, b + nb, ... and leaves its |.|^2 partial in
 // part[b] (M) or part[nb + b] (M^dagger); one more block a kernel does the
-// part[b] (M) or part[nb + b] (M^dagger); one more block a kernel does the
 // scalar work.
 //
 // Kernels k = 0..15 of M and M^dagger, after k_lz_tick, are captured as a
@@ -303,11 +302,10 @@ template <class T>
 struct PlaneM {
     typedef typename unit_of<T>::type V;
     V* vt;
-    int done;              // the solve has stopped: looked at after the first unit
+    int done;              // the solve has stopped: no item is begun
     double loc;
     __device__ __forceinline__ bool operator()(V acc[4], int64_t e, int64_t cst, uint32_t o,
                                                bool act, int, uint32_t) {
-        if (done) return false;
         if (!act) return true;
         // |vt|^2 is summed in FP64 from the first term: a pair's partial sum
         // in FP32 made the FP32 force solves 7% longer (alpha~ and beta steer
@@ -351,7 +349,6 @@ struct PlaneMd {
     }
     __device__ __forceinline__ bool operator()(V acc[4], int64_t e, int64_t cst, uint32_t o,
                                                bool act, int u, uint32_t site) {
-        if (done) return false;
         // FP64: q_j and q_{j-1} are loaded in front of the sum's block barriers.
         // FP32: behind them; the stencil of a pair leaves no registers for
         // them (100 bytes of spills; 24^3x24 M^dagger 2.5 us longer, against

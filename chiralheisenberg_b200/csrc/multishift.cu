@@ -15,8 +15,8 @@
 //
 // The corrections of several shifts run as one batch (plane_cg.cuh): their
 // scalars stay on the device and each iteration is three launches for all of
-// them: 20 shifts at 16^3x16 to 1e-10 take 91 ms.  One shift at a time, with
-// the scalars on the host (two round trips an iteration), they took 615 ms.
+// them: 20 shifts at 16^3x16 to 1e-10 take 92 to 99 ms.  One shift at a time, with
+// the scalars on the host (two round trips an iteration), they took 560 to 700 ms.
 #include <cmath>
 #include <cstring>
 #include <vector>

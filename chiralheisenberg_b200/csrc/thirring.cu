@@ -253,10 +253,11 @@ struct PoleCoef {
 // implicit types.  The q of a chunk of iterations are kept, and k_thr_poles
 // takes p_k and x_k through all of them at once, so the 2*ndiag vectors are read
 // and written once a chunk instead of once an iteration.
-// At 12^3x12 with 12 poles (162 blocks: launches and latency) k_thr_m takes 6 us
-// and k_thr_md 9, k_thr_poles 28 for 16 iterations; a solve with its 12 link
-// forces 2.3 ms, against 10.2 with seven kernels an iteration, two of which
-// ended in a serial sum over 592 partials, and p_k and x_k updated every time.
+// At 12^3x12 with 12 poles (162 blocks: launches and latency) an iteration takes
+// 9.8 us, k_thr_poles' share in it (28 us a chunk of 16); the call with 160
+// iterations, its 12 link forces and its host copies 2.3 to 2.5 ms, against 9.9 to 10.4
+// with seven kernels an iteration, two of which ended in a serial sum over 592
+// partials, and p_k and x_k updated every time.
 constexpr int kThrBlock = 128;
 constexpr int kThrChunk = 16;                  // q kept, at most
 // The q that a handle keeps: a longer chunk is an option, so it takes at most a

@@ -185,8 +185,10 @@ int chdwf_congrad_static(const void* Phi, void* x, const void* chi, int ksize, i
  * launches per CG stage; every system has its own lattice size, chi, imass,
  * hpin, am3, ibound, REAL*4 scalars and stopping test (congrad's rule with
  * residual res).  Pointers are device memory; x is the initial guess on
- * input.  itercg[i], status[i] per system; the return value is the worst
- * status. */
+ * input, and the solver's own storage while the call runs.  itercg[i],
+ * status[i] per system; the return value is the worst status.  After
+ * CHDWF_CUDA_ERROR an x is its guess or whatever iterate was reached, in its
+ * layout, and itercg and status of its system are not set. */
 typedef struct {
     int ksize, ksizet, kthird;
     int imass;
@@ -251,9 +253,9 @@ int chdwf_traj_propagator(chdwf_ctx* ctx, int ittt, int idsource, float res, flo
                           int imass, double* walls, int* itercg);
 /* nsrc wall-source propagators of fermion() in one batched solve (the
  * reference runs them one after the other, rhmc/cheisdwf.f:937-1012): source
- * i on timeslice ittt[i], Dirac idsource[i], as chdwf_traj_propagator; all
- * share chit, so chdwf_congrad_batch runs them as multi-right-hand-side
- * groups.  Each solve's arithmetic is that of chdwf_traj_propagator.  walls
+ * i on timeslice ittt[i], Dirac idsource[i], as chdwf_traj_propagator, by
+ * chdwf_congrad_batch.  Each solve's arithmetic is that of
+ * chdwf_traj_propagator.  walls
  * receives nsrc blocks of 8*kvol complex128 in chdwf_traj_propagator's
  * layout, itercg[i] the iterations of source i. */
 int chdwf_traj_propagators(chdwf_ctx* ctx, int nsrc, const int* ittt, const int* idsource,
